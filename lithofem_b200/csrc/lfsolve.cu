@@ -18,10 +18,10 @@
 //     gemm); the L and U blocks are copied to the factor store;
 //   solve (device): forward and backward sweeps over the tree, each front's
 //     right-hand side gathered from the global vector and its children's
-//     update vectors (no atomics); fronts up to SMALL_M rows in one block
-//     each (the vector in shared memory), larger ones through library
-//     trsm / gemm; A^T is solved with the same factors (U^T forward, L^T
-//     backward, inverse pivots last);
+//     update vectors (no atomics), the triangles in steps of 256 pivots with
+//     the 32 x 32 diagonal blocks kept as inverses (lfsolve_sweeps.cuh); A^T
+//     is solved with the same factors (U^T forward, L^T backward, inverse
+//     pivots last);
 //   refine: FP64 residual on the complex128 CSR, corrections from the
 //     factors, per right-hand-side column.
 #include <cublas_v2.h>
@@ -87,15 +87,6 @@ inline long long align_up(long long x) { return (x + ALIGN - 1) / ALIGN * ALIGN;
 constexpr int FPAD = 16;
 inline int pad_up(int x) { return (x + FPAD - 1) / FPAD * FPAD; }
 
-// fronts with at most SMALL_M rows, SMALL_K pivots and 2 k + r <= SMALL_BWD
-// are solved by one block each, with the right-hand-side block in shared
-// memory: m x nrhs entries forward, (2 k + r) x nrhs backward, at most
-// 192 kB in complex128 (two right-hand sides a pass); the block takes one
-// barrier per pivot, so fronts with more pivots go to the library path
-constexpr int SMALL_M = 4096;
-constexpr int SMALL_K = 256;
-constexpr int SMALL_BWD = 6144;
-constexpr int SOLVE_THREADS = 256;
 constexpr int MAX_NRHS_PASS = 2;  // right-hand sides per solve pass
 constexpr int LANES = 8;          // streams (and library handles) for the fronts
 constexpr int BATCH_MIN = 128;    // depths with this many fronts use batched calls
@@ -137,6 +128,9 @@ struct HostBuf {
   bool empty() const { return n == 0; }
 };
 
+// largest rows, pivots and update rows of a depth's fronts
+struct SolveShape { int m = 0, k = 0, r = 0; };
+
 struct Plan {
   int n = 0, n_ess = 0, nn = 0;       // rows, essential rows, numbered rows
   long long nnz = 0;
@@ -145,6 +139,7 @@ struct Plan {
   std::vector<int> perm, iperm;       // new -> original, original -> new (-1: essential)
   std::vector<int> node_of;           // new index -> node
   std::vector<std::vector<int>> by_depth;
+  std::vector<SolveShape> shape;      // per depth
   std::vector<long long> arena_size;  // per depth (entries)
   long long factor_entries = 0, vec_rows = 0;
   std::vector<int> r_orig;            // update rows (original indices), node blocks
@@ -381,9 +376,14 @@ int build_plan(int n, const int *I, const int *J, long long nnz, int ne, int nd,
     P.stride[d] = align_up(ld * ld);
   }
   long long fac = 0, roff = 0, vec = 0;
+  P.shape.assign(P.max_depth + 1, {});
   for (int d = 0; d <= P.max_depth; ++d)
     for (int s : P.by_depth[d]) {
       Node &N = P.nodes[s];
+      SolveShape &Z = P.shape[d];
+      Z.m = std::max(Z.m, N.m);
+      Z.k = std::max(Z.k, N.k);
+      Z.r = std::max(Z.r, N.m - N.k);
       N.arena_off = P.arena_size[d];
       if (P.batched[d]) {
         N.ld = P.kpad[d] + P.rpad[d];
@@ -406,6 +406,7 @@ int build_plan(int n, const int *I, const int *J, long long nnz, int ne, int nd,
     }
   P.factor_entries = fac;
   P.vec_rows = vec;
+  if (vec >= (1LL << 31)) return fail(LFSOLVE_ERR_ARG, "the fronts' rows exceed 2^31");
   for (int d = 0; d <= P.max_depth; ++d)
     P.peak_front_entries = std::max(P.peak_front_entries,
                                     P.arena_size[d] + (d < P.max_depth ? P.arena_size[d + 1] : 0));
@@ -774,265 +775,9 @@ __global__ void k_split_b(int kk, int r, const cuComplex *__restrict__ U, int ld
 }
 
 // ---------------------------------------------------------------------------
-// solve kernels.  Vector blocks: node s owns V[vec_off .. vec_off + m) per
-// right-hand-side column, columns nrhs apart by vec_rows (VR).
+// solve kernels
 // ---------------------------------------------------------------------------
-// gather: v[0:k] = b[perm[p0 + t]], v[k:m] = 0, plus the children's update
-// rows (v_child[k_c + t] at rel[t]); one block per node of the depth
-template <typename T>
-__global__ void k_gather_rhs(const int *__restrict__ list, const NodeDev *__restrict__ nodes,
-                             const int *__restrict__ child, const int *__restrict__ rel,
-                             const int *__restrict__ perm, const T *__restrict__ b, int ldb,
-                             T *__restrict__ V, long long VR, int nrhs) {
-  const int s = list[blockIdx.x];
-  const NodeDev N = nodes[s];
-  for (int c = 0; c < nrhs; ++c) {
-    T *v = V + N.vec_off + c * VR;
-    const T *bc = b + (long long)c * ldb;
-    for (int a = threadIdx.x; a < N.m; a += blockDim.x)
-      v[a] = a < N.k ? bc[perm[N.p0 + a]] : czero<T>();
-  }
-  __syncthreads();
-  for (int q = 0; q < 2; ++q) {  // children in turn: no two writers of one row
-    const int cs = child[2 * s + q];
-    if (cs < 0) continue;
-    const NodeDev C = nodes[cs];
-    const int r = C.m - C.k;
-    const int *rl = rel + C.r_off;
-    for (int c = 0; c < nrhs; ++c) {
-      T *v = V + N.vec_off + c * VR;
-      const T *u = V + C.vec_off + C.k + c * VR;
-      for (int a = threadIdx.x; a < r; a += blockDim.x) v[rl[a]] = cadd(v[rl[a]], u[a]);
-    }
-    __syncthreads();
-  }
-}
-
-// forward elimination of small fronts, in place on the vector block:
-// TRANS = 0: pivots, L11 (unit) and L21: v[0:k] = y1, v[k:m] -= L21 y1;
-// TRANS = 1: U11^T z1 = v[0:k], v[k:m] -= U12^T z1
-template <typename T, int TRANS>
-__global__ void __launch_bounds__(SOLVE_THREADS)
-k_fwd_small(const int *__restrict__ list, const NodeDev *__restrict__ nodes,
-            const T *__restrict__ fac, const int *__restrict__ ipiv, T *__restrict__ V,
-            long long VR, int nrhs) {
-  extern __shared__ unsigned char smraw[];
-  T *sv = reinterpret_cast<T *>(smraw);  // m x nrhs
-  __shared__ T red[SOLVE_THREADS / 32][MAX_NRHS_PASS];
-  const int s = list[blockIdx.x];
-  const NodeDev N = nodes[s];
-  const int m = N.m, k = N.k, tid = threadIdx.x;
-  const T *Pf = fac + N.fac_off;
-  const T *U12 = Pf + (long long)m * k;
-  for (int c = 0; c < nrhs; ++c)
-    for (int a = tid; a < m; a += blockDim.x) sv[a + c * m] = V[N.vec_off + a + c * VR];
-  __syncthreads();
-  if (TRANS == 0) {
-    if (tid == 0)
-      for (int i = 0; i < k; ++i) {
-        const int p = ipiv[N.p0 + i] - 1;
-        if (p != i)
-          for (int c = 0; c < nrhs; ++c) {
-            const T t = sv[i + c * m];
-            sv[i + c * m] = sv[p + c * m];
-            sv[p + c * m] = t;
-          }
-      }
-    __syncthreads();
-    for (int j = 0; j < k; ++j) {
-      const T *col = Pf + (long long)j * m;
-      T y[MAX_NRHS_PASS];
-      for (int c = 0; c < nrhs; ++c) y[c] = sv[j + c * m];
-      for (int a = j + 1 + tid; a < m; a += blockDim.x) {
-        const T l = col[a];
-        for (int c = 0; c < nrhs; ++c) sv[a + c * m] = cfms(sv[a + c * m], l, y[c]);
-      }
-      __syncthreads();
-    }
-  } else {
-    // z_j = (v_j - sum_{i<j} U[i][j] z_i) / U[j][j]: column j of U11 is
-    // contiguous; one block reduction per pivot
-    const int lane = tid & 31, w = tid >> 5;
-    for (int j = 0; j < k; ++j) {
-      const T *col = Pf + (long long)j * m;
-      T acc[MAX_NRHS_PASS];
-      for (int c = 0; c < nrhs; ++c) acc[c] = czero<T>();
-      for (int i = tid; i < j; i += blockDim.x) {
-        const T u = col[i];
-        for (int c = 0; c < nrhs; ++c) acc[c] = cadd(acc[c], cmul(u, sv[i + c * m]));
-      }
-      for (int c = 0; c < nrhs; ++c)
-        for (int o = 16; o; o >>= 1) {
-          acc[c].x += __shfl_xor_sync(0xffffffffu, acc[c].x, o);
-          acc[c].y += __shfl_xor_sync(0xffffffffu, acc[c].y, o);
-        }
-      if (lane == 0)
-        for (int c = 0; c < nrhs; ++c) red[w][c] = acc[c];
-      __syncthreads();
-      if (tid == 0) {
-        const T d = col[j];
-        for (int c = 0; c < nrhs; ++c) {
-          T sum = czero<T>();
-          for (int q = 0; q < (int)(blockDim.x >> 5); ++q) sum = cadd(sum, red[q][c]);
-          sv[j + c * m] = cdiv(csub(sv[j + c * m], sum), d);
-        }
-      }
-      __syncthreads();
-    }
-    // v[k + t] -= sum_i U12[i][t] z_i: a warp per update row, column t of
-    // U12 contiguous
-    const int r = m - k;
-    for (int t = w; t < r; t += blockDim.x >> 5) {
-      const T *col = U12 + (long long)t * k;
-      T acc[MAX_NRHS_PASS];
-      for (int c = 0; c < nrhs; ++c) acc[c] = czero<T>();
-      for (int i = lane; i < k; i += 32) {
-        const T u = col[i];
-        for (int c = 0; c < nrhs; ++c) acc[c] = cadd(acc[c], cmul(u, sv[i + c * m]));
-      }
-      for (int c = 0; c < nrhs; ++c)
-        for (int o = 16; o; o >>= 1) {
-          acc[c].x += __shfl_xor_sync(0xffffffffu, acc[c].x, o);
-          acc[c].y += __shfl_xor_sync(0xffffffffu, acc[c].y, o);
-        }
-      if (lane == 0)
-        for (int c = 0; c < nrhs; ++c) sv[k + t + c * m] = csub(sv[k + t + c * m], acc[c]);
-    }
-    __syncthreads();
-  }
-  for (int c = 0; c < nrhs; ++c)
-    for (int a = tid; a < m; a += blockDim.x) V[N.vec_off + a + c * VR] = sv[a + c * m];
-}
-
-// backward substitution of small fronts; x (original numbering, ld ldx):
-// TRANS = 0: x1 = U11^-1 (y1 - U12 x_R);
-// TRANS = 1: w = L11^-T (z1 - L21^T x_R), then the inverse row swaps
-template <typename T, int TRANS>
-__global__ void __launch_bounds__(SOLVE_THREADS)
-k_bwd_small(const int *__restrict__ list, const NodeDev *__restrict__ nodes,
-            const T *__restrict__ fac, const int *__restrict__ ipiv,
-            const int *__restrict__ perm, const int *__restrict__ r_orig,
-            const T *__restrict__ V, long long VR, T *__restrict__ x, int ldx, int nrhs) {
-  extern __shared__ unsigned char smraw[];
-  const int s = list[blockIdx.x];
-  const NodeDev N = nodes[s];
-  const int m = N.m, k = N.k, r = m - k, tid = threadIdx.x;
-  T *st = reinterpret_cast<T *>(smraw);  // k x nrhs: right-hand side
-  T *sx = st + (size_t)k * nrhs;         // k x nrhs: solution
-  T *sr = sx + (size_t)k * nrhs;         // r x nrhs: x of the update rows
-  __shared__ T red[SOLVE_THREADS / 32][MAX_NRHS_PASS];
-  const T *Pf = fac + N.fac_off;
-  const T *U12 = Pf + (long long)m * k;
-  const int *ro = r_orig + N.r_off;
-  for (int c = 0; c < nrhs; ++c) {
-    for (int a = tid; a < k; a += blockDim.x) st[a + c * k] = V[N.vec_off + a + c * VR];
-    for (int a = tid; a < r; a += blockDim.x) sr[a + c * r] = x[(long long)c * ldx + ro[a]];
-  }
-  __syncthreads();
-  const int lane = tid & 31, w = tid >> 5;
-  if (TRANS == 0) {
-    // st -= U12 x_R: a thread per pivot row, U12 columns contiguous
-    for (int i = tid; i < k; i += blockDim.x) {
-      T acc[MAX_NRHS_PASS];
-      for (int c = 0; c < nrhs; ++c) acc[c] = st[i + c * k];
-      for (int t = 0; t < r; ++t) {
-        const T u = U12[i + (long long)t * k];
-        for (int c = 0; c < nrhs; ++c) acc[c] = cfms(acc[c], u, sr[t + c * r]);
-      }
-      for (int c = 0; c < nrhs; ++c) st[i + c * k] = acc[c];
-    }
-    __syncthreads();
-    // back substitution with U11: one barrier per pivot (st[j] is final at
-    // step j; the solution goes to sx, which nobody reads in the loop)
-    for (int j = k - 1; j >= 0; --j) {
-      const T *col = Pf + (long long)j * m;
-      const T d = col[j];
-      T xj[MAX_NRHS_PASS];
-      for (int c = 0; c < nrhs; ++c) xj[c] = cdiv(st[j + c * k], d);
-      if (tid == 0)
-        for (int c = 0; c < nrhs; ++c) sx[j + c * k] = xj[c];
-      for (int i = tid; i < j; i += blockDim.x) {
-        const T u = col[i];
-        for (int c = 0; c < nrhs; ++c) st[i + c * k] = cfms(st[i + c * k], u, xj[c]);
-      }
-      __syncthreads();
-    }
-  } else {
-    // st -= L21^T x_R: a warp per pivot column, rows k..m-1 of P contiguous
-    for (int j = w; j < k; j += blockDim.x >> 5) {
-      const T *col = Pf + (long long)j * m + k;
-      T acc[MAX_NRHS_PASS];
-      for (int c = 0; c < nrhs; ++c) acc[c] = czero<T>();
-      for (int t = lane; t < r; t += 32) {
-        const T l = col[t];
-        for (int c = 0; c < nrhs; ++c) acc[c] = cadd(acc[c], cmul(l, sr[t + c * r]));
-      }
-      for (int c = 0; c < nrhs; ++c)
-        for (int o = 16; o; o >>= 1) {
-          acc[c].x += __shfl_xor_sync(0xffffffffu, acc[c].x, o);
-          acc[c].y += __shfl_xor_sync(0xffffffffu, acc[c].y, o);
-        }
-      if (lane == 0)
-        for (int c = 0; c < nrhs; ++c) st[j + c * k] = csub(st[j + c * k], acc[c]);
-    }
-    __syncthreads();
-    // L11^T (unit upper) back substitution: w_j = st_j - sum_{i>j} L[i][j] w_i
-    for (int j = k - 1; j >= 0; --j) {
-      const T *col = Pf + (long long)j * m;
-      T acc[MAX_NRHS_PASS];
-      for (int c = 0; c < nrhs; ++c) acc[c] = czero<T>();
-      for (int i = j + 1 + tid; i < k; i += blockDim.x) {
-        const T l = col[i];
-        for (int c = 0; c < nrhs; ++c) acc[c] = cadd(acc[c], cmul(l, sx[i + c * k]));
-      }
-      for (int c = 0; c < nrhs; ++c)
-        for (int o = 16; o; o >>= 1) {
-          acc[c].x += __shfl_xor_sync(0xffffffffu, acc[c].x, o);
-          acc[c].y += __shfl_xor_sync(0xffffffffu, acc[c].y, o);
-        }
-      if (lane == 0)
-        for (int c = 0; c < nrhs; ++c) red[w][c] = acc[c];
-      __syncthreads();
-      if (tid == 0)
-        for (int c = 0; c < nrhs; ++c) {
-          T sum = czero<T>();
-          for (int q = 0; q < (int)(blockDim.x >> 5); ++q) sum = cadd(sum, red[q][c]);
-          sx[j + c * k] = csub(st[j + c * k], sum);
-        }
-      __syncthreads();
-    }
-    if (tid == 0)
-      for (int i = k - 1; i >= 0; --i) {
-        const int p = ipiv[N.p0 + i] - 1;
-        if (p != i)
-          for (int c = 0; c < nrhs; ++c) {
-            const T t = sx[i + c * k];
-            sx[i + c * k] = sx[p + c * k];
-            sx[p + c * k] = t;
-          }
-      }
-    __syncthreads();
-  }
-  for (int c = 0; c < nrhs; ++c)
-    for (int a = tid; a < k; a += blockDim.x) x[(long long)c * ldx + perm[N.p0 + a]] = sx[a + c * k];
-}
-
-// big fronts: row swaps of the pivot rows of a vector block (forward,
-// TRANS = 0) or the inverse swaps (TRANS = 1); one thread
-template <typename T, int INV>
-__global__ void k_laswp(int k, const int *__restrict__ ipiv, T *__restrict__ v, int ldv, int nrhs) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  for (int q = 0; q < k; ++q) {
-    const int i = INV ? k - 1 - q : q;
-    const int p = ipiv[i] - 1;
-    if (p != i)
-      for (int c = 0; c < nrhs; ++c) {
-        const T t = v[i + (long long)c * ldv];
-        v[i + (long long)c * ldv] = v[p + (long long)c * ldv];
-        v[p + (long long)c * ldv] = t;
-      }
-  }
-}
+#include "lfsolve_sweeps.cuh"
 
 // Pivot permutation of every front: the front's sequential row swaps
 // (ipiv, 1-based) applied to the identity, so that the swapped vector is
@@ -1081,41 +826,9 @@ __global__ void k_perm_cols(int k, const int *__restrict__ perm, T *__restrict__
   for (int i = threadIdx.x; i < k; i += blockDim.x) col[i] = sv[perm[i]];
 }
 
-// big fronts: the pivot rows of a vector block permuted (INV = 0: row i
-// takes row perm[i]; INV = 1: row i goes to perm[i]); a block per column,
-// the k rows staged in shared memory
-template <typename T, int INV>
-__global__ void k_perm_pivots(int k, const int *__restrict__ perm, T *__restrict__ v, int ldv) {
-  extern __shared__ unsigned char perm_sm[];
-  T *sv = reinterpret_cast<T *>(perm_sm);
-  T *vc = v + (long long)blockIdx.x * ldv;
-  for (int i = threadIdx.x; i < k; i += blockDim.x) sv[i] = vc[i];
-  __syncthreads();
-  for (int i = threadIdx.x; i < k; i += blockDim.x) {
-    if (INV) vc[perm[i]] = sv[i];
-    else vc[i] = sv[perm[i]];
-  }
-}
-// pivots of a vector block that the shared-memory permutation can take
+// pivots that the shared-memory permutation of the update columns can take
 template <typename T>
 constexpr int perm_smem_max() { return (int)(160 * 1024 / sizeof(T)); }
-
-// big fronts: x_R gathered into a dense block (r x nrhs, ld r), and the
-// pivots' solution scattered back to x
-template <typename T>
-__global__ void k_gather_rows(int r, const int *__restrict__ ro, const T *__restrict__ x,
-                              int ldx, T *__restrict__ out, int nrhs) {
-  for (int c = 0; c < nrhs; ++c)
-    for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < r; a += gridDim.x * blockDim.x)
-      out[a + (long long)c * r] = x[(long long)c * ldx + ro[a]];
-}
-template <typename T>
-__global__ void k_scatter_pivots(int k, const int *__restrict__ pv, const T *__restrict__ v,
-                                 long long VR, T *__restrict__ x, int ldx, int nrhs) {
-  for (int c = 0; c < nrhs; ++c)
-    for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < k; a += gridDim.x * blockDim.x)
-      x[(long long)c * ldx + pv[a]] = v[a + c * VR];
-}
 
 // x[ess] = b[ess]
 template <typename T>
@@ -1311,14 +1024,15 @@ struct lfsolve {
   std::vector<long long *> d_asm_dst;
   std::vector<EaItem *> d_ea[2], d_co;    // per depth: extend-add items per slot, copy-out items
   std::vector<int> n_ea[2], n_co;
-  std::vector<int *> d_small, d_all;      // per depth: small fronts, all fronts
+  std::vector<int *> d_all;               // per depth: its fronts
   int *d_rel_fac = nullptr;               // child rows in the parents' front layout
   std::vector<EaItem *> d_sw;             // batched depths: swap items (front, columns)
   std::vector<int> n_sw;
   void **d_ptrs = nullptr;                // batched pointer arrays (3 x max fronts)
   int *d_bpiv = nullptr, *d_binf = nullptr;
-  std::vector<std::vector<int>> big;      // per depth: big fronts (host ids)
-  std::vector<int> n_small;
+  int *d_src = nullptr;                   // children's vector rows per vector row
+  InvItem *d_inv = nullptr;               // diagonal blocks kept as inverses
+  int n_inv = 0;
   // factors
   int prec = -1;
   void *d_fac = nullptr;
@@ -1342,9 +1056,8 @@ struct lfsolve {
   int lpiv_n[LANES] = {};
   cublasHandle_t blas_main = nullptr;
   // solve scratch
-  void *d_V = nullptr, *d_bw = nullptr, *d_xr = nullptr;
-  size_t xr_lane = 0;  // entries of one lane's x_R scratch
-  size_t V_bytes = 0, bw_bytes = 0, xr_bytes = 0;
+  void *d_V = nullptr, *d_Y = nullptr, *d_bw = nullptr;
+  size_t V_bytes = 0, Y_bytes = 0, bw_bytes = 0;
   double2 *d_r = nullptr, *d_x64 = nullptr;
   size_t r_bytes = 0;
   double *d_part = nullptr, *d_scale = nullptr;
@@ -1371,10 +1084,6 @@ int upload(T **dst, const std::vector<T> &v, cudaStream_t st) {
   return LFSOLVE_OK;
 }
 
-bool is_small(const Node &N) {
-  return N.m <= SMALL_M && N.k <= SMALL_K && 2 * N.k + (N.m - N.k) <= SMALL_BWD;
-}
-
 int ensure_uploaded(lfsolve *s) {
   if (s->uploaded) return LFSOLVE_OK;
   Plan &P = s->P;
@@ -1398,16 +1107,28 @@ int ensure_uploaded(lfsolve *s) {
   if ((rc = upload(&s->d_rorig, P.r_orig, st))) return rc;
   if ((rc = upload(&s->d_ess, P.ess, st))) return rc;
   if ((rc = upload(&s->d_tpos, P.tpos, st))) return rc;
+  // per vector row: the child rows that the forward sweep adds to it
+  std::vector<int> src(2 * (size_t)P.vec_rows, -1);
+  std::vector<InvItem> inv;
+  for (int i = 0; i < ns; ++i) {
+    const Node &N = P.nodes[i];
+    for (int q = 0; q < N.nchild; ++q) {
+      const Node &C = P.nodes[N.child[q]];
+      for (int t = 0; t < C.m - C.k; ++t)
+        src[2 * (size_t)(N.vec_off + P.rel[C.r_off + t]) + q] = (int)(C.vec_off + C.k + t);
+    }
+    for (int j0 = 0; j0 < N.k; j0 += 32) inv.push_back({i, j0});
+  }
+  if ((rc = upload(&s->d_src, src, st))) return rc;
+  if ((rc = upload(&s->d_inv, inv, st))) return rc;
+  s->n_inv = (int)inv.size();
   const int D = P.max_depth + 1;
   s->d_asm_src.assign(D, nullptr);
   s->d_asm_dst.assign(D, nullptr);
   for (int q = 0; q < 2; ++q) { s->d_ea[q].assign(D, nullptr); s->n_ea[q].assign(D, 0); }
   s->d_co.assign(D, nullptr);
   s->n_co.assign(D, 0);
-  s->d_small.assign(D, nullptr);
   s->d_all.assign(D, nullptr);
-  s->n_small.assign(D, 0);
-  s->big.assign(D, {});
   s->d_sw.assign(D, nullptr);
   s->n_sw.assign(D, 0);
   long long maxb = 1, maxpiv = 1;
@@ -1423,7 +1144,6 @@ int ensure_uploaded(lfsolve *s) {
     if ((rc = upload(&s->d_asm_src[d], P.asm_src[d], st))) return rc;
     if ((rc = upload(&s->d_asm_dst[d], P.asm_dst[d], st))) return rc;
     std::vector<EaItem> ea[2], co;
-    std::vector<int> small;
     for (int id : P.by_depth[d]) {
       const Node &N = P.nodes[id];
       for (int q = 0; q < N.nchild; ++q) {
@@ -1432,8 +1152,6 @@ int ensure_uploaded(lfsolve *s) {
         for (int c0 = 0; c0 < r; c0 += 32) ea[q].push_back({N.child[q], c0});
       }
       for (int c0 = 0; c0 < N.m; c0 += 32) co.push_back({id, c0});
-      if (is_small(N)) small.push_back(id);
-      else s->big[d].push_back(id);
     }
     for (int q = 0; q < 2; ++q) {
       if ((rc = upload(&s->d_ea[q][d], ea[q], st))) return rc;
@@ -1450,8 +1168,6 @@ int ensure_uploaded(lfsolve *s) {
     }
     if ((rc = upload(&s->d_co[d], co, st))) return rc;
     s->n_co[d] = (int)co.size();
-    if ((rc = upload(&s->d_small[d], small, st))) return rc;
-    s->n_small[d] = (int)small.size();
     if ((rc = upload(&s->d_all[d], P.by_depth[d], st))) return rc;
   }
   LS_CUDA(cudaStreamSynchronize(st));
@@ -1463,19 +1179,17 @@ int ensure_lanes(lfsolve *s) {
   if (s->blas_main) return LFSOLVE_OK;
   LS_BLAS(cublasCreate(&s->blas_main));
   LS_BLAS(cublasSetStream(s->blas_main, s->stream));
-  // the vector permutations stage up to 160 kB of pivot rows
-  LS_CUDA(cudaFuncSetAttribute(k_perm_pivots<cuComplex, 0>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-  LS_CUDA(cudaFuncSetAttribute(k_perm_pivots<cuComplex, 1>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-  LS_CUDA(cudaFuncSetAttribute(k_perm_pivots<cuDoubleComplex, 0>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-  LS_CUDA(cudaFuncSetAttribute(k_perm_pivots<cuDoubleComplex, 1>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
+  // the column permutations stage up to 160 kB of pivot rows
   LS_CUDA(cudaFuncSetAttribute(k_perm_cols<cuComplex>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
   LS_CUDA(cudaFuncSetAttribute(k_perm_cols<cuDoubleComplex>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
+  LS_CUDA(cudaFuncSetAttribute(k_diag_inverse<cuComplex>,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)inv_smem<cuComplex>()));
+  LS_CUDA(cudaFuncSetAttribute(k_diag_inverse<cuDoubleComplex>,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)inv_smem<cuDoubleComplex>()));
   for (int l = 0; l < LANES; ++l) {
     LS_CUDA(cudaStreamCreateWithFlags(&s->lane[l], cudaStreamNonBlocking));
     LS_BLAS(cublasCreate(&s->blas[l]));
@@ -1510,6 +1224,8 @@ int join_lanes(lfsolve *s) {
   }
   return LFSOLVE_OK;
 }
+
+int chunks(int n) { return n > 0 ? (n + SW_CHUNK - 1) / SW_CHUNK : 0; }
 
 int grid_for(long long n, int threads) {
   return (int)std::max<long long>(1, std::min<long long>((n + threads - 1) / threads, 148LL * 16));
@@ -1747,6 +1463,12 @@ int factor_impl(lfsolve *s, const double2 *vals) {
     if (prof) LS_CUDA(cudaEventRecord(evs[2 * d + 1], st));
   }
   LS_CUDA(cudaFreeAsync(arena[0], st));
+  // the sweeps read the diagonal blocks as inverses
+  if (s->n_inv > 0) {
+    k_diag_inverse<T><<<(s->n_inv + INV_WARPS - 1) / INV_WARPS, INV_WARPS * 32, inv_smem<T>(), st>>>(
+        s->n_inv, s->d_inv, s->d_nodes, fac);
+    LS_CUDA(cudaGetLastError());
+  }
   if (prof) {
     LS_CUDA(cudaStreamSynchronize(st));
     for (int d = D - 1; d >= 0; --d) {
@@ -1769,20 +1491,35 @@ int factor_impl(lfsolve *s, const double2 *vals) {
   return LFSOLVE_OK;
 }
 
-size_t small_fwd_smem(int m, int nrhs, size_t es) { return (size_t)m * nrhs * es; }
+// one launch of a phase over the fronts of a depth, at most nch chunks each
+template <typename T, int NR, int TRANS, int PH>
+int sweep_phase(const Sweep<T> &S, int nch, int fronts, int j0, cudaStream_t st) {
+  if (nch <= 0) return LFSOLVE_OK;
+  // grid.y holds 65,535 fronts
+  for (int f0 = 0; f0 < fronts; f0 += 65535) {
+    Sweep<T> P = S;
+    P.list = S.list + f0;
+    k_sweep<T, NR, TRANS, PH><<<dim3((unsigned)nch, (unsigned)std::min(65535, fronts - f0)), SW_T, 0,
+                                st>>>(P, j0);
+    LS_CUDA(cudaGetLastError());
+  }
+  return LFSOLVE_OK;
+}
 
-// one pass of at most MAX_NRHS_PASS columns: b (n x nr, ld n, precision T,
-// original numbering) -> x (same layout)
-template <typename T>
-int solve_pass(lfsolve *s, int nr, const T *b, T *x, int trans) {
+// A block per front walks through its phases where that fills the GPU or the
+// fronts are so small that launches would dominate; else a launch per phase.
+bool front_per_block(size_t fronts, int max_m) { return fronts >= 512 || max_m <= 160; }
+
+// one pass of NR columns: b (n x NR, ld n, precision T, original numbering)
+// -> x (same layout)
+template <typename T, int NR, int TRANS>
+int solve_pass(lfsolve *s, const T *b, T *x) {
   Plan &P = s->P;
   cudaStream_t st = s->stream;
-  const int D = P.max_depth + 1;
-  const T *fac = static_cast<const T *>(s->d_fac);
-  T *V = static_cast<T *>(s->d_V);
-  const long long VR = P.vec_rows;
-  const T one = CT<T>::mk(1.0, 0.0), mone = CT<T>::mk(-1.0, 0.0);
-  const int n = P.n;
+  const int D = P.max_depth + 1, n = P.n;
+  Sweep<T> S{s->d_nodes, nullptr, static_cast<const T *>(s->d_fac), s->d_perm, s->d_pperm,
+             s->d_rorig, s->d_src, static_cast<T *>(s->d_V), static_cast<T *>(s->d_Y),
+             P.vec_rows, P.nn, n, b, x};
   // LFSOLVE_PROFILE set: per-depth device times of both sweeps
   const bool prof = std::getenv("LFSOLVE_PROFILE") != nullptr;
   std::vector<cudaEvent_t> evs;
@@ -1790,153 +1527,69 @@ int solve_pass(lfsolve *s, int nr, const T *b, T *x, int trans) {
     evs.resize(4 * D);
     for (auto &e : evs) LS_CUDA(cudaEventCreate(&e));
   }
+  int rc;
   // forward, deepest level first
   for (int d = D - 1; d >= 0; --d) {
     if (prof) LS_CUDA(cudaEventRecord(evs[4 * d], st));
     const int cnt = (int)P.by_depth[d].size();
-    k_gather_rhs<T><<<cnt, 256, 0, st>>>(s->d_all[d], s->d_nodes, s->d_child, s->d_rel,
-                                         s->d_perm, b, n, V, VR, nr);
-    LS_CUDA(cudaGetLastError());
-    if (s->n_small[d] > 0) {
-      int mmax = 0;
-      for (int id : P.by_depth[d])
-        if (is_small(P.nodes[id])) mmax = std::max(mmax, P.nodes[id].m);
-      const size_t sm = small_fwd_smem(mmax, nr, sizeof(T));
-      if (trans) {
-        LS_CUDA(cudaFuncSetAttribute(k_fwd_small<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        k_fwd_small<T, 1><<<s->n_small[d], SOLVE_THREADS, sm, st>>>(s->d_small[d], s->d_nodes, fac,
-                                                                    s->d_ipiv, V, VR, nr);
-      } else {
-        LS_CUDA(cudaFuncSetAttribute(k_fwd_small<T, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        k_fwd_small<T, 0><<<s->n_small[d], SOLVE_THREADS, sm, st>>>(s->d_small[d], s->d_nodes, fac,
-                                                                    s->d_ipiv, V, VR, nr);
-      }
+    const SolveShape &Z = P.shape[d];
+    S.list = s->d_all[d];
+    if (front_per_block(cnt, Z.m)) {
+      k_sweep_fwd_front<T, NR, TRANS><<<cnt, SW_T, 0, st>>>(S);
       LS_CUDA(cudaGetLastError());
-    }
-    // large fronts: library calls, the fronts of the depth spread over the
-    // lanes (independent vector blocks)
-    if (!s->big[d].empty()) {
-      int rc = fork_lanes(s);
-      if (rc) return rc;
-      int li = 0;
-      for (int id : s->big[d]) {
-        const Node &N = P.nodes[id];
-        const int m = N.m, k = N.k, r = m - k;
-        if (k == 0) continue;  // the gathered block is its update already
-        const int l = li++ % LANES;
-        cublasHandle_t bh = s->blas[l];
-        T *v = V + N.vec_off;
-        const T *Pf = fac + N.fac_off;
-        const T *U12 = Pf + (long long)m * k;
-        if (!trans) {
-          if (k <= perm_smem_max<T>())
-            k_perm_pivots<T, 0><<<nr, 1024, (size_t)k * sizeof(T), s->lane[l]>>>(
-                k, s->d_pperm + N.p0, v, (int)VR);
-          else
-            k_laswp<T, 0><<<1, 32, 0, s->lane[l]>>>(k, s->d_ipiv + N.p0, v, (int)VR, nr);
-          LS_CUDA(cudaGetLastError());
-          LS_BLAS(trsm(bh, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_N,
-                       CUBLAS_DIAG_UNIT, k, nr, &one, Pf, m, v, (int)VR));
-          if (r > 0)
-            LS_BLAS(gemm(bh, CUBLAS_OP_N, CUBLAS_OP_N, r, nr, k, &mone, Pf + k, m, v, (int)VR,
-                         &one, v + k, (int)VR));
-        } else {
-          LS_BLAS(trsm(bh, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_T,
-                       CUBLAS_DIAG_NON_UNIT, k, nr, &one, Pf, m, v, (int)VR));
-          if (r > 0)
-            LS_BLAS(gemm(bh, CUBLAS_OP_T, CUBLAS_OP_N, r, nr, k, &mone, U12, k, v, (int)VR,
-                         &one, v + k, (int)VR));
-        }
+    } else {
+      if ((rc = sweep_phase<T, NR, TRANS, PH_GATHER>(S, (Z.m + SW_T - 1) / SW_T, cnt, 0, st))) return rc;
+      for (int j0 = 0; j0 < Z.k; j0 += SB) {
+        const int below = TRANS ? Z.k - j0 - SB : std::max(Z.m - j0 - SB, Z.r);
+        if ((rc = sweep_phase<T, NR, TRANS, PH_FWD_A>(S, 1, cnt, j0, st))) return rc;
+        if ((rc = sweep_phase<T, NR, TRANS, PH_FWD_B>(S, chunks(below), cnt, j0, st))) return rc;
       }
-      if ((rc = join_lanes(s))) return rc;
+      if (TRANS && (rc = sweep_phase<T, NR, TRANS, PH_FWD_U>(S, chunks(Z.r), cnt, 0, st))) return rc;
     }
     if (prof) LS_CUDA(cudaEventRecord(evs[4 * d + 1], st));
   }
   // essential rows
   if (P.n_ess > 0) {
-    k_ess_copy<T><<<grid_for(P.n_ess, 256), 256, 0, st>>>(P.n_ess, s->d_ess, b, n, x, n, nr);
+    k_ess_copy<T><<<grid_for(P.n_ess, 256), 256, 0, st>>>(P.n_ess, s->d_ess, b, n, x, n, NR);
     LS_CUDA(cudaGetLastError());
   }
   // backward, root first
   for (int d = 0; d < D; ++d) {
     if (prof) LS_CUDA(cudaEventRecord(evs[4 * d + 2], st));
-    if (s->n_small[d] > 0) {
-      int need = 0;  // rows of the largest (2 k + r) shared block
-      for (int id : P.by_depth[d]) {
-        const Node &N = P.nodes[id];
-        if (is_small(N)) need = std::max(need, 2 * N.k + (N.m - N.k));
-      }
-      const size_t sm = (size_t)need * nr * sizeof(T);
-      if (trans) {
-        LS_CUDA(cudaFuncSetAttribute(k_bwd_small<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        k_bwd_small<T, 1><<<s->n_small[d], SOLVE_THREADS, sm, st>>>(
-            s->d_small[d], s->d_nodes, fac, s->d_ipiv, s->d_perm, s->d_rorig, V, VR, x, n, nr);
-      } else {
-        LS_CUDA(cudaFuncSetAttribute(k_bwd_small<T, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        k_bwd_small<T, 0><<<s->n_small[d], SOLVE_THREADS, sm, st>>>(
-            s->d_small[d], s->d_nodes, fac, s->d_ipiv, s->d_perm, s->d_rorig, V, VR, x, n, nr);
-      }
+    const int cnt = (int)P.by_depth[d].size();
+    const SolveShape &Z = P.shape[d];
+    S.list = s->d_all[d];
+    if (front_per_block(cnt, Z.m)) {
+      k_sweep_bwd_front<T, NR, TRANS><<<cnt, SW_T, 0, st>>>(S);
       LS_CUDA(cudaGetLastError());
-    }
-    if (!s->big[d].empty()) {
-      int rc = fork_lanes(s);
-      if (rc) return rc;
-      int li = 0;
-      for (int id : s->big[d]) {
-        const Node &N = P.nodes[id];
-        const int m = N.m, k = N.k, r = m - k;
-        if (k == 0) continue;
-        const int l = li++ % LANES;
-        cublasHandle_t bh = s->blas[l];
-        cudaStream_t ls = s->lane[l];
-        T *v = V + N.vec_off;
-        const T *Pf = fac + N.fac_off;
-        const T *U12 = Pf + (long long)m * k;
-        T *xr = static_cast<T *>(s->d_xr) + (size_t)l * s->xr_lane;  // this lane's scratch
-        if (r > 0) {
-          k_gather_rows<T><<<grid_for(r, 256), 256, 0, ls>>>(r, s->d_rorig + N.r_off, x, n, xr, nr);
-          LS_CUDA(cudaGetLastError());
-        }
-        if (!trans) {
-          if (r > 0)
-            LS_BLAS(gemm(bh, CUBLAS_OP_N, CUBLAS_OP_N, k, nr, r, &mone, U12, k, xr, r, &one, v,
-                         (int)VR));
-          LS_BLAS(trsm(bh, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_N,
-                       CUBLAS_DIAG_NON_UNIT, k, nr, &one, Pf, m, v, (int)VR));
-        } else {
-          if (r > 0)
-            LS_BLAS(gemm(bh, CUBLAS_OP_T, CUBLAS_OP_N, k, nr, r, &mone, Pf + k, m, xr, r, &one, v,
-                         (int)VR));
-          LS_BLAS(trsm(bh, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_T,
-                       CUBLAS_DIAG_UNIT, k, nr, &one, Pf, m, v, (int)VR));
-          if (k <= perm_smem_max<T>())
-            k_perm_pivots<T, 1><<<nr, 1024, (size_t)k * sizeof(T), ls>>>(
-                k, s->d_pperm + N.p0, v, (int)VR);
-          else
-            k_laswp<T, 1><<<1, 32, 0, ls>>>(k, s->d_ipiv + N.p0, v, (int)VR, nr);
-          LS_CUDA(cudaGetLastError());
-        }
-        k_scatter_pivots<T><<<grid_for(k, 256), 256, 0, ls>>>(k, s->d_perm + N.p0, v, VR, x, n, nr);
-        LS_CUDA(cudaGetLastError());
+    } else if (Z.k > 0) {
+      if (Z.r > 0 && (rc = sweep_phase<T, NR, TRANS, PH_BWD_R>(S, chunks(Z.k), cnt, 0, st))) return rc;
+      for (int j0 = (Z.k - 1) / SB * SB; j0 >= 0; j0 -= SB) {
+        if ((rc = sweep_phase<T, NR, TRANS, PH_BWD_A>(S, 1, cnt, j0, st))) return rc;
+        if ((rc = sweep_phase<T, NR, TRANS, PH_BWD_B>(S, chunks(j0), cnt, j0, st))) return rc;
       }
-      if ((rc = join_lanes(s))) return rc;
     }
     if (prof) LS_CUDA(cudaEventRecord(evs[4 * d + 3], st));
   }
   if (prof) {
     LS_CUDA(cudaStreamSynchronize(st));
     for (int d = D - 1; d >= 0; --d) {
-      float f = 0.f, b = 0.f;
+      float f = 0.f, w = 0.f;
       LS_CUDA(cudaEventElapsedTime(&f, evs[4 * d], evs[4 * d + 1]));
-      LS_CUDA(cudaEventElapsedTime(&b, evs[4 * d + 2], evs[4 * d + 3]));
-      std::printf("lfsolve solve profile (%s, %d rhs): depth %2d fronts %5zu (%zu large)  "
-                  "forward %7.3f ms  backward %7.3f ms\n", trans ? "A^T" : "A", nr, d,
-                  P.by_depth[d].size(), s->big[d].size(), f, b);
+      LS_CUDA(cudaEventElapsedTime(&w, evs[4 * d + 2], evs[4 * d + 3]));
+      std::printf("lfsolve solve profile (%s, %d rhs): depth %2d fronts %5zu  "
+                  "forward %7.3f ms  backward %7.3f ms\n", TRANS ? "A^T" : "A", NR, d,
+                  P.by_depth[d].size(), f, w);
     }
     std::fflush(stdout);
     for (auto &e : evs) cudaEventDestroy(e);
   }
   return LFSOLVE_OK;
+}
+template <typename T>
+int solve_pass(lfsolve *s, int nr, const T *b, T *x, int trans) {
+  if (nr == 1) return trans ? solve_pass<T, 1, 1>(s, b, x) : solve_pass<T, 1, 0>(s, b, x);
+  return trans ? solve_pass<T, 2, 1>(s, b, x) : solve_pass<T, 2, 0>(s, b, x);
 }
 
 int ensure_solve_scratch(lfsolve *s, size_t es) {
@@ -1947,14 +1600,11 @@ int ensure_solve_scratch(lfsolve *s, size_t es) {
     LS_CUDA(cudaMalloc(&s->d_V, V));
     s->V_bytes = V;
   }
-  size_t rmax = 1;
-  for (const Node &N : P.nodes) rmax = std::max(rmax, (size_t)(N.m - N.k));
-  s->xr_lane = rmax * MAX_NRHS_PASS;
-  const size_t xr = s->xr_lane * LANES * es;
-  if (s->xr_bytes < xr) {
-    if (s->d_xr) LS_CUDA(cudaFree(s->d_xr));
-    LS_CUDA(cudaMalloc(&s->d_xr, xr));
-    s->xr_bytes = xr;
+  const size_t Y = (size_t)std::max(1, P.nn) * MAX_NRHS_PASS * es;
+  if (s->Y_bytes < Y) {
+    if (s->d_Y) LS_CUDA(cudaFree(s->d_Y));
+    LS_CUDA(cudaMalloc(&s->d_Y, Y));
+    s->Y_bytes = Y;
   }
   const size_t bw = (size_t)P.n * 2 * MAX_NRHS_PASS * es;  // b and x in the factor precision
   if (s->bw_bytes < bw) {
@@ -2388,7 +2038,7 @@ void lfsolve_destroy(lfsolve *s) {
   if (s->stream) cudaStreamSynchronize(s->stream);
   free_factors(s);
   void *bufs[] = {s->d_nodes, s->d_child, s->d_rel, s->d_perm, s->d_rorig, s->d_ess, s->d_tpos,
-                  s->d_ipiv, s->d_info, s->d_V, s->d_bw, s->d_xr, s->d_r, s->d_part, s->d_scale,
+                  s->d_ipiv, s->d_info, s->d_V, s->d_Y, s->d_bw, s->d_src, s->d_inv, s->d_r, s->d_part, s->d_scale,
                   s->d_pperm};
   for (void *p : bufs)
     if (p) cudaFree(p);
@@ -2396,7 +2046,6 @@ void lfsolve_destroy(lfsolve *s) {
   for (auto *p : s->d_asm_dst) if (p) cudaFree(p);
   for (int q = 0; q < 2; ++q) for (auto *p : s->d_ea[q]) if (p) cudaFree(p);
   for (auto *p : s->d_co) if (p) cudaFree(p);
-  for (auto *p : s->d_small) if (p) cudaFree(p);
   for (auto *p : s->d_sw) if (p) cudaFree(p);
   if (s->d_rel_fac) cudaFree(s->d_rel_fac);
   if (s->d_ptrs) cudaFree(s->d_ptrs);

@@ -1,0 +1,489 @@
+// Triangular sweeps of the multifrontal solve, included by lfsolve.cu inside
+// its namespace (after NodeDev and the complex helpers).
+//
+// A front's factors are P (m x k: L11\U11, then L21) and U12 (k x r).  A
+// substitution with L11 or U11 is a serial chain of k pivots.  Here it is cut
+// into steps of SB pivots: one block solves a step's SB x SB triangle
+// (diag_solve), then as many blocks as there are rows apply its columns.
+// Inside the triangle the chain is cut to SB / 32 links, because the 32 x 32
+// blocks on the diagonal of L11 and U11 are kept as their inverses
+// (k_diag_inverse, once per factorization, in place).  32 is as far as the
+// inverses go: with 32 x 32 blocks the residuals of complex128 solves are
+// those of plain substitution (1.5e-12 on a 111k-row contact hole, 1.6e-12
+// before), with 256 x 256 blocks they grow up to elevenfold.
+//
+// Bound: every factor entry is read once a sweep pair from HBM; on the
+// smallest systems the launches.
+//
+// Vectors: node s owns V[vec_off .. vec_off + m) per right-hand-side column
+// (columns VR apart); Y[p0 .. p0 + k) (columns nn apart) holds its
+// intermediate pivot values.
+//
+// Step of a front, pivots J = [j0, j1):
+//   forward,  A:    Y_J = L_JJ^-1 V_J;      V_rest -= P_rest,J Y_J
+//   forward,  A^T:  Y_J = U_JJ^-T V_J;      V_(>J) -= P_J,(>J)^T Y_J; after
+//                   the last step V_R -= U12^T Y
+//   backward, A:    Y -= U12 x_R; then from the last step: V_J = U_JJ^-1 Y_J,
+//                   Y_(<J) -= P_(<J),J V_J
+//   backward, A^T:  Y -= L21^T x_R; then V_J = L_JJ^-T Y_J,
+//                   Y_(<J) -= P_J,(<J)^T V_J
+constexpr int SB = 256;        // pivots of a step
+constexpr int SW_T = 256;      // threads of a sweep block (one per pivot of a step)
+constexpr int SW_W = SW_T / 32;
+constexpr int SW_TILE = 256;   // vector entries staged at a time
+constexpr int SW_CHUNK = 32;   // rows (or columns of the transposed product) a block forms at once
+static_assert(SB == SW_T, "diag_solve takes a pivot a thread");
+
+template <typename T> __device__ __forceinline__ void cfma(T &a, T x, T y) {
+  a.x = fma(x.x, y.x, a.x); a.x = fma(-x.y, y.y, a.x);
+  a.y = fma(x.x, y.y, a.y); a.y = fma(x.y, y.x, a.y);
+}
+
+template <typename T> struct Sweep {
+  const NodeDev *nodes;
+  const int *list;          // the fronts of the depth
+  const T *fac;
+  const int *perm, *pperm;  // elimination order; pivot permutation of every front
+  const int *rorig;         // update rows in the original numbering
+  const int *src;           // per vector row: the two children's rows that add to it (-1: none)
+  T *V, *Y;
+  long long VR;
+  int nn, n;
+  const T *b;               // right-hand side (n a column, original numbering)
+  T *x;                     // solution
+};
+
+template <typename T, int NR> struct SweepSmem {
+  T in[SW_TILE * NR];
+  T red[SW_W * SW_CHUNK * NR];
+};
+
+// out[q] (threads 0..31: row r0 + lane) = sum over c < nc of A[row, c] in(c, q),
+// the warps taking every SW_W-th column, eight loads in flight a thread;
+// reduced in warp order
+template <typename T, int NR, class In>
+__device__ __forceinline__ void tile_rows(const T *__restrict__ A, int ld, int r0, int nr, int nc,
+                                          In in, SweepSmem<T, NR> &sm, T (&out)[NR]) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int row = r0 + lane;
+  const T *Ar = A + min(row, nr - 1);
+  T acc[NR];
+#pragma unroll
+  for (int q = 0; q < NR; ++q) acc[q] = czero<T>();
+  for (int t0 = 0; t0 < nc; t0 += SW_TILE) {
+    const int tn = min(SW_TILE, nc - t0);
+    __syncthreads();
+    for (int t = threadIdx.x; t < tn * NR; t += SW_T) sm.in[t] = in(t0 + t / NR, t % NR);
+    __syncthreads();
+    int c = w;
+    for (; c + 7 * SW_W < tn; c += 8 * SW_W) {
+      T a[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) a[u] = Ar[(long long)(t0 + c + u * SW_W) * ld];
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+#pragma unroll
+        for (int q = 0; q < NR; ++q) cfma(acc[q], a[u], sm.in[(c + u * SW_W) * NR + q]);
+    }
+    for (; c < tn; c += SW_W) {
+      const T a = Ar[(long long)(t0 + c) * ld];
+#pragma unroll
+      for (int q = 0; q < NR; ++q) cfma(acc[q], a, sm.in[c * NR + q]);
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < NR; ++q) sm.red[(w * SW_CHUNK + lane) * NR + q] = acc[q];
+  __syncthreads();
+  if (w == 0)
+#pragma unroll
+    for (int q = 0; q < NR; ++q) {
+      T s = sm.red[lane * NR + q];
+#pragma unroll
+      for (int v = 1; v < SW_W; ++v) s = cadd(s, sm.red[(v * SW_CHUNK + lane) * NR + q]);
+      out[q] = s;
+    }
+}
+
+// out[u][q] (every lane of warp w: column c0 + w + SW_W u) = sum over rows i < nr
+// of A[i, column] in(i, q): lanes along the contiguous rows, four columns a
+// warp with their loads in flight together
+template <typename T, int NR, class In>
+__device__ __forceinline__ void tile_cols(const T *__restrict__ A, int ld, int nr, int c0, int nc,
+                                          In in, SweepSmem<T, NR> &sm,
+                                          T (&out)[SW_CHUNK / SW_W][NR]) {
+  constexpr int NC = SW_CHUNK / SW_W;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const T *Ac[NC];
+#pragma unroll
+  for (int u = 0; u < NC; ++u) {
+    Ac[u] = A + (long long)min(c0 + w + SW_W * u, nc - 1) * ld;
+#pragma unroll
+    for (int q = 0; q < NR; ++q) out[u][q] = czero<T>();
+  }
+  for (int t0 = 0; t0 < nr; t0 += SW_TILE) {
+    const int tn = min(SW_TILE, nr - t0);
+    __syncthreads();
+    for (int t = threadIdx.x; t < tn * NR; t += SW_T) sm.in[t] = in(t0 + t / NR, t % NR);
+    __syncthreads();
+#pragma unroll 2
+    for (int i = lane; i < tn; i += 32) {
+      T a[NC];
+#pragma unroll
+      for (int u = 0; u < NC; ++u) a[u] = Ac[u][t0 + i];
+#pragma unroll
+      for (int u = 0; u < NC; ++u)
+#pragma unroll
+        for (int q = 0; q < NR; ++q) cfma(out[u][q], a[u], sm.in[i * NR + q]);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < NC; ++u)
+#pragma unroll
+    for (int q = 0; q < NR; ++q)
+      for (int o = 16; o; o >>= 1) {
+        out[u][q].x += __shfl_xor_sync(0xffffffffu, out[u][q].x, o);
+        out[u][q].y += __shfl_xor_sync(0xffffffffu, out[u][q].y, o);
+      }
+}
+
+// f(column, out[q]) for the chunk's columns below nc, one lane each
+template <typename T, int NR, class F>
+__device__ __forceinline__ void each_col(T (&out)[SW_CHUNK / SW_W][NR], int c0, int nc, F f) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+  for (int u = 0; u < SW_CHUNK / SW_W; ++u) {
+    const int col = c0 + w + SW_W * u;
+    if (lane == u && col < nc) f(col, out[u]);
+  }
+}
+
+// The triangle of one step, v[q] = this thread's pivot of the step (thread t:
+// pivot t < nb), in place: forward with L (TRANS = 0) or U^T, backward with U
+// or L^T.  A thread keeps its own entry in a register and reads its row (for
+// the transposed triangles its column) of D a link of 32 entries at a time:
+// AHEAD a whole link before it is used (a block alone on its SM), else 16
+// entries at once (several blocks a SM, fewer registers).  The warp of a link
+// multiplies by the inverse through shuffles and hands its 32 results to the
+// others.
+template <typename T, int NR, int TRANS, int BWD, bool AHEAD>
+__device__ __forceinline__ void diag_solve(const T *__restrict__ D, int ld, int nb, T (&v)[NR],
+                                           T *ys) {
+  constexpr int H = AHEAD ? 32 : 16;
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const int links = (nb + 31) / 32;
+  T a[H], nx[AHEAD ? 32 : 1];
+  auto load = [&](int s, int l0, T *dst) {
+    // entries a link needs: its own warp's inverse, later warps' updates
+    const bool need = t < nb && (BWD ? w <= s : w >= s);
+#pragma unroll
+    for (int i = 0; i < H; ++i) {
+      const int l = l0 + i, o = 32 * s + l;
+      const bool on = w != s ? true
+                     : TRANS ? (BWD ? l > lane : l <= lane)
+                             : (BWD ? l >= lane : l < lane);
+      dst[i] = need && on && o < nb ? D[TRANS ? o + (long long)t * ld : t + (long long)o * ld]
+                                    : czero<T>();
+    }
+  };
+  if (AHEAD) load(BWD ? links - 1 : 0, 0, nx);
+  for (int u = 0; u < links; ++u) {
+    const int s = BWD ? links - 1 - u : u;
+    if (AHEAD) {
+#pragma unroll
+      for (int l = 0; l < H; ++l) a[l] = nx[AHEAD ? l : 0];
+      if (u + 1 < links) load(BWD ? s - 1 : s + 1, 0, nx);
+    } else {
+      load(s, 0, a);
+    }
+    T *y = ys + (u & 1) * 32 * NR;
+    if (w == s) {
+      T o[NR];
+#pragma unroll
+      for (int q = 0; q < NR; ++q) o[q] = (TRANS == BWD) ? v[q] : czero<T>();  // unit diagonal of L
+#pragma unroll
+      for (int h = 0; h < 32 / H; ++h) {
+        if (h > 0) load(s, h * H, a);
+#pragma unroll
+        for (int i = 0; i < H; ++i)
+#pragma unroll
+          for (int q = 0; q < NR; ++q) {
+            T b;
+            b.x = __shfl_sync(0xffffffffu, v[q].x, h * H + i);
+            b.y = __shfl_sync(0xffffffffu, v[q].y, h * H + i);
+            cfma(o[q], a[i], b);
+          }
+      }
+#pragma unroll
+      for (int q = 0; q < NR; ++q) {
+        v[q] = o[q];
+        y[lane * NR + q] = o[q];
+      }
+    }
+    __syncthreads();
+    if (BWD ? w < s : w > s) {
+      T o[NR];
+#pragma unroll
+      for (int q = 0; q < NR; ++q) o[q] = czero<T>();
+#pragma unroll
+      for (int h = 0; h < 32 / H; ++h) {
+        if (h > 0) load(s, h * H, a);
+#pragma unroll
+        for (int i = 0; i < H; ++i)
+#pragma unroll
+          for (int q = 0; q < NR; ++q) cfma(o[q], a[i], y[(h * H + i) * NR + q]);
+      }
+#pragma unroll
+      for (int q = 0; q < NR; ++q) v[q] = csub(v[q], o[q]);
+    }
+  }
+  __syncthreads();
+}
+
+__device__ __forceinline__ int chunks_of(int n) { return (n + SW_CHUNK - 1) / SW_CHUNK; }
+
+// One front's part of each phase: `ch` = chunk, and the number of chunks.
+template <typename T, int NR, int TRANS, bool AHEAD> struct Front {
+  const Sweep<T> &S;
+  const NodeDev N;
+  SweepSmem<T, NR> &sm;
+  const T *P, *U12;
+  T *V, *Y;
+  int m, k, r;
+  __device__ Front(const Sweep<T> &S_, int id, SweepSmem<T, NR> &sm_)
+      : S(S_), N(S_.nodes[id]), sm(sm_), m(N.m), k(N.k), r(N.m - N.k) {
+    P = S.fac + N.fac_off;
+    U12 = P + (long long)m * k;
+    V = S.V + N.vec_off;
+    Y = S.Y + N.p0;
+  }
+  // rows [a0, m) step da of the front's right-hand side: its pivots' entries
+  // (in pivot order for A) plus the children's update rows
+  __device__ void gather(int a0, int da) {
+    for (int a = a0; a < m; a += da) {
+      const int v = a >= k ? a : TRANS ? a : S.pperm[N.p0 + a];
+      const int2 c = reinterpret_cast<const int2 *>(S.src)[N.vec_off + v];
+      const int g = a < k ? S.perm[N.p0 + v] : -1;
+#pragma unroll
+      for (int q = 0; q < NR; ++q) {
+        T s = g >= 0 ? S.b[(long long)q * S.n + g] : czero<T>();
+        if (c.x >= 0) s = cadd(s, S.V[c.x + q * S.VR]);
+        if (c.y >= 0) s = cadd(s, S.V[c.y + q * S.VR]);
+        V[a + q * S.VR] = s;
+      }
+    }
+  }
+  __device__ void fwd_a(int j0) {
+    const int nb = min(SB, k - j0), i = threadIdx.x;
+    T v[NR];
+#pragma unroll
+    for (int q = 0; q < NR; ++q) v[q] = i < nb ? V[j0 + i + q * S.VR] : czero<T>();
+    diag_solve<T, NR, TRANS, 0, AHEAD>(P + j0 + (long long)j0 * m, m, nb, v, sm.in);
+    if (i < nb)
+#pragma unroll
+      for (int q = 0; q < NR; ++q) Y[j0 + i + (long long)q * S.nn] = v[q];
+  }
+  __device__ int fwd_b_chunks(int j0) const {
+    return chunks_of((TRANS ? k : m) - min(k, j0 + SB));
+  }
+  __device__ void fwd_b(int j0, int ch) {
+    const int nb = min(SB, k - j0), j1 = j0 + nb;
+    auto in = [&](int t, int q) { return Y[j0 + t + (long long)q * S.nn]; };
+    if (TRANS) {
+      T o[SW_CHUNK / SW_W][NR];
+      tile_cols<T, NR>(P + j0 + (long long)j1 * m, m, nb, ch * SW_CHUNK, k - j1, in, sm, o);
+      each_col<T, NR>(o, ch * SW_CHUNK, k - j1, [&](int c, T (&v)[NR]) {
+#pragma unroll
+        for (int q = 0; q < NR; ++q) V[j1 + c + q * S.VR] = csub(V[j1 + c + q * S.VR], v[q]);
+      });
+    } else {
+      T o[NR];
+      tile_rows<T, NR>(P + j1 + (long long)j0 * m, m, ch * SW_CHUNK, m - j1, nb, in, sm, o);
+      const int i = j1 + ch * SW_CHUNK + threadIdx.x;
+      if (threadIdx.x < 32 && i < m)
+#pragma unroll
+        for (int q = 0; q < NR; ++q) V[i + q * S.VR] = csub(V[i + q * S.VR], o[q]);
+    }
+  }
+  __device__ int fwd_u_chunks() const { return TRANS ? chunks_of(r) : 0; }
+  __device__ void fwd_u(int ch) {
+    T o[SW_CHUNK / SW_W][NR];
+    tile_cols<T, NR>(U12, k, k, ch * SW_CHUNK, r,
+                               [&](int t, int q) { return Y[t + (long long)q * S.nn]; }, sm, o);
+    each_col<T, NR>(o, ch * SW_CHUNK, r, [&](int c, T (&v)[NR]) {
+#pragma unroll
+      for (int q = 0; q < NR; ++q) V[k + c + q * S.VR] = csub(V[k + c + q * S.VR], v[q]);
+    });
+  }
+  __device__ int bwd_r_chunks() const { return r > 0 ? chunks_of(k) : 0; }
+  __device__ void bwd_r(int ch) {
+    const int *ro = S.rorig + N.r_off;
+    auto in = [&](int t, int q) { return S.x[(long long)q * S.n + ro[t]]; };
+    if (TRANS) {
+      T o[SW_CHUNK / SW_W][NR];
+      tile_cols<T, NR>(P + k, m, r, ch * SW_CHUNK, k, in, sm, o);
+      each_col<T, NR>(o, ch * SW_CHUNK, k, [&](int c, T (&v)[NR]) {
+#pragma unroll
+        for (int q = 0; q < NR; ++q) {
+          T &y = Y[c + (long long)q * S.nn];
+          y = csub(y, v[q]);
+        }
+      });
+    } else {
+      T o[NR];
+      tile_rows<T, NR>(U12, k, ch * SW_CHUNK, k, r, in, sm, o);
+      const int i = ch * SW_CHUNK + threadIdx.x;
+      if (threadIdx.x < 32 && i < k)
+#pragma unroll
+        for (int q = 0; q < NR; ++q) {
+          T &y = Y[i + (long long)q * S.nn];
+          y = csub(y, o[q]);
+        }
+    }
+  }
+  __device__ void bwd_a(int j0) {
+    const int nb = min(SB, k - j0), i = threadIdx.x;
+    T v[NR];
+#pragma unroll
+    for (int q = 0; q < NR; ++q) v[q] = i < nb ? Y[j0 + i + (long long)q * S.nn] : czero<T>();
+    diag_solve<T, NR, TRANS, 1, AHEAD>(P + j0 + (long long)j0 * m, m, nb, v, sm.in);
+    if (i >= nb) return;
+    // the pivots' solution: for the front's own products, and to x
+    const int g = S.perm[N.p0 + (TRANS ? S.pperm[N.p0 + j0 + i] : j0 + i)];
+#pragma unroll
+    for (int q = 0; q < NR; ++q) {
+      V[j0 + i + q * S.VR] = v[q];
+      S.x[(long long)q * S.n + g] = v[q];
+    }
+  }
+  __device__ int bwd_b_chunks(int j0) const { return chunks_of(j0); }
+  __device__ void bwd_b(int j0, int ch) {
+    const int nb = min(SB, k - j0);
+    auto in = [&](int t, int q) { return V[j0 + t + q * S.VR]; };
+    if (TRANS) {
+      T o[SW_CHUNK / SW_W][NR];
+      tile_cols<T, NR>(P + j0, m, nb, ch * SW_CHUNK, j0, in, sm, o);
+      each_col<T, NR>(o, ch * SW_CHUNK, j0, [&](int c, T (&v)[NR]) {
+#pragma unroll
+        for (int q = 0; q < NR; ++q) {
+          T &y = Y[c + (long long)q * S.nn];
+          y = csub(y, v[q]);
+        }
+      });
+    } else {
+      T o[NR];
+      tile_rows<T, NR>(P + (long long)j0 * m, m, ch * SW_CHUNK, j0, nb, in, sm, o);
+      const int i = ch * SW_CHUNK + threadIdx.x;
+      if (threadIdx.x < 32 && i < j0)
+#pragma unroll
+        for (int q = 0; q < NR; ++q) {
+          T &y = Y[i + (long long)q * S.nn];
+          y = csub(y, o[q]);
+        }
+    }
+  }
+};
+
+// Depths of many fronts (or of small ones): a block per front walks through
+// all its phases, one launch a depth and sweep.
+template <typename T, int NR, int TRANS>
+__global__ void __launch_bounds__(SW_T, sizeof(T) == 8 ? 3 : 2) k_sweep_fwd_front(const Sweep<T> S) {
+  __shared__ SweepSmem<T, NR> sm;
+  Front<T, NR, TRANS, false> F(S, S.list[blockIdx.x], sm);
+  F.gather(threadIdx.x, SW_T);
+  __syncthreads();
+  for (int j0 = 0; j0 < F.k; j0 += SB) {
+    F.fwd_a(j0);
+    __syncthreads();
+    for (int c = 0; c < F.fwd_b_chunks(j0); ++c) F.fwd_b(j0, c);
+    __syncthreads();
+  }
+  for (int c = 0; c < F.fwd_u_chunks(); ++c) F.fwd_u(c);
+}
+template <typename T, int NR, int TRANS>
+__global__ void __launch_bounds__(SW_T, sizeof(T) == 8 ? 3 : 2) k_sweep_bwd_front(const Sweep<T> S) {
+  __shared__ SweepSmem<T, NR> sm;
+  Front<T, NR, TRANS, false> F(S, S.list[blockIdx.x], sm);
+  for (int c = 0; c < F.bwd_r_chunks(); ++c) F.bwd_r(c);
+  __syncthreads();
+  for (int j0 = (F.k - 1) / SB * SB; j0 >= 0 && F.k > 0; j0 -= SB) {
+    F.bwd_a(j0);
+    __syncthreads();
+    for (int c = 0; c < F.bwd_b_chunks(j0); ++c) F.bwd_b(j0, c);
+    __syncthreads();
+  }
+}
+
+// Depths of few large fronts: a launch per phase, a block per (chunk, front).
+enum { PH_GATHER, PH_FWD_A, PH_FWD_B, PH_FWD_U, PH_BWD_R, PH_BWD_A, PH_BWD_B };
+template <typename T, int NR, int TRANS, int PH>
+__global__ void __launch_bounds__(SW_T) k_sweep(const Sweep<T> S, int j0) {
+  __shared__ SweepSmem<T, NR> sm;
+  Front<T, NR, TRANS, sizeof(T) == 8> F(S, S.list[blockIdx.y], sm);
+  const int ch = blockIdx.x;
+  if (PH == PH_GATHER) {
+    F.gather(ch * SW_T + threadIdx.x, gridDim.x * SW_T);
+    return;
+  }
+  if (j0 >= F.k) return;
+  if (PH == PH_FWD_A) F.fwd_a(j0);
+  if (PH == PH_FWD_B) { if (ch < F.fwd_b_chunks(j0)) F.fwd_b(j0, ch); }
+  if (PH == PH_FWD_U) { if (ch < F.fwd_u_chunks()) F.fwd_u(ch); }
+  if (PH == PH_BWD_R) { if (ch < F.bwd_r_chunks()) F.bwd_r(ch); }
+  if (PH == PH_BWD_A) F.bwd_a(j0);
+  if (PH == PH_BWD_B) { if (ch < F.bwd_b_chunks(j0)) F.bwd_b(j0, ch); }
+}
+
+// ---------------------------------------------------------------------------
+// Inverses of the 32 x 32 blocks on the diagonals of L11 and U11, in place in
+// the factor store: a warp per (front, block), by substitution, a lane per
+// column of the inverse in registers, the block in shared memory.
+constexpr int INV_WARPS = 4;
+struct InvItem { int node, j0; };
+template <typename T>
+__global__ void __launch_bounds__(INV_WARPS * 32)
+k_diag_inverse(int cnt, const InvItem *__restrict__ items, const NodeDev *__restrict__ nodes,
+               T *fac) {
+  extern __shared__ __align__(16) unsigned char inv_raw[];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int i0 = blockIdx.x * INV_WARPS + w;
+  if (i0 >= cnt) return;
+  T(*B)[33] = reinterpret_cast<T(*)[33]>(inv_raw) + 32 * w;
+  const InvItem it = items[i0];
+  const NodeDev N = nodes[it.node];
+  const int ld = N.m, n = min(32, N.k - it.j0);
+  T *D = fac + N.fac_off + it.j0 + (long long)it.j0 * ld;
+  for (int c = 0; c < 32; ++c)  // identity past the block
+    B[lane][c] = lane < n && c < n ? D[lane + (long long)c * ld]
+                                   : CT<T>::mk(lane == c ? 1.0 : 0.0, 0.0);
+  __syncwarp();
+  T x[32];
+  // column `lane` of L^-1
+#pragma unroll
+  for (int i = 0; i < 32; ++i) {
+    T s = CT<T>::mk(i == lane ? 1.0 : 0.0, 0.0);
+#pragma unroll
+    for (int l = 0; l < i; ++l) s = cfms(s, B[i][l], x[l]);
+    x[i] = s;
+  }
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 32; ++i)
+    if (i > lane && i < n) D[i + (long long)lane * ld] = x[i];
+  // column `lane` of U^-1 (the diagonal's reciprocals are shared first)
+  const T rd = cdiv(CT<T>::mk(1.0, 0.0), B[lane][lane]);
+  __syncwarp();
+  B[lane][lane] = rd;
+  __syncwarp();
+#pragma unroll
+  for (int i = 31; i >= 0; --i) {
+    T s = CT<T>::mk(i == lane ? 1.0 : 0.0, 0.0);
+#pragma unroll
+    for (int l = i + 1; l < 32; ++l) s = cfms(s, B[i][l], x[l]);
+    x[i] = cmul(s, B[i][i]);
+  }
+#pragma unroll
+  for (int i = 0; i < 32; ++i)
+    if (i <= lane && lane < n) D[i + (long long)lane * ld] = x[i];
+}
+template <typename T> constexpr size_t inv_smem() { return (size_t)INV_WARPS * 32 * 33 * sizeof(T); }

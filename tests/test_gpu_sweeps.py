@@ -1,0 +1,66 @@
+"""The triangular sweeps at the edges of their steps (256 pivots), links (32)
+and row chunks, on synthetic two-element meshes: the separator's front has s
+pivots, each leaf's a pivots and s update rows, so a and s set every size.
+Reference: a dense complex128 solve of the same matrix.  The matrix is
+diagonally dominant (condition number below 10), so the error of a backward
+stable solve is a small multiple of the unit roundoff times the front size:
+1e-12 covers complex128 (2^-53) and 1e-3 ... 1e-4 complex64 (2^-24) with n up
+to 1600; the gates are 1e-11 and 5e-4."""
+
+from __future__ import annotations
+
+import ctypes as ct
+
+import numpy as np
+import pytest
+
+from lithofem_b200 import solver
+from lithofem_b200.solver import C64, C128, DirectSolver
+
+pytestmark = pytest.mark.gpu
+GATE = {C64: 5e-4, C128: 1e-11}
+
+
+def two_elements(a: int, s: int, seed: int):
+    """(solver analysed for the mesh, dense A): element 0 owns DOFs [0, a + s),
+    element 1 owns [a, 2 a + s)."""
+    nd, n = a + s, 2 * a + s
+    dof = np.concatenate([np.arange(nd), np.arange(a, n)]).astype(np.int32)
+    mask = np.zeros((n, n), dtype=bool)
+    mask[:nd, :nd] = True
+    mask[a:, a:] = True
+    rng = np.random.default_rng(seed)
+    A = np.where(mask, rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)), 0)
+    A += np.diag(6.0 * np.sqrt(n) * np.exp(2j * np.pi * rng.random(n)))
+    J = np.nonzero(mask)[1].astype(np.int32)
+    I = np.concatenate([[0], np.cumsum(mask.sum(1))]).astype(np.int32)
+    cen = np.array([[0.0, 0.0, 0.0], [1.0, 0.0, 0.0]])
+    sv = DirectSolver(0)
+    ip = solver._ip
+    assert sv._check(solver.lib().lfsolve_analyze(
+        sv._s, n, ip(I), ip(J), len(J), 2, nd, ip(dof), cen.ctypes.data_as(ct.POINTER(ct.c_double)),
+        None, 0, 1)), sv.last_error
+    return sv, A, A[mask]
+
+
+@pytest.mark.parametrize("prec", [C64, C128], ids=["c64", "c128"])
+@pytest.mark.parametrize("a,s", [(1, 1), (31, 33), (32, 32), (33, 95), (65, 96), (255, 257),
+                                 (256, 256), (257, 1), (1, 300), (513, 255), (511, 544)])
+def test_sweeps_match_a_dense_solve(a, s, prec):
+    import torch
+    sv, A, vals = two_elements(a, s, seed=1000 * a + s)
+    n = len(A)
+    v = torch.from_numpy(vals).cuda()
+    assert sv.FactorDevice(v.data_ptr(), prec), sv.last_error
+    assert sorted(set(sv.Fronts()["k"])) == sorted({a, s})
+    rng = np.random.default_rng(n)
+    for nrhs in (1, 2, 3):
+        B = rng.standard_normal((nrhs, n)) + 1j * rng.standard_normal((nrhs, n))
+        b = torch.from_numpy(B).cuda()
+        x = torch.empty_like(b)
+        for transpose, M in ((False, A), (True, A.T)):
+            assert sv.Backsolve(nrhs, b.data_ptr(), x.data_ptr(), transpose), sv.last_error
+            want = np.linalg.solve(M, B.T).T
+            err = np.linalg.norm(x.cpu().numpy() - want) / np.linalg.norm(want)
+            assert err <= GATE[prec], (nrhs, transpose, err)
+    sv.Release()
