@@ -12,10 +12,11 @@
 //   factor (device): depth by depth from the deepest level, the fronts of a
 //     level are zeroed, receive their original entries (CSR position ->
 //     front offset map) and their children's Schur complements (extend-add),
-//     and are partially factored: P [F11 F12] = L11 [U11 U12] with partial
-//     pivoting among the front's pivot rows (library getrf on the k x m pivot
-//     row panel), L21 = F21 U11^-1 (library trsm), F22 -= L21 U12 (library
-//     gemm); the L and U blocks are copied to the factor store;
+//     and are partially factored: P F11 = L11 U11 with partial pivoting among
+//     the front's pivot rows, all fronts of the level together in own kernels
+//     (lfsolve_lu.cuh), U12 = L11^-1 P F12 and L21 = F21 U11^-1 (library
+//     trsm), F22 -= L21 U12 (library gemm); the L and U blocks are copied to
+//     the factor store;
 //   solve (device): forward and backward sweeps over the tree, each front's
 //     right-hand side gathered from the global vector and its children's
 //     update vectors (no atomics), the triangles in steps of 256 pivots with
@@ -554,7 +555,11 @@ __device__ __forceinline__ cuComplex cdiv(cuComplex a, cuComplex b) { return cuC
 __device__ __forceinline__ cuDoubleComplex cdiv(cuDoubleComplex a, cuDoubleComplex b) { return cuCdiv(a, b); }
 template <typename T> __device__ __forceinline__ T czero() { return CT<T>::mk(0.0, 0.0); }
 // a - b c
-template <typename T> __device__ __forceinline__ T cfms(T a, T b, T c) { return csub(a, cmul(b, c)); }
+template <typename T> __device__ __forceinline__ T cfms(T a, T b, T c) {
+  a.x = fma(-b.x, c.x, a.x); a.x = fma(b.y, c.y, a.x);
+  a.y = fma(-b.x, c.y, a.y); a.y = fma(-b.y, c.x, a.y);
+  return a;
+}
 
 // original entries into the fronts of one depth
 template <typename T>
@@ -665,40 +670,6 @@ __global__ void k_make_ptrs(int cnt, T *arena, long long stride, int kpad, int l
   p21[i] = F + kpad;
 }
 
-// the real part of the batched pivots / infos to the per-node arrays
-__global__ void k_take_pivots(const int *__restrict__ list, const NodeDev *__restrict__ nodes,
-                              int kpad, const int *__restrict__ piv, const int *__restrict__ inf,
-                              int *__restrict__ ipiv, int *__restrict__ info) {
-  const int i = blockIdx.x;
-  const int id = list[i];
-  const NodeDev N = nodes[id];
-  for (int t = threadIdx.x; t < N.k; t += blockDim.x) ipiv[N.p0 + t] = piv[(long long)i * kpad + t];
-  if (threadIdx.x == 0) info[id] = inf[i];
-}
-
-// batched depths: the fronts' row interchanges on their update columns,
-// item = (front, first of 32 columns)
-template <typename T>
-__global__ void k_swap_cols_batched(const EaItem *__restrict__ items,
-                                    const NodeDev *__restrict__ nodes,
-                                    const int *__restrict__ ipiv, T *__restrict__ arena) {
-  const EaItem it = items[blockIdx.x];
-  const NodeDev N = nodes[it.child];
-  const int r = N.m - N.k;
-  const int c = it.col0 + threadIdx.x;
-  if (threadIdx.x >= 32 || c >= r) return;
-  T *col = arena + N.arena_off + (long long)(N.roff + c) * N.ld;
-  const int *pv = ipiv + N.p0;
-  for (int i = 0; i < N.k; ++i) {
-    const int q = pv[i] - 1;
-    if (q != i) {
-      const T t = col[i];
-      col[i] = col[q];
-      col[q] = t;
-    }
-  }
-}
-
 // y = A x (or A^T x through the transposed positions) in FP64, a warp per
 // row; one column
 __global__ void k_spmv(int n, const int *__restrict__ I, const int *__restrict__ J,
@@ -777,12 +748,12 @@ __global__ void k_split_b(int kk, int r, const cuComplex *__restrict__ U, int ld
 // ---------------------------------------------------------------------------
 // solve kernels
 // ---------------------------------------------------------------------------
+#include "lfsolve_lu.cuh"
 #include "lfsolve_sweeps.cuh"
 
-// Pivot permutation of every front: the front's sequential row swaps
-// (ipiv, 1-based) applied to the identity, so that the swapped vector is
-// v[perm[i]] at row i and the inverse swaps put row i at perm[i]; a block
-// per front, the swaps in shared memory up to cap pivots (global beyond)
+// Pivot order of a front from the library's sequential row swaps (ipiv,
+// 1-based, applied to the identity), so that the swapped vector is v[perm[i]]
+// at row i; the swaps in shared memory up to PERM_CAP pivots (global beyond)
 constexpr int PERM_CAP = 12288;
 __device__ void perm_from_ipiv(int k, const int *__restrict__ pv, int *__restrict__ dst,
                                int *__restrict__ sp) {
@@ -802,31 +773,12 @@ __device__ void perm_from_ipiv(int k, const int *__restrict__ pv, int *__restric
   if (k <= PERM_CAP)
     for (int i = threadIdx.x; i < k; i += blockDim.x) dst[i] = sp[i];
 }
-__global__ void k_ipiv_to_perm(const NodeDev *__restrict__ nodes, const int *__restrict__ ipiv,
-                               int *__restrict__ perm) {
-  __shared__ int sp[PERM_CAP];
-  const NodeDev N = nodes[blockIdx.x];
-  perm_from_ipiv(N.k, ipiv + N.p0, perm + N.p0, sp);
-}
 // one front's permutation (k pivots at pv) into perm
 __global__ void k_ipiv_to_perm_one(int k, const int *__restrict__ pv, int *__restrict__ perm) {
   __shared__ int sp[PERM_CAP];
   perm_from_ipiv(k, pv, perm, sp);
 }
-// the factorization's row interchanges on the ncol update columns of a
-// front (A: the first k rows of column c at A + c ld): a block per column,
-// the k rows staged in shared memory, row i taking row perm[i]
-template <typename T>
-__global__ void k_perm_cols(int k, const int *__restrict__ perm, T *__restrict__ A, int ld) {
-  extern __shared__ unsigned char pc_sm[];
-  T *sv = reinterpret_cast<T *>(pc_sm);
-  T *col = A + (long long)blockIdx.x * ld;
-  for (int i = threadIdx.x; i < k; i += blockDim.x) sv[i] = col[i];
-  __syncthreads();
-  for (int i = threadIdx.x; i < k; i += blockDim.x) col[i] = sv[perm[i]];
-}
-
-// pivots that the shared-memory permutation of the update columns can take
+// pivots that k_perm_f12 can stage
 template <typename T>
 constexpr int perm_smem_max() { return (int)(160 * 1024 / sizeof(T)); }
 
@@ -969,14 +921,6 @@ inline cublasStatus_t gemm(cublasHandle_t h, cublasOperation_t ta, cublasOperati
   return cublasZgemm(h, ta, tb, m, n, k, al, A, lda, B, ldb, be, C, ldc);
 }
 
-inline cublasStatus_t getrf_batched(cublasHandle_t h, int n, cuComplex *const A[], int lda, int *piv,
-                                   int *info, int b) {
-  return cublasCgetrfBatched(h, n, A, lda, piv, info, b);
-}
-inline cublasStatus_t getrf_batched(cublasHandle_t h, int n, cuDoubleComplex *const A[], int lda,
-                                   int *piv, int *info, int b) {
-  return cublasZgetrfBatched(h, n, A, lda, piv, info, b);
-}
 inline cublasStatus_t trsm_batched(cublasHandle_t h, cublasSideMode_t sd, cublasFillMode_t ul,
                                    cublasOperation_t tr, cublasDiagType_t dg, int m, int n,
                                    const cuComplex *al, const cuComplex *const A[], int lda,
@@ -1026,18 +970,17 @@ struct lfsolve {
   std::vector<int> n_ea[2], n_co;
   std::vector<int *> d_all;               // per depth: its fronts
   int *d_rel_fac = nullptr;               // child rows in the parents' front layout
-  std::vector<EaItem *> d_sw;             // batched depths: swap items (front, columns)
-  std::vector<int> n_sw;
   void **d_ptrs = nullptr;                // batched pointer arrays (3 x max fronts)
-  int *d_bpiv = nullptr, *d_binf = nullptr;
+  LuSwaps *d_swaps = nullptr;             // a step's interchanges (max fronts of a depth)
   int *d_src = nullptr;                   // children's vector rows per vector row
   InvItem *d_inv = nullptr;               // diagonal blocks kept as inverses
   int n_inv = 0;
   // factors
   int prec = -1;
   void *d_fac = nullptr;
-  int *d_ipiv = nullptr, *d_info = nullptr;
-  int *d_pperm = nullptr;  // per-front pivot permutations (from d_ipiv)
+  int *d_info = nullptr;
+  int *d_pperm = nullptr;  // per-front pivot permutations
+  int lu_cluster[2] = {0, 0};  // largest panel cluster the device takes, per precision
   // lanes
   cudaStream_t lane[LANES] = {};
   cublasHandle_t blas[LANES] = {};
@@ -1129,17 +1072,10 @@ int ensure_uploaded(lfsolve *s) {
   s->d_co.assign(D, nullptr);
   s->n_co.assign(D, 0);
   s->d_all.assign(D, nullptr);
-  s->d_sw.assign(D, nullptr);
-  s->n_sw.assign(D, 0);
-  long long maxb = 1, maxpiv = 1;
-  for (int d = 0; d < D; ++d)
-    if (P.batched[d]) {
-      maxb = std::max<long long>(maxb, (long long)P.by_depth[d].size());
-      maxpiv = std::max<long long>(maxpiv, (long long)P.by_depth[d].size() * P.kpad[d]);
-    }
+  size_t maxb = 1;
+  for (int d = 0; d < D; ++d) maxb = std::max(maxb, P.by_depth[d].size());
   LS_CUDA(cudaMalloc((void **)&s->d_ptrs, sizeof(void *) * 3 * maxb));
-  LS_CUDA(cudaMalloc((void **)&s->d_bpiv, sizeof(int) * maxpiv));
-  LS_CUDA(cudaMalloc((void **)&s->d_binf, sizeof(int) * maxb));
+  LS_CUDA(cudaMalloc((void **)&s->d_swaps, sizeof(LuSwaps) * maxb));
   for (int d = 0; d < D; ++d) {
     if ((rc = upload(&s->d_asm_src[d], P.asm_src[d], st))) return rc;
     if ((rc = upload(&s->d_asm_dst[d], P.asm_dst[d], st))) return rc;
@@ -1157,15 +1093,6 @@ int ensure_uploaded(lfsolve *s) {
       if ((rc = upload(&s->d_ea[q][d], ea[q], st))) return rc;
       s->n_ea[q][d] = (int)ea[q].size();
     }
-    if (P.batched[d]) {
-      std::vector<EaItem> sw;
-      for (int id : P.by_depth[d]) {
-        const Node &N = P.nodes[id];
-        for (int c0 = 0; c0 < N.m - N.k; c0 += 32) sw.push_back({id, c0});
-      }
-      if ((rc = upload(&s->d_sw[d], sw, st))) return rc;
-      s->n_sw[d] = (int)sw.size();
-    }
     if ((rc = upload(&s->d_co[d], co, st))) return rc;
     s->n_co[d] = (int)co.size();
     if ((rc = upload(&s->d_all[d], P.by_depth[d], st))) return rc;
@@ -1175,15 +1102,53 @@ int ensure_uploaded(lfsolve *s) {
   return LFSOLVE_OK;
 }
 
+template <typename T>
+cudaLaunchConfig_t lu_panel_config(int fronts, int csize, int threads, cudaStream_t st,
+                                   cudaLaunchAttribute *attr) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(fronts * csize));
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = (size_t)threads * LU_NB * sizeof(T);
+  cfg.stream = st;
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = (unsigned)csize;
+  attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
+// the largest power-of-two cluster of full panel blocks that fits the device
+template <typename T> int lu_clusters(int *out) {
+  LS_CUDA(cudaFuncSetAttribute(k_lu_panel<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  LS_CUDA(cudaFuncSetAttribute(k_lu_panel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)(LU_ROWS<T> * LU_NB * sizeof(T))));
+  *out = 1;
+  for (int c = 2; c <= LU_MAX_CLUSTER; c *= 2) {
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = lu_panel_config<T>(1, c, LU_ROWS<T>, nullptr, &attr);
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k_lu_panel<T>, &cfg) != cudaSuccess || n < 1) {
+      cudaGetLastError();  // this size is not on offer
+      break;
+    }
+    *out = c;
+  }
+  return LFSOLVE_OK;
+}
+
 int ensure_lanes(lfsolve *s) {
   if (s->blas_main) return LFSOLVE_OK;
   LS_BLAS(cublasCreate(&s->blas_main));
   LS_BLAS(cublasSetStream(s->blas_main, s->stream));
   // the column permutations stage up to 160 kB of pivot rows
-  LS_CUDA(cudaFuncSetAttribute(k_perm_cols<cuComplex>,
+  LS_CUDA(cudaFuncSetAttribute(k_perm_f12<cuComplex>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-  LS_CUDA(cudaFuncSetAttribute(k_perm_cols<cuDoubleComplex>,
+  LS_CUDA(cudaFuncSetAttribute(k_perm_f12<cuDoubleComplex>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
+  int rc;
+  if ((rc = lu_clusters<cuComplex>(&s->lu_cluster[LFSOLVE_C64]))) return rc;
+  if ((rc = lu_clusters<cuDoubleComplex>(&s->lu_cluster[LFSOLVE_C128]))) return rc;
   LS_CUDA(cudaFuncSetAttribute(k_diag_inverse<cuComplex>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)inv_smem<cuComplex>()));
@@ -1307,6 +1272,114 @@ int schur_tf32x3_batched(lfsolve *s, cuComplex *arena, long long S, int ld, int 
   return LFSOLVE_OK;
 }
 
+// P F11 = L11 U11 of every front of depth d with at most cap pivots, the pivot
+// order applied to F12 too
+template <typename T>
+int lu_depth(lfsolve *s, int d, T *arena, int cap) {
+  Plan &P = s->P;
+  cudaStream_t st = s->stream;
+  const int cnt = (int)P.by_depth[d].size();
+  int kmax = 0, rmax = 0;
+  for (int id : P.by_depth[d]) {
+    const Node &N = P.nodes[id];
+    if (N.k > cap) continue;
+    kmax = std::max(kmax, N.k);
+    rmax = std::max(rmax, N.m - N.k);
+  }
+  const int *list = s->d_all[d];
+  for (int j0 = 0; j0 < kmax; j0 += LU_NB) {
+    const int rows = kmax - j0;
+    int csize = 1;
+    // the fewest blocks that hold the rows: smaller blocks in larger clusters
+    // cost more in cluster barriers than they save in issue slots (4,200 pivots
+    // in complex64: 17.7 ms with 640 rows a block, 18.4 with 320, 19.3 with 160)
+    while (csize * LU_ROWS<T> < rows) csize *= 2;
+    const int threads = ((rows + csize - 1) / csize + 31) / 32 * 32;
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = lu_panel_config<T>(cnt, csize, threads, st, &attr);
+    LS_CUDA(cudaLaunchKernelEx(&cfg, k_lu_panel<T>, list, (const NodeDev *)s->d_nodes, arena, j0,
+                               csize, cap, s->d_swaps, s->d_pperm, s->d_info));
+    const int strips = (kmax + LU_STRIP<T> - 1) / LU_STRIP<T>;
+    if (kmax > LU_NB) {
+      // rows of the update split where the strips alone leave SMs idle
+      const int groups = (rows - LU_NB + LU_STRIP_T - 1) / LU_STRIP_T;
+      const bool split = groups > 1 && (long long)cnt * ((rows - 1) / LU_STRIP<T>) < 2 * 148;
+      for (int f0 = 0; f0 < cnt; f0 += 65535) {
+        const dim3 g((unsigned)strips, (unsigned)std::min(65535, cnt - f0));
+        const int *li = list + f0;
+        const LuSwaps *sw = s->d_swaps + f0;
+        if (!split) {
+          k_lu_strip<T, 0><<<g, LU_STRIP_T, 0, st>>>(li, s->d_nodes, arena, j0, cap, sw);
+        } else {
+          k_lu_strip<T, 1><<<g, LU_STRIP_T, 0, st>>>(li, s->d_nodes, arena, j0, cap, sw);
+          k_lu_strip<T, 2><<<dim3(g.x, g.y, (unsigned)groups), LU_STRIP_T, 0, st>>>(
+              li, s->d_nodes, arena, j0, cap, sw);
+        }
+        LS_CUDA(cudaGetLastError());
+      }
+    }
+  }
+  if (kmax > 1 && rmax > 0) {
+    const size_t per = (size_t)kmax * sizeof(T);
+    const int warps = (int)std::max<size_t>(1, std::min<size_t>(8, 48 * 1024 / per));
+    for (int f0 = 0; f0 < cnt; f0 += 65535) {
+      k_perm_f12<T><<<dim3((unsigned)((rmax + warps - 1) / warps),
+                           (unsigned)std::min(65535, cnt - f0)), warps * 32, per * warps, st>>>(
+          list + f0, s->d_nodes, arena, cap, s->d_pperm, kmax);
+      LS_CUDA(cudaGetLastError());
+    }
+  }
+  return LFSOLVE_OK;
+}
+
+// The same for the fronts of depth d with more than cap pivots: the library's
+// getrf on the padded pivot block, its swaps on F12, spread over the lanes
+template <typename T>
+int lu_library(lfsolve *s, int d, T *arena, int cap) {
+  Plan &P = s->P;
+  cudaStream_t st = s->stream;
+  int lw_max = 0, kk_max = 0;
+  for (int id : P.by_depth[d]) {
+    const Node &N = P.nodes[id];
+    if (N.k <= cap) continue;
+    int lw = 0;
+    LS_BLAS(getrf_buf(s->sol[0], N.roff, N.roff, arena + N.arena_off, N.ld, &lw));
+    lw_max = std::max(lw_max, lw);
+    kk_max = std::max(kk_max, N.roff);
+  }
+  if (kk_max == 0) return LFSOLVE_OK;
+  for (int l = 0; l < LANES; ++l) {
+    if (s->work_bytes[l] < (size_t)lw_max * sizeof(T)) {
+      LS_CUDA(cudaStreamSynchronize(st));
+      if (s->work[l]) LS_CUDA(cudaFree(s->work[l]));
+      s->work_bytes[l] = (size_t)lw_max * sizeof(T);
+      LS_CUDA(cudaMalloc(&s->work[l], s->work_bytes[l]));
+    }
+    if (s->lpiv_n[l] < kk_max) {
+      LS_CUDA(cudaStreamSynchronize(st));
+      if (s->lpiv[l]) LS_CUDA(cudaFree(s->lpiv[l]));
+      s->lpiv_n[l] = kk_max;
+      LS_CUDA(cudaMalloc((void **)&s->lpiv[l], sizeof(int) * kk_max));
+    }
+  }
+  int rc = fork_lanes(s), li = 0;
+  if (rc) return rc;
+  for (int id : P.by_depth[d]) {
+    const Node &N = P.nodes[id];
+    if (N.k <= cap) continue;
+    const int l = li++ % LANES, k = N.k, r = N.m - N.k, kk = N.roff;
+    T *F = arena + N.arena_off;
+    LS_BLAS(getrf(s->sol[l], kk, kk, F, N.ld, static_cast<T *>(s->work[l]), s->lpiv[l],
+                  s->d_info + id));
+    if (r > 0)
+      k_swap_cols<T><<<(r + 127) / 128, 128, 0, s->lane[l]>>>(k, r, s->lpiv[l],
+                                                              F + (long long)kk * N.ld, N.ld);
+    k_ipiv_to_perm_one<<<1, 256, 0, s->lane[l]>>>(k, s->lpiv[l], s->d_pperm + N.p0);
+    LS_CUDA(cudaGetLastError());
+  }
+  return join_lanes(s);
+}
+
 template <typename T>
 int factor_impl(lfsolve *s, const double2 *vals) {
   Plan &P = s->P;
@@ -1322,6 +1395,10 @@ int factor_impl(lfsolve *s, const double2 *vals) {
   T *fac = static_cast<T *>(s->d_fac);
   std::vector<T *> arena(D, nullptr);
   const T one = CT<T>::mk(1.0, 0.0), mone = CT<T>::mk(-1.0, 0.0);
+  // pivot blocks beyond the panel kernel's rows go through the library
+  // (LFSOLVE_LU_MAX lowers the bound)
+  int lu_cap = std::min(LU_ROWS<T> * s->lu_cluster[s->prec], perm_smem_max<T>());
+  if (const char *e = std::getenv("LFSOLVE_LU_MAX")) lu_cap = std::min(lu_cap, std::max(0, std::atoi(e)));
   for (int d = D - 1; d >= 0; --d) {
     if (prof) LS_CUDA(cudaEventRecord(evs[2 * d], st));
     const size_t bytes = (size_t)P.arena_size[d] * sizeof(T);
@@ -1354,16 +1431,9 @@ int factor_impl(lfsolve *s, const double2 *vals) {
       T **p12 = p11 + cnt, **p21 = p12 + cnt;
       k_make_ptrs<T><<<(cnt + 127) / 128, 128, 0, st>>>(cnt, arena[d], S, kp, ld, p11, p12, p21);
       LS_CUDA(cudaGetLastError());
-      LS_BLAS(getrf_batched(s->blas_main, kp, p11, ld, s->d_bpiv, s->d_binf, cnt));
-      k_take_pivots<<<cnt, 128, 0, st>>>(s->d_all[d], s->d_nodes, kp, s->d_bpiv, s->d_binf,
-                                         s->d_ipiv, s->d_info);
-      LS_CUDA(cudaGetLastError());
+      int rcl = lu_depth<T>(s, d, arena[d], lu_cap);
+      if (rcl || (rcl = lu_library<T>(s, d, arena[d], lu_cap))) return rcl;
       if (rp > 0) {
-        if (s->n_sw[d] > 0) {
-          k_swap_cols_batched<T><<<s->n_sw[d], 32, 0, st>>>(s->d_sw[d], s->d_nodes, s->d_ipiv,
-                                                            arena[d]);
-          LS_CUDA(cudaGetLastError());
-        }
         LS_BLAS(trsm_batched(s->blas_main, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_N,
                              CUBLAS_DIAG_UNIT, kp, rp, &one, p11, ld, p12, ld, cnt));
         LS_BLAS(trsm_batched(s->blas_main, CUBLAS_SIDE_RIGHT, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_N,
@@ -1385,35 +1455,11 @@ int factor_impl(lfsolve *s, const double2 *vals) {
       if (prof) LS_CUDA(cudaEventRecord(evs[2 * d + 1], st));
       continue;
     }
-    // workspace and pivot scratch for the largest front of the depth
-    int lw_max = 0, kk_max = 0;
-    for (int id : P.by_depth[d]) {
-      const Node &N = P.nodes[id];
-      if (N.k == 0) continue;
-      int lw = 0;
-      LS_BLAS(getrf_buf(s->sol[0], N.roff, N.roff, arena[d] + N.arena_off, N.ld, &lw));
-      lw_max = std::max(lw_max, lw);
-      kk_max = std::max(kk_max, N.roff);
-    }
-    for (int l = 0; l < LANES; ++l) {
-      if (s->work_bytes[l] < (size_t)lw_max * sizeof(T)) {
-        LS_CUDA(cudaStreamSynchronize(st));
-        if (s->work[l]) LS_CUDA(cudaFree(s->work[l]));
-        s->work_bytes[l] = (size_t)lw_max * sizeof(T);
-        LS_CUDA(cudaMalloc(&s->work[l], s->work_bytes[l]));
-      }
-      if (s->lpiv_n[l] < kk_max) {
-        LS_CUDA(cudaStreamSynchronize(st));
-        if (s->lpiv[l]) LS_CUDA(cudaFree(s->lpiv[l]));
-        s->lpiv_n[l] = kk_max;
-        LS_CUDA(cudaMalloc((void **)&s->lpiv[l], sizeof(int) * kk_max));
-      }
-    }
     const int cnt = (int)P.by_depth[d].size();
     k_dummy_diag<T><<<cnt, 128, 0, st>>>(s->d_all[d], s->d_nodes, arena[d]);
     LS_CUDA(cudaGetLastError());
-    int rc = fork_lanes(s);
-    if (rc) return rc;
+    int rc = lu_depth<T>(s, d, arena[d], lu_cap);
+    if (rc || (rc = lu_library<T>(s, d, arena[d], lu_cap)) || (rc = fork_lanes(s))) return rc;
     // largest fronts first, spread over the lanes
     std::vector<int> order(P.by_depth[d]);
     std::sort(order.begin(), order.end(),
@@ -1424,24 +1470,10 @@ int factor_impl(lfsolve *s, const double2 *vals) {
       if (N.k == 0) continue;
       const int l = li++ % LANES;
       T *F = arena[d] + N.arena_off;
-      const int k = N.k, r = N.m - N.k, kk = N.roff, ld = N.ld;
-      // P F11 = L11 U11 (library getrf on the kk x kk block: the k real
-      // pivots, then dummy identity pivots that never swap), the real swaps
-      // on F12, U12 = L11^-1 P F12, L21 = F21 U11^-1, F22 -= L21 U12
-      LS_BLAS(getrf(s->sol[l], kk, kk, F, ld, static_cast<T *>(s->work[l]), s->lpiv[l],
-                    s->d_info + id));
-      LS_CUDA(cudaMemcpyAsync(s->d_ipiv + N.p0, s->lpiv[l], sizeof(int) * k,
-                              cudaMemcpyDeviceToDevice, s->lane[l]));
+      const int r = N.m - N.k, kk = N.roff, ld = N.ld;
+      // U12 = L11^-1 P F12, L21 = F21 U11^-1, F22 -= L21 U12 (dummy identity
+      // pivots k .. kk-1)
       if (r > 0) {
-        if (k <= perm_smem_max<T>()) {
-          k_ipiv_to_perm_one<<<1, 256, 0, s->lane[l]>>>(k, s->d_ipiv + N.p0, s->lpiv[l]);
-          k_perm_cols<T><<<r, 256, (size_t)k * sizeof(T), s->lane[l]>>>(
-              k, s->lpiv[l], F + (long long)kk * ld, ld);
-        } else {
-          k_swap_cols<T><<<(r + 127) / 128, 128, 0, s->lane[l]>>>(k, r, s->d_ipiv + N.p0,
-                                                                  F + (long long)kk * ld, ld);
-        }
-        LS_CUDA(cudaGetLastError());
         LS_BLAS(trsm(s->blas[l], CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_N,
                      CUBLAS_DIAG_UNIT, kk, r, &one, F, ld, F + (long long)kk * ld, ld));
         LS_BLAS(trsm(s->blas[l], CUBLAS_SIDE_RIGHT, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_N,
@@ -1879,18 +1911,13 @@ int lfsolve_factor(lfsolve *s, const void *d_vals, int prec) {
     LS_CUDA(cudaMalloc(&s->d_fac, std::max<size_t>((size_t)s->P.factor_entries * es, 256)));
     s->prec = prec;
   }
-  if (!s->d_ipiv) LS_CUDA(cudaMalloc((void **)&s->d_ipiv, sizeof(int) * std::max(1, s->P.nn)));
+  if (!s->d_pperm) LS_CUDA(cudaMalloc((void **)&s->d_pperm, sizeof(int) * std::max(1, s->P.nn)));
   if (!s->d_info) LS_CUDA(cudaMalloc((void **)&s->d_info, sizeof(int) * s->P.nodes.size()));
   LS_CUDA(cudaMemsetAsync(s->d_info, 0, sizeof(int) * s->P.nodes.size(), s->stream));
   LS_CUDA(cudaEventRecord(s->t0, s->stream));
   rc = prec == LFSOLVE_C64 ? factor_impl<cuComplex>(s, static_cast<const double2 *>(d_vals))
                            : factor_impl<cuDoubleComplex>(s, static_cast<const double2 *>(d_vals));
   if (rc) return rc;
-  // the fronts' pivot permutations for the solves' row interchanges
-  if (!s->d_pperm) LS_CUDA(cudaMalloc((void **)&s->d_pperm, sizeof(int) * std::max(1, s->P.nn)));
-  k_ipiv_to_perm<<<(unsigned)s->P.nodes.size(), 128, 0, s->stream>>>(s->d_nodes, s->d_ipiv,
-                                                                      s->d_pperm);
-  LS_CUDA(cudaGetLastError());
   LS_CUDA(cudaEventRecord(s->t1, s->stream));
   LS_CUDA(cudaStreamSynchronize(s->stream));
   LS_CUDA(cudaEventElapsedTime(&s->st.factor_ms, s->t0, s->t1));
@@ -2038,7 +2065,7 @@ void lfsolve_destroy(lfsolve *s) {
   if (s->stream) cudaStreamSynchronize(s->stream);
   free_factors(s);
   void *bufs[] = {s->d_nodes, s->d_child, s->d_rel, s->d_perm, s->d_rorig, s->d_ess, s->d_tpos,
-                  s->d_ipiv, s->d_info, s->d_V, s->d_Y, s->d_bw, s->d_src, s->d_inv, s->d_r, s->d_part, s->d_scale,
+                  s->d_info, s->d_V, s->d_Y, s->d_bw, s->d_src, s->d_inv, s->d_r, s->d_part, s->d_scale,
                   s->d_pperm};
   for (void *p : bufs)
     if (p) cudaFree(p);
@@ -2046,11 +2073,9 @@ void lfsolve_destroy(lfsolve *s) {
   for (auto *p : s->d_asm_dst) if (p) cudaFree(p);
   for (int q = 0; q < 2; ++q) for (auto *p : s->d_ea[q]) if (p) cudaFree(p);
   for (auto *p : s->d_co) if (p) cudaFree(p);
-  for (auto *p : s->d_sw) if (p) cudaFree(p);
   if (s->d_rel_fac) cudaFree(s->d_rel_fac);
   if (s->d_ptrs) cudaFree(s->d_ptrs);
-  if (s->d_bpiv) cudaFree(s->d_bpiv);
-  if (s->d_binf) cudaFree(s->d_binf);
+  if (s->d_swaps) cudaFree(s->d_swaps);
   for (auto *p : s->d_all) if (p) cudaFree(p);
   for (int l = 0; l < LANES; ++l) {
     if (s->work[l]) cudaFree(s->work[l]);
