@@ -14,9 +14,10 @@
 //     front offset map) and their children's Schur complements (extend-add),
 //     and are partially factored: P F11 = L11 U11 with partial pivoting among
 //     the front's pivot rows, all fronts of the level together in own kernels
-//     (lfsolve_lu.cuh), U12 = L11^-1 P F12 and L21 = F21 U11^-1 (library
-//     trsm), F22 -= L21 U12 (library gemm); the L and U blocks are copied to
-//     the factor store;
+//     (lfsolve_lu.cuh), U12 = L11^-1 P F12 and L21 = F21 U11^-1 in leaves of
+//     64 pivots with matrix products between them (lfsolve_trsm.cuh), F22 -=
+//     L21 U12 (library gemm; complex64 on TF32 tensor cores in split form);
+//     the L and U blocks are copied to the factor store;
 //   solve (device): forward and backward sweeps over the tree, each front's
 //     right-hand side gathered from the global vector and its children's
 //     update vectors (no atomics), the triangles in steps of 256 pivots with
@@ -90,10 +91,20 @@ inline int pad_up(int x) { return (x + FPAD - 1) / FPAD * FPAD; }
 
 constexpr int MAX_NRHS_PASS = 2;  // right-hand sides per solve pass
 constexpr int LANES = 8;          // streams (and library handles) for the fronts
-constexpr int BATCH_MIN = 128;    // depths with this many fronts use batched calls
+constexpr int BATCH_MIN = 128;    // depths with this many fronts use batched calls,
+constexpr double BATCH_PADDING = 1.25;  // and those whose fronts padding grows by less
 // complex64 fronts whose Schur update F22 -= L21 U12 has at least this many
 // complex multiply-adds use three TF32 tensor-core GEMMs on split operands
 constexpr double TF32X3_MIN_MACS = 2e9;
+// pivots one product of the large TF32 terms accumulates: the tensor cores
+// truncate as they add, so that deeper products lose accuracy (residual after
+// two corrections on a 271k-row line grating: 8.6e-10 with all pivots at once,
+// 3.0e-10 with 512, 1.0e-10 with 256, 5.6e-11 with 128; 1.3e-9 before the
+// update blocks ran in this form), and each piece reads and writes the result
+// once more (its factorization: 99.8, 100.7, 103.1, 109.6 ms)
+constexpr int TF32_PIVOTS = 512;
+// memory the split operands of fronts in flight may take
+constexpr size_t SPLIT_BYTES = (size_t)6 << 30;
 
 // ---------------------------------------------------------------------------
 // analysis (host)
@@ -361,19 +372,24 @@ int build_plan(int n, const int *I, const int *J, long long nnz, int ne, int nd,
   P.stride.assign(P.max_depth + 1, 0);
   // LFSOLVE_BATCH_MIN overrides the front count from which a depth is batched
   int batch_min = BATCH_MIN;
-  if (const char *e = std::getenv("LFSOLVE_BATCH_MIN")) batch_min = std::max(1, std::atoi(e));
+  const char *batch_env = std::getenv("LFSOLVE_BATCH_MIN");
+  if (batch_env) batch_min = std::max(1, std::atoi(batch_env));
   for (int d = 0; d <= P.max_depth; ++d) {
-    if ((int)P.by_depth[d].size() < batch_min) continue;
+    const int cnt = (int)P.by_depth[d].size();
     int kp = 0, rp = 0;
+    double real = 0.0;  // entries of the fronts as they are
     for (int s : P.by_depth[d]) {
       kp = std::max(kp, P.nodes[s].k);
       rp = std::max(rp, P.nodes[s].m - P.nodes[s].k);
+      real += (double)P.nodes[s].m * P.nodes[s].m;
     }
-    if (kp == 0) continue;
+    kp = pad_up(kp);
+    const long long ld = pad_up(kp + rp);
+    const bool alike = !batch_env && cnt > 1 && (double)ld * ld * cnt <= BATCH_PADDING * real;
+    if (kp == 0 || (cnt < batch_min && !alike)) continue;
     P.batched[d] = 1;
-    P.kpad[d] = pad_up(kp);
-    P.rpad[d] = pad_up(P.kpad[d] + rp) - P.kpad[d];
-    const long long ld = P.kpad[d] + P.rpad[d];
+    P.kpad[d] = kp;
+    P.rpad[d] = (int)ld - kp;
     P.stride[d] = align_up(ld * ld);
   }
   long long fac = 0, roff = 0, vec = 0;
@@ -658,18 +674,6 @@ __global__ void k_dummy_diag(const int *__restrict__ list, const NodeDev *__rest
     F[i + (long long)i * N.ld] = CT<T>::mk(1.0, 0.0);
 }
 
-// pointer arrays of a batched depth: F11, F12 and F21 of front i
-template <typename T>
-__global__ void k_make_ptrs(int cnt, T *arena, long long stride, int kpad, int ld, T **p11,
-                            T **p12, T **p21) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= cnt) return;
-  T *F = arena + (long long)i * stride;
-  p11[i] = F;
-  p12[i] = F + (long long)kpad * ld;
-  p21[i] = F + kpad;
-}
-
 // y = A x (or A^T x through the transposed positions) in FP64, a warp per
 // row; one column
 __global__ void k_spmv(int n, const int *__restrict__ I, const int *__restrict__ J,
@@ -692,64 +696,12 @@ __global__ void k_spmv(int n, const int *__restrict__ I, const int *__restrict__
   if (lane == 0) y[row] = make_double2(ar, ai);
 }
 
-// Error-compensated TF32 operands of F22 -= L21 U12 (complex64, kk pivot
-// columns incl. dummies, r update rows), in a real formulation: the complex
-// product is the real product of A (2r x 2kk; column 2j is column j of L21
-// read as (re, im) float pairs, column 2j + 1 that of i L21) and B (2kk x r;
-// U12 read as (re, im) pairs), and the real result read as floats is F22
-// itself (leading dimension 2 ld).  Every float x is split as hi = its TF32
-// rounding (cvt.rna.tf32.f32, 10 mantissa bits) and lo = x - hi;
-// hi hi' + hi lo' + lo hi' carries the product to about 2^-22 relative on
-// TF32 tensor cores.  A is stored as [hi | lo] (2r x 4kk, leading dimension
-// lda), B as [lo ; hi] (4kk x r, leading dimension 4kk), so that two GEMMs
-// ([hi | lo] [lo ; hi] and hi hi) cover the three products.
-__device__ __forceinline__ float tf32_round(float x) {
-  unsigned u;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(x));
-  return __uint_as_float(u);
-}
-__device__ __forceinline__ void tf32_split(cuComplex v, float2 &h, float2 &l) {
-  h = make_float2(tf32_round(v.x), tf32_round(v.y));
-  l = make_float2(v.x - h.x, v.y - h.y);
-}
-// nb fronts of the same shape: front f's block at L + f sL, its operand at
-// A + f sA (B + f sB)
-__global__ void k_split_a(int r, int kk, const cuComplex *__restrict__ L, int ld,
-                          float *__restrict__ A, int lda, int nb, long long sL, long long sA) {
-  const long long per = (long long)r * kk, n = per * nb, lo_off = (long long)2 * kk * lda;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
-       t += (long long)gridDim.x * blockDim.x) {
-    const long long f = t / per, u = t - f * per;
-    const int i = (int)(u % r), j = (int)(u / r);
-    float2 h, l;
-    tf32_split(L[f * sL + i + (long long)j * ld], h, l);
-    float *c0 = A + f * sA + (long long)(2 * j) * lda + 2 * i;  // column 2j; 2j + 1 one lda on
-    *reinterpret_cast<float2 *>(c0) = h;
-    *reinterpret_cast<float2 *>(c0 + lda) = make_float2(-h.y, h.x);
-    *reinterpret_cast<float2 *>(c0 + lo_off) = l;
-    *reinterpret_cast<float2 *>(c0 + lo_off + lda) = make_float2(-l.y, l.x);
-  }
-}
-__global__ void k_split_b(int kk, int r, const cuComplex *__restrict__ U, int ld,
-                          float *__restrict__ B, int nb, long long sU, long long sB) {
-  const long long per = (long long)kk * r, n = per * nb;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
-       t += (long long)gridDim.x * blockDim.x) {
-    const long long f = t / per, u = t - f * per;
-    const int j = (int)(u % kk), c = (int)(u / kk);
-    float2 h, l;
-    tf32_split(U[f * sU + j + (long long)c * ld], h, l);
-    float *col = B + f * sB + (long long)c * 4 * kk;
-    *reinterpret_cast<float2 *>(col + 2 * j) = l;
-    *reinterpret_cast<float2 *>(col + 2 * kk + 2 * j) = h;
-  }
-}
-
 // ---------------------------------------------------------------------------
 // solve kernels
 // ---------------------------------------------------------------------------
 #include "lfsolve_lu.cuh"
 #include "lfsolve_sweeps.cuh"
+#include "lfsolve_trsm.cuh"
 
 // Pivot order of a front from the library's sequential row swaps (ipiv,
 // 1-based, applied to the identity), so that the swapped vector is v[perm[i]]
@@ -899,40 +851,6 @@ inline cusolverStatus_t getrf(cusolverDnHandle_t h, int m, int n, cuComplex *A, 
 inline cusolverStatus_t getrf(cusolverDnHandle_t h, int m, int n, cuDoubleComplex *A, int lda, cuDoubleComplex *w, int *ip, int *info) {
   return cusolverDnZgetrf(h, m, n, A, lda, w, ip, info);
 }
-inline cublasStatus_t trsm(cublasHandle_t h, cublasSideMode_t sd, cublasFillMode_t ul, cublasOperation_t tr,
-                           cublasDiagType_t dg, int m, int n, const cuComplex *al, const cuComplex *A, int lda,
-                           cuComplex *B, int ldb) {
-  return cublasCtrsm(h, sd, ul, tr, dg, m, n, al, A, lda, B, ldb);
-}
-inline cublasStatus_t trsm(cublasHandle_t h, cublasSideMode_t sd, cublasFillMode_t ul, cublasOperation_t tr,
-                           cublasDiagType_t dg, int m, int n, const cuDoubleComplex *al, const cuDoubleComplex *A,
-                           int lda, cuDoubleComplex *B, int ldb) {
-  return cublasZtrsm(h, sd, ul, tr, dg, m, n, al, A, lda, B, ldb);
-}
-inline cublasStatus_t gemm(cublasHandle_t h, cublasOperation_t ta, cublasOperation_t tb, int m, int n, int k,
-                           const cuComplex *al, const cuComplex *A, int lda, const cuComplex *B, int ldb,
-                           const cuComplex *be, cuComplex *C, int ldc) {
-  return cublasCgemm(h, ta, tb, m, n, k, al, A, lda, B, ldb, be, C, ldc);
-}
-inline cublasStatus_t gemm(cublasHandle_t h, cublasOperation_t ta, cublasOperation_t tb, int m, int n, int k,
-                           const cuDoubleComplex *al, const cuDoubleComplex *A, int lda,
-                           const cuDoubleComplex *B, int ldb, const cuDoubleComplex *be, cuDoubleComplex *C,
-                           int ldc) {
-  return cublasZgemm(h, ta, tb, m, n, k, al, A, lda, B, ldb, be, C, ldc);
-}
-
-inline cublasStatus_t trsm_batched(cublasHandle_t h, cublasSideMode_t sd, cublasFillMode_t ul,
-                                   cublasOperation_t tr, cublasDiagType_t dg, int m, int n,
-                                   const cuComplex *al, const cuComplex *const A[], int lda,
-                                   cuComplex *const B[], int ldb, int b) {
-  return cublasCtrsmBatched(h, sd, ul, tr, dg, m, n, al, A, lda, B, ldb, b);
-}
-inline cublasStatus_t trsm_batched(cublasHandle_t h, cublasSideMode_t sd, cublasFillMode_t ul,
-                                   cublasOperation_t tr, cublasDiagType_t dg, int m, int n,
-                                   const cuDoubleComplex *al, const cuDoubleComplex *const A[],
-                                   int lda, cuDoubleComplex *const B[], int ldb, int b) {
-  return cublasZtrsmBatched(h, sd, ul, tr, dg, m, n, al, A, lda, B, ldb, b);
-}
 inline cublasStatus_t gemm_sb(cublasHandle_t h, int m, int n, int k, const cuComplex *al,
                               const cuComplex *A, int lda, long long sa, const cuComplex *B, int ldb,
                               long long sb, const cuComplex *be, cuComplex *C, int ldc, long long sc,
@@ -970,11 +888,10 @@ struct lfsolve {
   std::vector<int> n_ea[2], n_co;
   std::vector<int *> d_all;               // per depth: its fronts
   int *d_rel_fac = nullptr;               // child rows in the parents' front layout
-  void **d_ptrs = nullptr;                // batched pointer arrays (3 x max fronts)
   LuSwaps *d_swaps = nullptr;             // a step's interchanges (max fronts of a depth)
   int *d_src = nullptr;                   // children's vector rows per vector row
   InvItem *d_inv = nullptr;               // diagonal blocks kept as inverses
-  int n_inv = 0;
+  std::vector<int> inv_at;                // per depth: its first entry (and the end)
   // factors
   int prec = -1;
   void *d_fac = nullptr;
@@ -988,13 +905,11 @@ struct lfsolve {
   void *work[LANES] = {};
   size_t work_bytes[LANES] = {};
   cudaEvent_t ev_main = nullptr, ev_lane[LANES] = {};
-  // the front workspace comes from a private pool that keeps its memory
-  // between depths and factorizations (a pool that hands memory back to the
-  // driver at every synchronize re-maps gigabytes per depth)
-  cudaMemPool_t pool = nullptr;
-  // 3xTF32 Schur updates of large complex64 fronts: per-lane split buffers
-  void *split[LANES] = {};
-  size_t split_bytes[LANES] = {};
+  // front workspace, kept between factorizations: the fronts of the even and
+  // of the odd depths (a depth reads its children's from the other one), and
+  // the split operands of the fronts in flight
+  void *d_arena[2] = {nullptr, nullptr}, *d_split = nullptr;
+  size_t arena_bytes[2] = {0, 0}, split_bytes = 0;
   int *lpiv[LANES] = {};  // pivots of a front's padded pivot block
   int lpiv_n[LANES] = {};
   cublasHandle_t blas_main = nullptr;
@@ -1052,7 +967,6 @@ int ensure_uploaded(lfsolve *s) {
   if ((rc = upload(&s->d_tpos, P.tpos, st))) return rc;
   // per vector row: the child rows that the forward sweep adds to it
   std::vector<int> src(2 * (size_t)P.vec_rows, -1);
-  std::vector<InvItem> inv;
   for (int i = 0; i < ns; ++i) {
     const Node &N = P.nodes[i];
     for (int q = 0; q < N.nchild; ++q) {
@@ -1060,11 +974,16 @@ int ensure_uploaded(lfsolve *s) {
       for (int t = 0; t < C.m - C.k; ++t)
         src[2 * (size_t)(N.vec_off + P.rel[C.r_off + t]) + q] = (int)(C.vec_off + C.k + t);
     }
-    for (int j0 = 0; j0 < N.k; j0 += 32) inv.push_back({i, j0});
+  }
+  std::vector<InvItem> inv;
+  s->inv_at.assign(1, 0);
+  for (const auto &fronts : P.by_depth) {
+    for (int i : fronts)
+      for (int j0 = 0; j0 < P.nodes[i].k; j0 += 32) inv.push_back({i, j0});
+    s->inv_at.push_back((int)inv.size());
   }
   if ((rc = upload(&s->d_src, src, st))) return rc;
   if ((rc = upload(&s->d_inv, inv, st))) return rc;
-  s->n_inv = (int)inv.size();
   const int D = P.max_depth + 1;
   s->d_asm_src.assign(D, nullptr);
   s->d_asm_dst.assign(D, nullptr);
@@ -1074,7 +993,6 @@ int ensure_uploaded(lfsolve *s) {
   s->d_all.assign(D, nullptr);
   size_t maxb = 1;
   for (int d = 0; d < D; ++d) maxb = std::max(maxb, P.by_depth[d].size());
-  LS_CUDA(cudaMalloc((void **)&s->d_ptrs, sizeof(void *) * 3 * maxb));
   LS_CUDA(cudaMalloc((void **)&s->d_swaps, sizeof(LuSwaps) * maxb));
   for (int d = 0; d < D; ++d) {
     if ((rc = upload(&s->d_asm_src[d], P.asm_src[d], st))) return rc;
@@ -1149,6 +1067,16 @@ int ensure_lanes(lfsolve *s) {
   int rc;
   if ((rc = lu_clusters<cuComplex>(&s->lu_cluster[LFSOLVE_C64]))) return rc;
   if ((rc = lu_clusters<cuDoubleComplex>(&s->lu_cluster[LFSOLVE_C128]))) return rc;
+  LS_CUDA(cudaFuncSetAttribute(k_leaf<cuComplex, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)sizeof(LeafSmem<cuComplex>)));
+  LS_CUDA(cudaFuncSetAttribute(k_leaf<cuComplex, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)sizeof(LeafSmem<cuComplex>)));
+  LS_CUDA(cudaFuncSetAttribute(k_leaf<cuDoubleComplex, true>,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)sizeof(LeafSmem<cuDoubleComplex>)));
+  LS_CUDA(cudaFuncSetAttribute(k_leaf<cuDoubleComplex, false>,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)sizeof(LeafSmem<cuDoubleComplex>)));
   LS_CUDA(cudaFuncSetAttribute(k_diag_inverse<cuComplex>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)inv_smem<cuComplex>()));
@@ -1164,13 +1092,6 @@ int ensure_lanes(lfsolve *s) {
     LS_CUDA(cudaEventCreateWithFlags(&s->ev_lane[l], cudaEventDisableTiming));
   }
   LS_CUDA(cudaEventCreateWithFlags(&s->ev_main, cudaEventDisableTiming));
-  cudaMemPoolProps props = {};
-  props.allocType = cudaMemAllocationTypePinned;
-  props.location.type = cudaMemLocationTypeDevice;
-  props.location.id = s->dev;
-  LS_CUDA(cudaMemPoolCreate(&s->pool, &props));
-  unsigned long long keep = ~0ull;
-  LS_CUDA(cudaMemPoolSetAttribute(s->pool, cudaMemPoolAttrReleaseThreshold, &keep));
   LS_CUDA(cudaEventCreate(&s->t0));
   LS_CUDA(cudaEventCreate(&s->t1));
   return LFSOLVE_OK;
@@ -1210,65 +1131,131 @@ template <> bool use_tf32x3<cuComplex>(lfsolve *) {
   return !(e && e[0] == '0');
 }
 
-// F22 -= L21 U12 of one complex64 front (at F, leading dimension ld, kk
-// pivot rows incl. dummies, r update rows) on lane l: split both operands,
-// then the two TF32 tensor-core GEMMs of the real formulation with FP32
-// accumulation into F22
-int schur_tf32x3(lfsolve *s, int l, cuComplex *F, int ld, int kk, int r) {
-  const long long lda = ((2LL * r + 31) / 32) * 32;
-  const size_t na = (size_t)lda * 4 * kk, need = (na + (size_t)4 * kk * r) * sizeof(float);
-  if (s->split_bytes[l] < need) {
-    LS_CUDA(cudaStreamSynchronize(s->lane[l]));
-    if (s->split[l]) LS_CUDA(cudaFree(s->split[l]));
-    LS_CUDA(cudaMalloc(&s->split[l], need));
-    s->split_bytes[l] = need;
+// C -= A B of every front of a group over the k pivots from p0: in the front's
+// own precision, or from split operands (rows from i0 of a left operand As,
+// columns from j0 of a right operand Bs) as two real TF32 products with FP32
+// accumulation
+template <typename T>
+int group_product(cublasHandle_t h, const Group<T> &G, int m, int n, int p0, int k, const T *A,
+                  const T *B, T *C, const Operand &As, int i0, const Operand &Bs, int j0) {
+  if (As.p) {
+    const float mone = -1.f, one = 1.f;
+    // nk pivots from q0; per = 4 or 2 columns a pivot
+    auto product = [&](int per, const float *a, const float *b, int q0, int nk) {
+      return cublasGemmStridedBatchedEx(
+          h, CUBLAS_OP_N, CUBLAS_OP_N, 2 * m, n, per * nk, &mone,
+          a + 2 * i0 + (long long)per * q0 * As.ld, CUDA_R_32F, (int)As.ld, per * As.n,
+          b + per * (q0 + (long long)j0 * G.kk), CUDA_R_32F, per * G.kk, per * Bs.n, &one, C,
+          CUDA_R_32F, 2 * G.ld, 2 * G.S, G.cnt, CUBLAS_COMPUTE_32F_FAST_TF32, CUBLAS_GEMM_DEFAULT);
+    };
+    LS_BLAS(product(4, As.both(0), Bs.both(0), p0, k));
+    for (int q0 = p0; q0 < p0 + k; q0 += TF32_PIVOTS)
+      LS_BLAS(product(2, As.hi(G.cnt, 0), Bs.hi(G.cnt, 0), q0, std::min(TF32_PIVOTS, p0 + k - q0)));
+    return LFSOLVE_OK;
   }
-  float *A = static_cast<float *>(s->split[l]);
-  float *B = A + na;
-  const int g = grid_for((long long)r * kk, 256);
-  k_split_a<<<g, 256, 0, s->lane[l]>>>(r, kk, F + kk, ld, A, (int)lda, 1, 0, 0);
-  LS_CUDA(cudaGetLastError());
-  k_split_b<<<g, 256, 0, s->lane[l]>>>(kk, r, F + (long long)kk * ld, ld, B, 1, 0, 0);
-  LS_CUDA(cudaGetLastError());
-  const float mone = -1.f, one = 1.f;
-  float *C = reinterpret_cast<float *>(F + kk + (long long)kk * ld);
-  LS_BLAS(cublasGemmEx(s->blas[l], CUBLAS_OP_N, CUBLAS_OP_N, 2 * r, r, 4 * kk, &mone, A,
-                       CUDA_R_32F, (int)lda, B, CUDA_R_32F, 4 * kk, &one, C, CUDA_R_32F, 2 * ld,
-                       CUBLAS_COMPUTE_32F_FAST_TF32, CUBLAS_GEMM_DEFAULT));
-  LS_BLAS(cublasGemmEx(s->blas[l], CUBLAS_OP_N, CUBLAS_OP_N, 2 * r, r, 2 * kk, &mone, A,
-                       CUDA_R_32F, (int)lda, B + 2 * kk, CUDA_R_32F, 4 * kk, &one, C,
-                       CUDA_R_32F, 2 * ld, CUBLAS_COMPUTE_32F_FAST_TF32, CUBLAS_GEMM_DEFAULT));
+  const T mone = CT<T>::mk(-1.0, 0.0), one = CT<T>::mk(1.0, 0.0);
+  LS_BLAS(gemm_sb(h, m, n, k, &mone, A, G.ld, G.S, B, G.ld, G.S, &one, C, G.ld, G.S, G.cnt));
   return LFSOLVE_OK;
 }
 
-// The same for all cnt fronts of a batched depth (uniform kk x r blocks,
-// front stride S entries, leading dimension ld) on the main stream, the
-// split operands in the solver's pool for the duration of the call
-int schur_tf32x3_batched(lfsolve *s, cuComplex *arena, long long S, int ld, int kk, int r,
-                         int cnt) {
-  cudaStream_t st = s->stream;
-  const long long lda = ((2LL * r + 31) / 32) * 32;
-  const long long na = lda * 4 * kk, nbf = 4LL * kk * r;
-  float *A = nullptr;
-  LS_CUDA(cudaMallocFromPoolAsync((void **)&A, sizeof(float) * (size_t)(na + nbf) * cnt, s->pool,
-                                  st));
-  float *B = A + na * cnt;
-  const int g = grid_for((long long)r * kk * cnt, 256);
-  k_split_a<<<g, 256, 0, st>>>(r, kk, arena + kk, ld, A, (int)lda, cnt, S, na);
-  LS_CUDA(cudaGetLastError());
-  k_split_b<<<g, 256, 0, st>>>(kk, r, arena + (long long)kk * ld, ld, B, cnt, S, nbf);
-  LS_CUDA(cudaGetLastError());
-  const float mone = -1.f, one = 1.f;
-  float *C = reinterpret_cast<float *>(arena + kk + (long long)kk * ld);
-  LS_BLAS(cublasGemmStridedBatchedEx(s->blas_main, CUBLAS_OP_N, CUBLAS_OP_N, 2 * r, r, 4 * kk,
-                                     &mone, A, CUDA_R_32F, (int)lda, na, B, CUDA_R_32F, 4 * kk,
-                                     nbf, &one, C, CUDA_R_32F, 2 * ld, 2 * S, cnt,
-                                     CUBLAS_COMPUTE_32F_FAST_TF32, CUBLAS_GEMM_DEFAULT));
-  LS_BLAS(cublasGemmStridedBatchedEx(s->blas_main, CUBLAS_OP_N, CUBLAS_OP_N, 2 * r, r, 2 * kk,
-                                     &mone, A, CUDA_R_32F, (int)lda, na, B + 2 * kk, CUDA_R_32F,
-                                     4 * kk, nbf, &one, C, CUDA_R_32F, 2 * ld, 2 * S, cnt,
-                                     CUBLAS_COMPUTE_32F_FAST_TF32, CUBLAS_GEMM_DEFAULT));
-  LS_CUDA(cudaFreeAsync(A, st));
+// one side of the update blocks: leaves and the products between them
+template <typename T, bool LEFT>
+int group_side(cudaStream_t st, cublasHandle_t h, const Group<T> &G) {
+  const int nl = (G.kk + LEAF - 1) / LEAF, ld = G.ld;
+  for (int i = 1; i <= nl; ++i) {
+    k_leaf<T, LEFT><<<dim3((unsigned)((G.r + LEAF_C - 1) / LEAF_C), (unsigned)G.cnt), LEAF_T,
+                      sizeof(LeafSmem<T>), st>>>(G, (i - 1) * LEAF);
+    LS_CUDA(cudaGetLastError());
+    if (i == nl) break;
+    const int t = i & -i, p0 = (i - t) * LEAF, pk = t * LEAF, q0 = i * LEAF;
+    const int qn = std::min(G.kk, std::min(nl, i + t) * LEAF) - q0;
+    T *F = G.F;
+    int rc;
+    if (LEFT)
+      rc = group_product<T>(h, G, qn, G.r, p0, pk, F + q0 + (long long)p0 * ld,
+                            F + p0 + (long long)G.kk * ld, F + q0 + (long long)G.kk * ld, G.AF, q0,
+                            G.BU, 0);
+    else
+      rc = group_product<T>(h, G, G.r, qn, p0, pk, F + G.kk + (long long)p0 * ld,
+                            F + p0 + (long long)q0 * ld, F + G.kk + (long long)q0 * ld, G.AL, 0,
+                            G.BF, q0);
+    if (rc) return rc;
+  }
+  return LFSOLVE_OK;
+}
+
+// floats of split operands a front needs
+inline size_t split_floats(int kk, int r) {
+  return (size_t)18 * kk * ((size_t)kk + r);
+}
+
+// U12, L21 and F22 -= L21 U12 of a group; buf: its products on TF32 tensor
+// cores with the split operands there (cnt x split_floats), null: in T
+template <typename T>
+int group_update(cudaStream_t st, cublasHandle_t h, Group<T> G, float *buf) {
+  if (buf) {
+    float *at = buf;
+    auto operand = [&](long long ld, long long n) {
+      const Operand o{at, ld, n};
+      at += 6 * n * G.cnt;
+      return o;
+    };
+    G.AF = operand(2LL * G.kk, 2LL * G.kk * G.kk);
+    G.BF = operand(0, (long long)G.kk * G.kk);
+    G.AL = operand(2LL * G.r, 2LL * G.r * G.kk);
+    G.BU = operand(0, (long long)G.kk * G.r);
+    const int nl = (G.kk + LEAF - 1) / LEAF;
+    if (nl > 1) {
+      k_split_f11<T><<<dim3((unsigned)(nl - 1), (unsigned)(nl - 1), (unsigned)G.cnt), LEAF_T, 0, st>>>(G);
+      LS_CUDA(cudaGetLastError());
+    }
+  }
+  int rc = group_side<T, true>(st, h, G);
+  if (rc || (rc = group_side<T, false>(st, h, G))) return rc;
+  T *F = G.F;
+  rc = group_product<T>(h, G, G.r, G.r, 0, G.kk, F + G.kk, F + (long long)G.kk * G.ld,
+                        F + G.kk + (long long)G.kk * G.ld, G.AL, 0, G.BU, 0);
+  return rc;
+}
+
+// how a depth's fronts are taken: step fronts at once (batched), or one a lane
+// on `lanes` streams; which go through split operands, and the floats of them
+// in flight
+struct DepthPlan { int step = 1, lanes = 1; size_t floats = 0; };
+template <typename T> bool front_split(lfsolve *s, double r, double kk, double cnt) {
+  return use_tf32x3<T>(s) && r * r * kk * cnt >= tf32x3_min();
+}
+template <typename T> DepthPlan depth_plan(lfsolve *s, int d) {
+  const Plan &P = s->P;
+  DepthPlan Q;
+  if (P.batched[d]) {
+    const int cnt = (int)P.by_depth[d].size(), kp = P.kpad[d], rp = P.rpad[d];
+    Q.step = std::min(cnt, 32768);
+    if (rp > 0 && front_split<T>(s, rp, kp, cnt)) {
+      const size_t per = split_floats(kp, rp);
+      Q.step = (int)std::max<size_t>(1, std::min<size_t>(Q.step, SPLIT_BYTES / (4 * per)));
+      Q.floats = per * Q.step;
+    }
+    return Q;
+  }
+  size_t need = 0;
+  for (int id : P.by_depth[d]) {
+    const Node &N = P.nodes[id];
+    if (N.k > 0 && N.m > N.k && front_split<T>(s, N.ld - N.roff, N.roff, 1))
+      need = std::max(need, split_floats(N.roff, N.ld - N.roff));
+  }
+  Q.lanes = need ? (int)std::max<size_t>(1, std::min<size_t>(LANES, SPLIT_BYTES / (4 * need))) : LANES;
+  Q.floats = need * Q.lanes;
+  return Q;
+}
+
+int ensure_bytes(void **p, size_t *have, size_t need) {
+  if (*have >= need) return LFSOLVE_OK;
+  if (*p) LS_CUDA(cudaFree(*p));
+  *p = nullptr;
+  *have = 0;
+  LS_CUDA(cudaMalloc(p, need));
+  *have = need;
   return LFSOLVE_OK;
 }
 
@@ -1393,8 +1380,20 @@ int factor_impl(lfsolve *s, const double2 *vals) {
     for (auto &e : evs) LS_CUDA(cudaEventCreate(&e));
   }
   T *fac = static_cast<T *>(s->d_fac);
-  std::vector<T *> arena(D, nullptr);
-  const T one = CT<T>::mk(1.0, 0.0), mone = CT<T>::mk(-1.0, 0.0);
+  std::vector<DepthPlan> plan(D);
+  size_t need[2] = {256, 256}, floats = 0;
+  for (int d = 0; d < D; ++d) {
+    plan[d] = depth_plan<T>(s, d);
+    need[d & 1] = std::max(need[d & 1], (size_t)P.arena_size[d] * sizeof(T));
+    floats = std::max(floats, plan[d].floats);
+  }
+  int rc;
+  for (int i = 0; i < 2; ++i)
+    if ((rc = ensure_bytes(&s->d_arena[i], &s->arena_bytes[i], need[i]))) return rc;
+  if (floats && (rc = ensure_bytes(&s->d_split, &s->split_bytes, floats * sizeof(float)))) return rc;
+  float *split_buf = static_cast<float *>(s->d_split);
+  std::vector<T *> arena(D);
+  for (int d = 0; d < D; ++d) arena[d] = static_cast<T *>(s->d_arena[d & 1]);
   // pivot blocks beyond the panel kernel's rows go through the library
   // (LFSOLVE_LU_MAX lowers the bound)
   int lu_cap = std::min(LU_ROWS<T> * s->lu_cluster[s->prec], perm_smem_max<T>());
@@ -1402,7 +1401,6 @@ int factor_impl(lfsolve *s, const double2 *vals) {
   for (int d = D - 1; d >= 0; --d) {
     if (prof) LS_CUDA(cudaEventRecord(evs[2 * d], st));
     const size_t bytes = (size_t)P.arena_size[d] * sizeof(T);
-    LS_CUDA(cudaMallocFromPoolAsync((void **)&arena[d], std::max<size_t>(bytes, 256), s->pool, st));
     LS_CUDA(cudaMemsetAsync(arena[d], 0, bytes, st));
     const long long na = (long long)P.asm_src[d].size();
     if (na > 0) {
@@ -1417,89 +1415,49 @@ int factor_impl(lfsolve *s, const double2 *vals) {
                                                          arena[d + 1], arena[d]);
           LS_CUDA(cudaGetLastError());
         }
-      LS_CUDA(cudaFreeAsync(arena[d + 1], st));
-      arena[d + 1] = nullptr;
-    }
-    if (P.batched[d]) {
-      // the whole depth at once on the uniform padded layout
-      const int cnt = (int)P.by_depth[d].size();
-      const int kp = P.kpad[d], rp = P.rpad[d], ld = kp + rp;
-      const long long S = P.stride[d];
-      k_dummy_diag<T><<<cnt, 128, 0, st>>>(s->d_all[d], s->d_nodes, arena[d]);
-      LS_CUDA(cudaGetLastError());
-      T **p11 = reinterpret_cast<T **>(s->d_ptrs);
-      T **p12 = p11 + cnt, **p21 = p12 + cnt;
-      k_make_ptrs<T><<<(cnt + 127) / 128, 128, 0, st>>>(cnt, arena[d], S, kp, ld, p11, p12, p21);
-      LS_CUDA(cudaGetLastError());
-      int rcl = lu_depth<T>(s, d, arena[d], lu_cap);
-      if (rcl || (rcl = lu_library<T>(s, d, arena[d], lu_cap))) return rcl;
-      if (rp > 0) {
-        LS_BLAS(trsm_batched(s->blas_main, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_N,
-                             CUBLAS_DIAG_UNIT, kp, rp, &one, p11, ld, p12, ld, cnt));
-        LS_BLAS(trsm_batched(s->blas_main, CUBLAS_SIDE_RIGHT, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_N,
-                             CUBLAS_DIAG_NON_UNIT, rp, kp, &one, p11, ld, p21, ld, cnt));
-        if (use_tf32x3<T>(s) && (double)rp * rp * kp * cnt >= tf32x3_min()) {
-          int rc3 = schur_tf32x3_batched(s, reinterpret_cast<cuComplex *>(arena[d]), S, ld, kp, rp,
-                                         cnt);
-          if (rc3) return rc3;
-        } else {
-          LS_BLAS(gemm_sb(s->blas_main, rp, rp, kp, &mone, arena[d] + kp, ld, S,
-                          arena[d] + (long long)kp * ld, ld, S, &one,
-                          arena[d] + kp + (long long)kp * ld, ld, S, cnt));
-        }
-      }
-      if (s->n_co[d] > 0) {
-        k_copy_out<T><<<s->n_co[d], 256, 0, st>>>(s->d_co[d], s->d_nodes, arena[d], fac);
-        LS_CUDA(cudaGetLastError());
-      }
-      if (prof) LS_CUDA(cudaEventRecord(evs[2 * d + 1], st));
-      continue;
     }
     const int cnt = (int)P.by_depth[d].size();
     k_dummy_diag<T><<<cnt, 128, 0, st>>>(s->d_all[d], s->d_nodes, arena[d]);
     LS_CUDA(cudaGetLastError());
-    int rc = lu_depth<T>(s, d, arena[d], lu_cap);
-    if (rc || (rc = lu_library<T>(s, d, arena[d], lu_cap)) || (rc = fork_lanes(s))) return rc;
-    // largest fronts first, spread over the lanes
-    std::vector<int> order(P.by_depth[d]);
-    std::sort(order.begin(), order.end(),
-              [&](int a, int b) { return P.nodes[a].m > P.nodes[b].m; });
-    int li = 0;
-    for (int id : order) {
-      const Node &N = P.nodes[id];
-      if (N.k == 0) continue;
-      const int l = li++ % LANES;
-      T *F = arena[d] + N.arena_off;
-      const int r = N.m - N.k, kk = N.roff, ld = N.ld;
-      // U12 = L11^-1 P F12, L21 = F21 U11^-1, F22 -= L21 U12 (dummy identity
-      // pivots k .. kk-1)
-      if (r > 0) {
-        LS_BLAS(trsm(s->blas[l], CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_N,
-                     CUBLAS_DIAG_UNIT, kk, r, &one, F, ld, F + (long long)kk * ld, ld));
-        LS_BLAS(trsm(s->blas[l], CUBLAS_SIDE_RIGHT, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_N,
-                     CUBLAS_DIAG_NON_UNIT, r, kk, &one, F, ld, F + kk, ld));
-        if (use_tf32x3<T>(s) && (double)r * r * kk >= tf32x3_min()) {
-          int rc3 = schur_tf32x3(s, l, reinterpret_cast<cuComplex *>(F), ld, kk, r);
-          if (rc3) return rc3;
-        } else {
-          LS_BLAS(gemm(s->blas[l], CUBLAS_OP_N, CUBLAS_OP_N, r, r, kk, &mone, F + kk, ld,
-                       F + (long long)kk * ld, ld, &one, F + kk + (long long)kk * ld, ld));
-        }
-      }
+    if ((rc = lu_depth<T>(s, d, arena[d], lu_cap)) || (rc = lu_library<T>(s, d, arena[d], lu_cap))) return rc;
+    // the update blocks and the sweeps read the diagonal blocks as inverses
+    const int ni = s->inv_at[d + 1] - s->inv_at[d];
+    if (ni > 0) {
+      k_diag_inverse<T><<<(ni + INV_WARPS - 1) / INV_WARPS, INV_WARPS * 32, inv_smem<T>(), st>>>(
+          ni, s->d_inv + s->inv_at[d], s->d_nodes, arena[d]);
+      LS_CUDA(cudaGetLastError());
     }
-    if ((rc = join_lanes(s))) return rc;
+    const DepthPlan &Q = plan[d];
+    if (P.batched[d]) {  // the uniform padded layout
+      const int kp = P.kpad[d], rp = P.rpad[d];
+      for (int f0 = 0; rp > 0 && f0 < cnt; f0 += Q.step) {
+        const Group<T> G{arena[d] + f0 * P.stride[d], P.stride[d], std::min(Q.step, cnt - f0), kp, rp,
+                         kp + rp, {}, {}, {}, {}};
+        if ((rc = group_update<T>(st, s->blas_main, G, Q.floats ? split_buf : nullptr))) return rc;
+      }
+    } else {
+      // largest fronts first, spread over the lanes
+      std::vector<int> order;
+      for (int id : P.by_depth[d])
+        if (P.nodes[id].k > 0 && P.nodes[id].m > P.nodes[id].k) order.push_back(id);
+      std::sort(order.begin(), order.end(),
+                [&](int a, int b) { return P.nodes[a].m > P.nodes[b].m; });
+      if ((rc = fork_lanes(s))) return rc;
+      int li = 0;
+      for (int id : order) {
+        const Node &N = P.nodes[id];
+        const int l = li++ % Q.lanes, kk = N.roff, r = N.ld - N.roff;
+        const Group<T> G{arena[d] + N.arena_off, 0, 1, kk, r, N.ld, {}, {}, {}, {}};
+        float *buf = front_split<T>(s, r, kk, 1) ? split_buf + l * (Q.floats / Q.lanes) : nullptr;
+        if ((rc = group_update<T>(s->lane[l], s->blas[l], G, buf))) return rc;
+      }
+      if ((rc = join_lanes(s))) return rc;
+    }
     if (s->n_co[d] > 0) {
       k_copy_out<T><<<s->n_co[d], 256, 0, st>>>(s->d_co[d], s->d_nodes, arena[d], fac);
       LS_CUDA(cudaGetLastError());
     }
     if (prof) LS_CUDA(cudaEventRecord(evs[2 * d + 1], st));
-  }
-  LS_CUDA(cudaFreeAsync(arena[0], st));
-  // the sweeps read the diagonal blocks as inverses
-  if (s->n_inv > 0) {
-    k_diag_inverse<T><<<(s->n_inv + INV_WARPS - 1) / INV_WARPS, INV_WARPS * 32, inv_smem<T>(), st>>>(
-        s->n_inv, s->d_inv, s->d_nodes, fac);
-    LS_CUDA(cudaGetLastError());
   }
   if (prof) {
     LS_CUDA(cudaStreamSynchronize(st));
@@ -1810,6 +1768,17 @@ int gmres_column(lfsolve *s, const int *d_I, const int *d_J, const double2 *vals
   return LFSOLVE_OK;
 }
 
+void free_workspace(lfsolve *s) {
+  for (int i = 0; i < 2; ++i) {
+    if (s->d_arena[i]) cudaFree(s->d_arena[i]);
+    s->d_arena[i] = nullptr;
+    s->arena_bytes[i] = 0;
+  }
+  if (s->d_split) cudaFree(s->d_split);
+  s->d_split = nullptr;
+  s->split_bytes = 0;
+}
+
 void free_factors(lfsolve *s) {
   if (s->d_fac) cudaFree(s->d_fac);
   s->d_fac = nullptr;
@@ -2052,10 +2021,7 @@ int lfsolve_release_factors(lfsolve *s) {
   if (!s) return fail(LFSOLVE_ERR_ARG, "NULL solver");
   cudaSetDevice(s->dev);
   free_factors(s);
-  if (s->pool) {
-    if (s->stream) cudaStreamSynchronize(s->stream);
-    cudaMemPoolTrimTo(s->pool, 0);
-  }
+  free_workspace(s);
   return LFSOLVE_OK;
 }
 
@@ -2064,6 +2030,7 @@ void lfsolve_destroy(lfsolve *s) {
   cudaSetDevice(s->dev);
   if (s->stream) cudaStreamSynchronize(s->stream);
   free_factors(s);
+  free_workspace(s);
   void *bufs[] = {s->d_nodes, s->d_child, s->d_rel, s->d_perm, s->d_rorig, s->d_ess, s->d_tpos,
                   s->d_info, s->d_V, s->d_Y, s->d_bw, s->d_src, s->d_inv, s->d_r, s->d_part, s->d_scale,
                   s->d_pperm};
@@ -2074,12 +2041,10 @@ void lfsolve_destroy(lfsolve *s) {
   for (int q = 0; q < 2; ++q) for (auto *p : s->d_ea[q]) if (p) cudaFree(p);
   for (auto *p : s->d_co) if (p) cudaFree(p);
   if (s->d_rel_fac) cudaFree(s->d_rel_fac);
-  if (s->d_ptrs) cudaFree(s->d_ptrs);
   if (s->d_swaps) cudaFree(s->d_swaps);
   for (auto *p : s->d_all) if (p) cudaFree(p);
   for (int l = 0; l < LANES; ++l) {
     if (s->work[l]) cudaFree(s->work[l]);
-    if (s->split[l]) cudaFree(s->split[l]);
     if (s->lpiv[l]) cudaFree(s->lpiv[l]);
     if (s->blas[l]) cublasDestroy(s->blas[l]);
     if (s->sol[l]) cusolverDnDestroy(s->sol[l]);
@@ -2087,7 +2052,6 @@ void lfsolve_destroy(lfsolve *s) {
     if (s->ev_lane[l]) cudaEventDestroy(s->ev_lane[l]);
   }
   if (s->blas_main) cublasDestroy(s->blas_main);
-  if (s->pool) cudaMemPoolDestroy(s->pool);
   if (s->ev_main) cudaEventDestroy(s->ev_main);
   if (s->t0) cudaEventDestroy(s->t0);
   if (s->t1) cudaEventDestroy(s->t1);

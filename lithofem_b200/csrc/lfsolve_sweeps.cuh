@@ -435,15 +435,15 @@ __global__ void __launch_bounds__(SW_T) k_sweep(const Sweep<T> S, int j0) {
 }
 
 // ---------------------------------------------------------------------------
-// Inverses of the 32 x 32 blocks on the diagonals of L11 and U11, in place in
-// the factor store: a warp per (front, block), by substitution, a lane per
+// Inverses of the 32 x 32 blocks on the diagonals of L11 and U11 of a depth's
+// fronts, in place: a warp per (front, block), by substitution, a lane per
 // column of the inverse in registers, the block in shared memory.
 constexpr int INV_WARPS = 4;
 struct InvItem { int node, j0; };
 template <typename T>
 __global__ void __launch_bounds__(INV_WARPS * 32)
 k_diag_inverse(int cnt, const InvItem *__restrict__ items, const NodeDev *__restrict__ nodes,
-               T *fac) {
+               T *arena) {
   extern __shared__ __align__(16) unsigned char inv_raw[];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int i0 = blockIdx.x * INV_WARPS + w;
@@ -451,8 +451,8 @@ k_diag_inverse(int cnt, const InvItem *__restrict__ items, const NodeDev *__rest
   T(*B)[33] = reinterpret_cast<T(*)[33]>(inv_raw) + 32 * w;
   const InvItem it = items[i0];
   const NodeDev N = nodes[it.node];
-  const int ld = N.m, n = min(32, N.k - it.j0);
-  T *D = fac + N.fac_off + it.j0 + (long long)it.j0 * ld;
+  const int ld = N.ld, n = min(32, N.k - it.j0);
+  T *D = arena + N.arena_off + it.j0 + (long long)it.j0 * ld;
   for (int c = 0; c < 32; ++c)  // identity past the block
     B[lane][c] = lane < n && c < n ? D[lane + (long long)c * ld]
                                    : CT<T>::mk(lane == c ? 1.0 : 0.0, 0.0);

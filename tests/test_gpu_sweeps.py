@@ -70,6 +70,16 @@ def test_pivot_blocks_beyond_the_panel(prec, monkeypatch):
     check(*two_elements(70, 33, seed=3, shuffled=True), 70, 33, prec, (1,))
 
 
+@pytest.mark.parametrize("batch_min", ["1", "1000"], ids=["batched", "per-front"])
+@pytest.mark.parametrize("a,s", [(16, 16), (64, 65), (65, 64), (130, 70), (600, 49)])
+def test_split_products(a, s, batch_min, monkeypatch):
+    """The update blocks' leaves of 64 pivots and split TF32 products, forced
+    on small fronts (2^-22 a product: inside the complex64 gate)."""
+    monkeypatch.setenv("LFSOLVE_TF32X3_MIN", "1")
+    monkeypatch.setenv("LFSOLVE_BATCH_MIN", batch_min)
+    check(*two_elements(a, s, seed=5 * a + s, shuffled=True), a, s, C64, (1,))
+
+
 def check(sv, A, vals, a, s, prec, columns):
     import torch
     n = len(A)
