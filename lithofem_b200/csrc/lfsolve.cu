@@ -90,6 +90,7 @@ constexpr int FPAD = 16;
 inline int pad_up(int x) { return (x + FPAD - 1) / FPAD * FPAD; }
 
 constexpr int MAX_NRHS_PASS = 2;  // right-hand sides per solve pass
+constexpr int SWEEP_BLOCKS = 1184;  // blocks of a sweep phase that fill the GPU (8 a SM)
 constexpr int LANES = 8;          // streams (and library handles) for the fronts
 constexpr int BATCH_MIN = 128;    // depths with this many fronts use batched calls,
 constexpr double BATCH_PADDING = 1.25;  // and those whose fronts padding grows by less
@@ -914,8 +915,8 @@ struct lfsolve {
   int lpiv_n[LANES] = {};
   cublasHandle_t blas_main = nullptr;
   // solve scratch
-  void *d_V = nullptr, *d_Y = nullptr, *d_bw = nullptr;
-  size_t V_bytes = 0, Y_bytes = 0, bw_bytes = 0;
+  void *d_V = nullptr, *d_Y = nullptr, *d_bw = nullptr, *d_part_y = nullptr;
+  size_t V_bytes = 0, Y_bytes = 0, bw_bytes = 0, part_y_bytes = 0;
   double2 *d_r = nullptr, *d_x64 = nullptr;
   size_t r_bytes = 0;
   double *d_part = nullptr, *d_scale = nullptr;
@@ -1481,17 +1482,25 @@ int factor_impl(lfsolve *s, const double2 *vals) {
   return LFSOLVE_OK;
 }
 
-// one launch of a phase over the fronts of a depth, at most nch chunks each
+// one launch of a phase over the fronts of a depth, at most nch chunks each in
+// nz parts; it may start while the launch before it is still running
 template <typename T, int NR, int TRANS, int PH>
-int sweep_phase(const Sweep<T> &S, int nch, int fronts, int j0, cudaStream_t st) {
+int sweep_phase(const Sweep<T> &S, int nch, int fronts, int j0, cudaStream_t st, int nz = 1) {
   if (nch <= 0) return LFSOLVE_OK;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
   // grid.y holds 65,535 fronts
   for (int f0 = 0; f0 < fronts; f0 += 65535) {
     Sweep<T> P = S;
     P.list = S.list + f0;
-    k_sweep<T, NR, TRANS, PH><<<dim3((unsigned)nch, (unsigned)std::min(65535, fronts - f0)), SW_T, 0,
-                                st>>>(P, j0);
-    LS_CUDA(cudaGetLastError());
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)nch, (unsigned)std::min(65535, fronts - f0), (unsigned)nz);
+    cfg.blockDim = dim3(SW_T);
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    LS_CUDA(cudaLaunchKernelEx(&cfg, k_sweep<T, NR, TRANS, PH>, P, j0));
   }
   return LFSOLVE_OK;
 }
@@ -1509,7 +1518,7 @@ int solve_pass(lfsolve *s, const T *b, T *x) {
   const int D = P.max_depth + 1, n = P.n;
   Sweep<T> S{s->d_nodes, nullptr, static_cast<const T *>(s->d_fac), s->d_perm, s->d_pperm,
              s->d_rorig, s->d_src, static_cast<T *>(s->d_V), static_cast<T *>(s->d_Y),
-             P.vec_rows, P.nn, n, b, x};
+             P.vec_rows, P.nn, n, b, x, static_cast<T *>(s->d_part_y)};
   // LFSOLVE_PROFILE set: per-depth device times of both sweeps
   const bool prof = std::getenv("LFSOLVE_PROFILE") != nullptr;
   std::vector<cudaEvent_t> evs;
@@ -1553,7 +1562,15 @@ int solve_pass(lfsolve *s, const T *b, T *x) {
       k_sweep_bwd_front<T, NR, TRANS><<<cnt, SW_T, 0, st>>>(S);
       LS_CUDA(cudaGetLastError());
     } else if (Z.k > 0) {
-      if (Z.r > 0 && (rc = sweep_phase<T, NR, TRANS, PH_BWD_R>(S, chunks(Z.k), cnt, 0, st))) return rc;
+      if (Z.r > 0) {
+        // the update rows in parts where the pivot chunks alone are too few
+        // blocks (or rows) to keep HBM busy, at least 256 rows each
+        const int nz = std::max(1, std::min(std::min(SW_PARTS, Z.r / 256),
+                                            SWEEP_BLOCKS / (chunks(Z.k) * cnt)));
+        if ((rc = sweep_phase<T, NR, TRANS, PH_BWD_R>(S, chunks(Z.k), cnt, 0, st, nz))) return rc;
+        if (nz > 1 && (rc = sweep_phase<T, NR, TRANS, PH_BWD_S>(S, (Z.k + SW_T - 1) / SW_T, cnt, nz, st)))
+          return rc;
+      }
       for (int j0 = (Z.k - 1) / SB * SB; j0 >= 0; j0 -= SB) {
         if ((rc = sweep_phase<T, NR, TRANS, PH_BWD_A>(S, 1, cnt, j0, st))) return rc;
         if ((rc = sweep_phase<T, NR, TRANS, PH_BWD_B>(S, chunks(j0), cnt, j0, st))) return rc;
@@ -1596,6 +1613,7 @@ int ensure_solve_scratch(lfsolve *s, size_t es) {
     LS_CUDA(cudaMalloc(&s->d_Y, Y));
     s->Y_bytes = Y;
   }
+  if (int rc = ensure_bytes(&s->d_part_y, &s->part_y_bytes, Y * SW_PARTS)) return rc;
   const size_t bw = (size_t)P.n * 2 * MAX_NRHS_PASS * es;  // b and x in the factor precision
   if (s->bw_bytes < bw) {
     if (s->d_bw) LS_CUDA(cudaFree(s->d_bw));
@@ -2032,7 +2050,7 @@ void lfsolve_destroy(lfsolve *s) {
   free_factors(s);
   free_workspace(s);
   void *bufs[] = {s->d_nodes, s->d_child, s->d_rel, s->d_perm, s->d_rorig, s->d_ess, s->d_tpos,
-                  s->d_info, s->d_V, s->d_Y, s->d_bw, s->d_src, s->d_inv, s->d_r, s->d_part, s->d_scale,
+                  s->d_info, s->d_V, s->d_Y, s->d_part_y, s->d_bw, s->d_src, s->d_inv, s->d_r, s->d_part, s->d_scale,
                   s->d_pperm};
   for (void *p : bufs)
     if (p) cudaFree(p);

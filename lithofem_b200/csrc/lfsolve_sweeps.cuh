@@ -51,16 +51,41 @@ template <typename T> struct Sweep {
   int nn, n;
   const T *b;               // right-hand side (n a column, original numbering)
   T *x;                     // solution
+  T *part;                  // partial sums of the backward sweep's first product
 };
+constexpr int SW_PARTS = 8;   // at most so many a pivot
 
 template <typename T, int NR> struct SweepSmem {
   T in[SW_TILE * NR];
   T red[SW_W * SW_CHUNK * NR];
 };
 
+// acc[q] += sum over c = c0, c0 + step, ... < c1 of A[row, c] in[c], A at the
+// lane's row; 128 bytes a lane in flight
+template <typename T, int NR>
+__device__ __forceinline__ void row_dot(const T *__restrict__ Ar, long long ld, int c0, int c1, int step,
+                                        const T *in, T (&acc)[NR]) {
+  constexpr int U = 128 / sizeof(T);
+  int c = c0;
+  for (; c + (U - 1) * step < c1; c += U * step) {
+    T a[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) a[u] = Ar[(c + u * step) * ld];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int q = 0; q < NR; ++q) cfma(acc[q], a[u], in[(c + u * step) * NR + q]);
+  }
+#pragma unroll 4
+  for (; c < c1; c += step) {
+    const T a = Ar[c * ld];
+#pragma unroll
+    for (int q = 0; q < NR; ++q) cfma(acc[q], a, in[c * NR + q]);
+  }
+}
+
 // out[q] (threads 0..31: row r0 + lane) = sum over c < nc of A[row, c] in(c, q),
-// the warps taking every SW_W-th column, eight loads in flight a thread;
-// reduced in warp order
+// the warps taking every SW_W-th column; reduced in warp order
 template <typename T, int NR, class In>
 __device__ __forceinline__ void tile_rows(const T *__restrict__ A, int ld, int r0, int nr, int nc,
                                           In in, SweepSmem<T, NR> &sm, T (&out)[NR]) {
@@ -75,21 +100,7 @@ __device__ __forceinline__ void tile_rows(const T *__restrict__ A, int ld, int r
     __syncthreads();
     for (int t = threadIdx.x; t < tn * NR; t += SW_T) sm.in[t] = in(t0 + t / NR, t % NR);
     __syncthreads();
-    int c = w;
-    for (; c + 7 * SW_W < tn; c += 8 * SW_W) {
-      T a[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) a[u] = Ar[(long long)(t0 + c + u * SW_W) * ld];
-#pragma unroll
-      for (int u = 0; u < 8; ++u)
-#pragma unroll
-        for (int q = 0; q < NR; ++q) cfma(acc[q], a[u], sm.in[(c + u * SW_W) * NR + q]);
-    }
-    for (; c < tn; c += SW_W) {
-      const T a = Ar[(long long)(t0 + c) * ld];
-#pragma unroll
-      for (int q = 0; q < NR; ++q) cfma(acc[q], a, sm.in[c * NR + q]);
-    }
+    row_dot<T, NR>(Ar + (long long)t0 * ld, ld, w, tn, SW_W, sm.in, acc);
   }
   __syncthreads();
 #pragma unroll
@@ -103,6 +114,40 @@ __device__ __forceinline__ void tile_rows(const T *__restrict__ A, int ld, int r
       for (int v = 1; v < SW_W; ++v) s = cadd(s, sm.red[(v * SW_CHUNK + lane) * NR + q]);
       out[q] = s;
     }
+}
+
+// The same for all nr rows of A, a warp per 32 rows and no reduction, where
+// there are enough of them (else the warps split the columns): store(row, out)
+template <typename T, int NR, class In, class F>
+__device__ __forceinline__ void all_rows(const T *__restrict__ A, int ld, int nr, int nc, In in,
+                                         SweepSmem<T, NR> &sm, F store) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nch = (nr + SW_CHUNK - 1) / SW_CHUNK;
+  if (nch < 6) {
+    for (int ch = 0; ch < nch; ++ch) {
+      T o[NR];
+      tile_rows<T, NR>(A, ld, ch * SW_CHUNK, nr, nc, in, sm, o);
+      const int i = ch * SW_CHUNK + threadIdx.x;
+      if (threadIdx.x < 32 && i < nr) store(i, o);
+    }
+    return;
+  }
+  for (int c0 = 0; c0 < nch; c0 += SW_W) {
+    const int row = (c0 + w) * SW_CHUNK + lane;
+    const T *Ar = A + min(row, nr - 1);
+    T acc[NR];
+#pragma unroll
+    for (int q = 0; q < NR; ++q) acc[q] = czero<T>();
+    for (int t0 = 0; t0 < nc; t0 += SW_TILE) {
+      const int tn = min(SW_TILE, nc - t0);
+      if (c0 == 0 || nc > SW_TILE) {
+        __syncthreads();
+        for (int t = threadIdx.x; t < tn * NR; t += SW_T) sm.in[t] = in(t0 + t / NR, t % NR);
+        __syncthreads();
+      }
+      if (c0 + w < nch) row_dot<T, NR>(Ar + (long long)t0 * ld, ld, 0, tn, 1, sm.in, acc);
+    }
+    if (row < nr) store(row, acc);
+  }
 }
 
 // out[u][q] (every lane of warp w: column c0 + w + SW_W u) = sum over rows i < nr
@@ -305,6 +350,22 @@ template <typename T, int NR, int TRANS, bool AHEAD> struct Front {
         for (int q = 0; q < NR; ++q) V[i + q * S.VR] = csub(V[i + q * S.VR], o[q]);
     }
   }
+  __device__ void fwd_b_all(int j0) {
+    if (TRANS) {
+      for (int c = 0; c < fwd_b_chunks(j0); ++c) fwd_b(j0, c);
+      return;
+    }
+    const int nb = min(SB, k - j0), j1 = j0 + nb;
+    all_rows<T, NR>(P + j1 + (long long)j0 * m, m, m - j1, nb,
+                    [&](int t, int q) { return Y[j0 + t + (long long)q * S.nn]; }, sm,
+                    [&](int i, T (&o)[NR]) {
+#pragma unroll
+                      for (int q = 0; q < NR; ++q) {
+                        T &v = V[j1 + i + q * S.VR];
+                        v = csub(v, o[q]);
+                      }
+                    });
+  }
   __device__ int fwd_u_chunks() const { return TRANS ? chunks_of(r) : 0; }
   __device__ void fwd_u(int ch) {
     T o[SW_CHUNK / SW_W][NR];
@@ -315,30 +376,56 @@ template <typename T, int NR, int TRANS, bool AHEAD> struct Front {
       for (int q = 0; q < NR; ++q) V[k + c + q * S.VR] = csub(V[k + c + q * S.VR], v[q]);
     });
   }
+  // Y -= U12 x_R (L21^T x_R): part z of nz of the update rows; one part
+  // subtracts, several leave their sums in S.part for bwd_s
   __device__ int bwd_r_chunks() const { return r > 0 ? chunks_of(k) : 0; }
-  __device__ void bwd_r(int ch) {
-    const int *ro = S.rorig + N.r_off;
+  __device__ void bwd_r(int ch, int z, int nz) {
+    const int per = (r + nz - 1) / nz, t0 = min(r, z * per), rn = min(r, t0 + per) - t0;
+    const int *ro = S.rorig + N.r_off + t0;
     auto in = [&](int t, int q) { return S.x[(long long)q * S.n + ro[t]]; };
+    auto put = [&](int i, T (&o)[NR]) {
+#pragma unroll
+      for (int q = 0; q < NR; ++q) {
+        T &y = Y[i + (long long)q * S.nn];
+        if (nz == 1) y = csub(y, o[q]);
+        else S.part[((long long)z * NR + q) * S.nn + N.p0 + i] = o[q];
+      }
+    };
     if (TRANS) {
       T o[SW_CHUNK / SW_W][NR];
-      tile_cols<T, NR>(P + k, m, r, ch * SW_CHUNK, k, in, sm, o);
-      each_col<T, NR>(o, ch * SW_CHUNK, k, [&](int c, T (&v)[NR]) {
-#pragma unroll
-        for (int q = 0; q < NR; ++q) {
-          T &y = Y[c + (long long)q * S.nn];
-          y = csub(y, v[q]);
-        }
-      });
+      tile_cols<T, NR>(P + k + t0, m, rn, ch * SW_CHUNK, k, in, sm, o);
+      each_col<T, NR>(o, ch * SW_CHUNK, k, put);
     } else {
       T o[NR];
-      tile_rows<T, NR>(U12, k, ch * SW_CHUNK, k, r, in, sm, o);
+      tile_rows<T, NR>(U12 + (long long)t0 * k, k, ch * SW_CHUNK, k, rn, in, sm, o);
       const int i = ch * SW_CHUNK + threadIdx.x;
-      if (threadIdx.x < 32 && i < k)
+      if (threadIdx.x < 32 && i < k) put(i, o);
+    }
+  }
+  __device__ void bwd_r_all() {
+    if (r == 0) return;
+    if (TRANS) {
+      for (int c = 0; c < bwd_r_chunks(); ++c) bwd_r(c, 0, 1);
+      return;
+    }
+    const int *ro = S.rorig + N.r_off;
+    all_rows<T, NR>(U12, k, k, r, [&](int t, int q) { return S.x[(long long)q * S.n + ro[t]]; }, sm,
+                    [&](int i, T (&o)[NR]) {
 #pragma unroll
-        for (int q = 0; q < NR; ++q) {
-          T &y = Y[i + (long long)q * S.nn];
-          y = csub(y, o[q]);
-        }
+                      for (int q = 0; q < NR; ++q) {
+                        T &y = Y[i + (long long)q * S.nn];
+                        y = csub(y, o[q]);
+                      }
+                    });
+  }
+  __device__ void bwd_s(int i, int nz) {
+    if (i >= k || r == 0) return;
+#pragma unroll
+    for (int q = 0; q < NR; ++q) {
+      T &y = Y[i + (long long)q * S.nn];
+      T v = y;
+      for (int z = 0; z < nz; ++z) v = csub(v, S.part[((long long)z * NR + q) * S.nn + N.p0 + i]);
+      y = v;
     }
   }
   __device__ void bwd_a(int j0) {
@@ -382,6 +469,30 @@ template <typename T, int NR, int TRANS, bool AHEAD> struct Front {
         }
     }
   }
+  __device__ void bwd_b_all(int j0) {
+    if (TRANS) {
+      for (int c = 0; c < bwd_b_chunks(j0); ++c) bwd_b(j0, c);
+      return;
+    }
+    const int nb = min(SB, k - j0);
+    if (j0 == 0) return;
+    all_rows<T, NR>(P + (long long)j0 * m, m, j0, nb,
+                    [&](int t, int q) { return V[j0 + t + q * S.VR]; }, sm,
+                    [&](int i, T (&o)[NR]) {
+#pragma unroll
+                      for (int q = 0; q < NR; ++q) {
+                        T &y = Y[i + (long long)q * S.nn];
+                        y = csub(y, o[q]);
+                      }
+                    });
+  }
+  // lines of the matrix a phase's block will read, asked for from HBM while
+  // the phase before is still under way
+  __device__ void ahead(const T *A, int ld, int rows, int cols) {
+    for (int c = threadIdx.x; c < cols; c += SW_T)
+      for (int b = 0; b < rows * (int)sizeof(T); b += 128)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char *>(A + (long long)c * ld) + b));
+  }
 };
 
 // Depths of many fronts (or of small ones): a block per front walks through
@@ -395,7 +506,7 @@ __global__ void __launch_bounds__(SW_T, sizeof(T) == 8 ? 3 : 2) k_sweep_fwd_fron
   for (int j0 = 0; j0 < F.k; j0 += SB) {
     F.fwd_a(j0);
     __syncthreads();
-    for (int c = 0; c < F.fwd_b_chunks(j0); ++c) F.fwd_b(j0, c);
+    F.fwd_b_all(j0);
     __syncthreads();
   }
   for (int c = 0; c < F.fwd_u_chunks(); ++c) F.fwd_u(c);
@@ -404,37 +515,68 @@ template <typename T, int NR, int TRANS>
 __global__ void __launch_bounds__(SW_T, sizeof(T) == 8 ? 3 : 2) k_sweep_bwd_front(const Sweep<T> S) {
   __shared__ SweepSmem<T, NR> sm;
   Front<T, NR, TRANS, false> F(S, S.list[blockIdx.x], sm);
-  for (int c = 0; c < F.bwd_r_chunks(); ++c) F.bwd_r(c);
+  F.bwd_r_all();
   __syncthreads();
   for (int j0 = (F.k - 1) / SB * SB; j0 >= 0 && F.k > 0; j0 -= SB) {
     F.bwd_a(j0);
     __syncthreads();
-    for (int c = 0; c < F.bwd_b_chunks(j0); ++c) F.bwd_b(j0, c);
+    F.bwd_b_all(j0);
     __syncthreads();
   }
 }
 
 // Depths of few large fronts: a launch per phase, a block per (chunk, front).
-enum { PH_GATHER, PH_FWD_A, PH_FWD_B, PH_FWD_U, PH_BWD_R, PH_BWD_A, PH_BWD_B };
+// The launches overlap (programmatic dependent launch): a block asks for its
+// part of the factors, which no phase writes, and only then waits for the
+// phase before.
+enum { PH_GATHER, PH_FWD_A, PH_FWD_B, PH_FWD_U, PH_BWD_R, PH_BWD_S, PH_BWD_A, PH_BWD_B };
 template <typename T, int NR, int TRANS, int PH>
 __global__ void __launch_bounds__(SW_T) k_sweep(const Sweep<T> S, int j0) {
   __shared__ SweepSmem<T, NR> sm;
+  cudaTriggerProgrammaticLaunchCompletion();
   Front<T, NR, TRANS, sizeof(T) == 8> F(S, S.list[blockIdx.y], sm);
-  const int ch = blockIdx.x;
-  if (PH == PH_GATHER) {
-    F.gather(ch * SW_T + threadIdx.x, gridDim.x * SW_T);
-    return;
+  const int ch = blockIdx.x, r0 = ch * SW_CHUNK;
+  const int nb = min(SB, F.k - j0), j1 = j0 + nb;
+  const bool on = PH == PH_GATHER || PH == PH_BWD_S ? true
+                  : j0 >= F.k                       ? false
+                  : PH == PH_FWD_B                  ? ch < F.fwd_b_chunks(j0)
+                  : PH == PH_FWD_U                  ? ch < F.fwd_u_chunks()
+                  : PH == PH_BWD_R                  ? ch < F.bwd_r_chunks()
+                  : PH == PH_BWD_B                  ? ch < F.bwd_b_chunks(j0)
+                                                    : true;
+  if (on) {
+    if (PH == PH_FWD_A || PH == PH_BWD_A) {
+      // the triangle: the lower (L) or upper (U) half of each of its columns
+      const bool lower = (TRANS != 0) == (PH == PH_BWD_A);
+      for (int c = threadIdx.x; c < nb; c += SW_T) {
+        const T *D = F.P + j0 + (long long)(j0 + c) * F.m;
+        for (int i = lower ? c & ~15 : 0; i < (lower ? nb : c + 1); i += 128 / (int)sizeof(T))
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(D + i));
+      }
+    }
+    const int n0 = min(SW_CHUNK, (TRANS ? (PH == PH_FWD_U ? F.r : PH == PH_FWD_B ? F.k - j1 : j0)
+                                        : (PH == PH_FWD_B ? F.m - j1 : j0)) - r0);
+    if (PH == PH_FWD_B) {
+      if (TRANS) F.ahead(F.P + j0 + (long long)(j1 + r0) * F.m, F.m, nb, n0);
+      else F.ahead(F.P + j1 + r0 + (long long)j0 * F.m, F.m, n0, nb);
+    }
+    if (PH == PH_BWD_B) {
+      if (TRANS) F.ahead(F.P + j0 + (long long)r0 * F.m, F.m, nb, n0);
+      else F.ahead(F.P + r0 + (long long)j0 * F.m, F.m, n0, nb);
+    }
   }
-  if (j0 >= F.k) return;
+  cudaGridDependencySynchronize();
+  if (PH == PH_GATHER) F.gather(ch * SW_T + threadIdx.x, gridDim.x * SW_T);
+  if (PH == PH_BWD_S) F.bwd_s(ch * SW_T + threadIdx.x, j0);  // j0: the number of parts
+  if (!on) return;
   if (PH == PH_FWD_A) F.fwd_a(j0);
-  if (PH == PH_FWD_B) { if (ch < F.fwd_b_chunks(j0)) F.fwd_b(j0, ch); }
-  if (PH == PH_FWD_U) { if (ch < F.fwd_u_chunks()) F.fwd_u(ch); }
-  if (PH == PH_BWD_R) { if (ch < F.bwd_r_chunks()) F.bwd_r(ch); }
+  if (PH == PH_FWD_B) F.fwd_b(j0, ch);
+  if (PH == PH_FWD_U) F.fwd_u(ch);
+  if (PH == PH_BWD_R) F.bwd_r(ch, blockIdx.z, gridDim.z);
   if (PH == PH_BWD_A) F.bwd_a(j0);
-  if (PH == PH_BWD_B) { if (ch < F.bwd_b_chunks(j0)) F.bwd_b(j0, ch); }
+  if (PH == PH_BWD_B) F.bwd_b(j0, ch);
 }
 
-// ---------------------------------------------------------------------------
 // Inverses of the 32 x 32 blocks on the diagonals of L11 and U11 of a depth's
 // fronts, in place: a warp per (front, block), by substitution, a lane per
 // column of the inverse in registers, the block in shared memory.
