@@ -2437,10 +2437,11 @@ int lfasm_assemble_rhs(lfasm_handle *h, const lfasm_incident_part *parts, int n_
   if (n_parts) LF_CUDA(upload(dcol, cols.data(), cols.size()));
   if (h->n_src) LF_CUDA(dmalloc(be, (size_t)h->n_src * ncol * h->nd));
   if (h->n_src && n_parts) {
-    const int wpb = 4;
-    k_rhs_elem<<<(h->n_src + wpb - 1) / wpb, wpb * 32, 0, h->stream>>>(
-        h->n_src, h->src_list, h->nd, h->p, h->rm.view(), h->J, h->Jinv, h->detJ, h->v0,
-        h->slab_of, h->delta, dw, n_slab, n_parts, dcol, ncol, h->pml.k0, h->fopack, be);
+    const auto kern = h->p == 1 ? k_rhs_elem<1> : h->p == 2 ? k_rhs_elem<2> : k_rhs_elem<3>;
+    const long long per = 4 * VEC_WARPS, np = (long long)h->n_src * ncol;
+    kern<<<(unsigned)((np + per - 1) / per), VEC_WARPS * 32, 0, h->stream>>>(
+        h->n_src, h->src_list, h->rm.view(), h->J, h->Jinv, h->detJ, h->v0, h->slab_of, h->delta, dw,
+        n_slab, n_parts, dcol, ncol, h->pml.k0, h->fopack, be);
     LF_LAUNCHED();
   } else if (h->n_src) {
     LF_CUDA(cudaMemsetAsync(be, 0, (size_t)h->n_src * ncol * h->nd * sizeof(dcplx), h->stream));
@@ -2497,11 +2498,12 @@ int lfasm_eps_gradient(lfasm_handle *h, const lfasm_incident_part *parts, int n_
   LF_CUDA(upload(dw, waves.data(), waves.size()));
   LF_CUDA(cudaMemsetAsync(d_grad, 0, (size_t)h->ne * sizeof(dcplx), h->stream));
   if (h->n_bulk) {
-    const int wpb = 4;
-    k_eps_grad<<<(h->n_bulk + wpb - 1) / wpb, wpb * 32, 0, h->stream>>>(
-        h->n_bulk, h->bulk_list, h->nd, h->p, h->rm.view(), h->J, h->Jinv, h->detJ, h->v0,
-        h->dof, h->sign, h->fopack, h->pml, h->slab_of, dw, n_slab, n_parts,
-        (const dcplx *)d_u, (const dcplx *)d_lambda, (dcplx *)d_grad);
+    const auto kern = h->p == 1 ? k_eps_grad<1> : h->p == 2 ? k_eps_grad<2> : k_eps_grad<3>;
+    const int per = 2 * VEC_WARPS;
+    kern<<<(h->n_bulk + per - 1) / per, VEC_WARPS * 32, 0, h->stream>>>(
+        h->n_bulk, h->bulk_list, h->rm.view(), h->J, h->Jinv, h->detJ, h->v0, h->dof, h->sign,
+        h->fopack, h->pml.k0, h->slab_of, dw, n_slab, n_parts, (const dcplx *)d_u,
+        (const dcplx *)d_lambda, (dcplx *)d_grad);
     LF_LAUNCHED();
   }
   LF_CUDA(cudaStreamSynchronize(h->stream));

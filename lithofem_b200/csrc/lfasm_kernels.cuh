@@ -2420,70 +2420,120 @@ struct SlabWaveD {
   dcplx A[3], B[3];
 };
 
-// one warp per source element; lanes over local dofs
-__global__ void k_rhs_elem(int nsrc, const int *__restrict__ list, int nd, int p, Rule rm,
-                           const double *__restrict__ J9, const double *__restrict__ Ji9,
-                           const double *__restrict__ detJ, const double *__restrict__ v0,
-                           const int *__restrict__ slab_of, const dcplx *__restrict__ delta,
-                           const SlabWaveD *__restrict__ waves, int n_slab, int n_parts,
-                           const int *__restrict__ col_of_part, int ncol, double k0,
-                           const unsigned *__restrict__ fopack, dcplx *__restrict__ be) {
-  const int lane = threadIdx.x & 31;
-  const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (i >= nsrc) return;
-  const int e = list[i];
+// Basis tables of the mass rule as DMMA left operands, 24 points staged at a
+// time (the p = 3 rule's count) in the order the lanes read them.
+constexpr int VEC_Q = 24;
+constexpr int VEC_WARPS = 8;
+template <int P> struct VecElem {
+  static constexpr int ND = P * (P + 2) * (P + 3) / 2;
+  static constexpr int KS = (ND + 3) / 4, MT = (ND + 7) / 8;
+};
+
+// one direction of a tabulated wave at height z: its amplitudes times
+// exp(i q (z - z0)) = exp(-Im(q) dz) (cos(Re(q) dz) + i sin(Re(q) dz))
+__device__ __forceinline__ dcplx wave_phase(const SlabWaveD &sw, bool down, double z) {
+  const dcplx q = down ? sw.qB : sw.qA;
+  const double dz = z - (down ? sw.zB : sw.zA);
+  const double m = exp(-q.im * dz);
+  double s, c;
+  sincos(q.re * dz, &s, &c);
+  return mk(m * c, m * s);
+}
+
+// Element source vectors b_k = sum_q w_q detJ k0^2 delta v_k(q) . E(q), dual
+// transform applied: be[(i ncol + c) nd + k].
+//
+// A product over (component, point) on FP64 tensor cores: the basis table
+// (nd rows) times J^-1 (w detJ k0^2 delta E) with (element, column, re / im)
+// as its columns, four elements x right-hand sides a warp.  A lane forms the
+// entries of the right operand that it feeds, one wave direction each, so
+// every exponential is evaluated once (with a lane per row each was evaluated
+// 64 times: 156 us for two columns of a 271k-row line grating, p = 3; 18 us
+// so).  Bound: the exponentials, sines and cosines.
+template <int P>
+__global__ void __launch_bounds__(VEC_WARPS * 32)
+k_rhs_elem(int nsrc, const int *__restrict__ list, Rule rm, const double *__restrict__ J9,
+           const double *__restrict__ Ji9, const double *__restrict__ detJ,
+           const double *__restrict__ v0, const int *__restrict__ slab_of,
+           const dcplx *__restrict__ delta, const SlabWaveD *__restrict__ waves, int n_slab,
+           int n_parts, const int *__restrict__ col_of_part, int ncol, double k0,
+           const unsigned *__restrict__ fopack, dcplx *__restrict__ be) {
+  constexpr int ND = VecElem<P>::ND, MT = VecElem<P>::MT;
+  __shared__ double As[VEC_Q / 4][3][MT][32];
+  const int lane = threadIdx.x & 31, t4 = lane & 3, g = lane >> 2;
+  const long long np = (long long)nsrc * ncol;
+  const long long p0 = (blockIdx.x * (long long)VEC_WARPS + (threadIdx.x >> 5)) * 4;
+  // right operand: column g is part g & 1 (re, im) of pair p0 + g / 2
+  const long long pr = min(p0 + (g >> 1), np - 1);
+  const int e = list[pr / ncol], c = (int)(pr % ncol);
+  const bool im = g & 1;
   double J[9], Ji[9];
   for (int t = 0; t < 9; ++t) { J[t] = J9[(size_t)e * 9 + t]; Ji[t] = Ji9[(size_t)e * 9 + t]; }
-  const double det = detJ[e];
-  const double x0[3] = {v0[(size_t)e * 3], v0[(size_t)e * 3 + 1], v0[(size_t)e * 3 + 2]};
-  const int slab = slab_of[e];
+  const double det = detJ[e], z0 = v0[(size_t)e * 3 + 2];
+  const SlabWaveD *wv = waves + slab_of[e];
   const dcplx fac = cscale(k0 * k0, delta[e]);
-  const unsigned fp = fopack ? fopack[e] : 0u;
-  for (int c = 0; c < ncol; ++c) {
-    for (int kb = 0; kb < nd; kb += 32) {
-      const int k = kb + lane;
-      double br = 0.0, bi = 0.0;
-      for (int q = 0; q < rm.nq; ++q) {
-        const double *xi = rm.ip + q * 3;
-        const double z = x0[2] + J[6] * xi[0] + J[7] * xi[1] + J[8] * xi[2];
-        dcplx ev[3] = {mk(0, 0), mk(0, 0), mk(0, 0)};
-        for (int pi = 0; pi < n_parts; ++pi) {
-          if (col_of_part[pi] != c) continue;
-          const SlabWaveD &sw = waves[(size_t)pi * n_slab + slab];
-          // exp(i q (z - zA)) = exp(-Im(q) dz) (cos(Re(q) dz) + i sin(Re(q) dz))
-          const double da = z - sw.zA, db = z - sw.zB;
-          const double ma = exp(-sw.qA.im * da), mb = exp(-sw.qB.im * db);
-          double sa, ca, sb, cb;
-          sincos(sw.qA.re * da, &sa, &ca);
-          sincos(sw.qB.re * db, &sb, &cb);
-          const dcplx up = mk(ma * ca, ma * sa), dn = mk(mb * cb, mb * sb);
-          for (int d = 0; d < 3; ++d)
-            ev[d] = cadd(ev[d], cadd(cmul(sw.A[d], up), cmul(sw.B[d], dn)));
-        }
-        const double w = rm.w[q] * det;
-        if (k < nd) {
-          const double *rv = rm.v + ((size_t)q * nd + k) * 3;
-          for (int d = 0; d < 3; ++d) {
-            const double pv = rv[0] * Ji[0 * 3 + d] + rv[1] * Ji[1 * 3 + d] + rv[2] * Ji[2 * 3 + d];
-            const dcplx f = cmul(fac, ev[d]);
-            br += w * pv * f.re;
-            bi += w * pv * f.im;
-          }
-        }
+  double acc[MT][2];
+#pragma unroll
+  for (int m = 0; m < MT; ++m) acc[m][0] = acc[m][1] = 0.0;
+  for (int q0 = 0; q0 < rm.nq; q0 += VEC_Q) {
+    __syncthreads();
+    for (int t = threadIdx.x; t < VEC_Q / 4 * 3 * MT * 32; t += VEC_WARPS * 32) {
+      const int l = t & 31, m = t / 32 % MT, d = t / (32 * MT) % 3, qs = t / (96 * MT);
+      const int q = q0 + 4 * qs + (l & 3);
+      As[qs][d][m][l] = q < rm.nq ? rm.vt[((size_t)d * rm.nq + q) * rm.ldt + m * 8 + (l >> 2)] : 0.0;
+    }
+    __syncthreads();
+    for (int qs = 0; qs < VEC_Q / 4 && q0 + 4 * qs < rm.nq; ++qs) {
+      const int q = min(q0 + 4 * qs + t4, rm.nq - 1);
+      const double *xi = rm.ip + q * 3;
+      const double z = z0 + J[6] * xi[0] + J[7] * xi[1] + J[8] * xi[2];
+      dcplx ev[3] = {mk(0, 0), mk(0, 0), mk(0, 0)};
+      for (int pi = 0; pi < n_parts; ++pi) {
+        if (col_of_part[pi] != c) continue;
+        const SlabWaveD &sw = wv[(size_t)pi * n_slab];
+        const dcplx ph = wave_phase(sw, im, z);  // up in the re lane, down in the im lane
+#pragma unroll
+        for (int d = 0; d < 3; ++d) ev[d] = cadd(ev[d], cmul(im ? sw.B[d] : sw.A[d], ph));
       }
-      // dual transform on the element vector: b <- M^T b on face pairs
-      const double obr = __shfl_xor_sync(0xffffffffu, br, 1);
-      const double obi = __shfl_xor_sync(0xffffffffu, bi, 1);
-      const int f = (p >= 2 && k < nd) ? face_of(k & ~1, p) : -1;
+      const double w = q0 + 4 * qs + t4 < rm.nq ? rm.w[q] * det : 0.0;
+      double f[3];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        ev[d].re += __shfl_xor_sync(0xffffffffu, ev[d].re, 4);
+        ev[d].im += __shfl_xor_sync(0xffffffffu, ev[d].im, 4);
+        const dcplx v = cmul(fac, ev[d]);
+        f[d] = w * (im ? v.im : v.re);
+      }
+      __syncwarp();
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        const double b = Ji[3 * d] * f[0] + Ji[3 * d + 1] * f[1] + Ji[3 * d + 2] * f[2];
+#pragma unroll
+        for (int m = 0; m < MT; ++m) dmma(acc[m][0], acc[m][1], As[qs][d][m][lane], b);
+      }
+    }
+  }
+  // the lane's results: row m 8 + g of pair p0 + t4; dual transform on the
+  // element vector: b <- M^T b on face pairs (the partner row is lane ^ 4)
+  const bool mine = p0 + t4 < np;
+  const unsigned fp = P > 1 && mine ? fopack[list[(p0 + t4) / ncol]] : 0u;
+#pragma unroll
+  for (int m = 0; m < MT; ++m) {
+    const int k = m * 8 + g;
+    double br = acc[m][0], bi = acc[m][1];
+    if (P > 1) {
+      const double obr = __shfl_xor_sync(0xffffffffu, br, 4);
+      const double obi = __shfl_xor_sync(0xffffffffu, bi, 4);
+      const int f = k < ND ? face_of(k & ~1, P) : -1;
       if (f >= 0) {
         const double *T = c_tinv + 4 * ((fp >> (8 * f)) & 0xffu);
         const int cp = k & 1;
         const double own = T[2 * cp + cp], oth = T[2 * cp + (1 - cp)];
-        const double nr = own * br + oth * obr, ni = own * bi + oth * obi;
-        br = nr; bi = ni;
+        br = own * br + oth * obr;
+        bi = own * bi + oth * obi;
       }
-      if (k < nd) be[((size_t)i * ncol + c) * nd + k] = mk(br, bi);
     }
+    if (mine && k < ND) be[(p0 + t4) * ND + k] = mk(br, bi);
   }
 }
 
@@ -2512,7 +2562,7 @@ __global__ void k_rhs_gather(int n, const int *__restrict__ ea_ptr, const int *_
 }
 
 // ---------------------------------------------------------------------------
-// Adjoint contraction for per-element permittivity (one warp per element).
+// Adjoint contraction for per-element permittivity.
 //
 // For l(u) = c^T u with A(eps) u = b(eps) and A^T lambda = c:
 //   dl/deps_e = lambda^T (db/deps_e - dA/deps_e u)
@@ -2522,102 +2572,118 @@ __global__ void k_rhs_gather(int n, const int *__restrict__ ea_ptr, const int *_
 // problem_common.inc:123-148), db_e/deps_e = k0^2 int v . Ehat
 // (ScatterSource, problem_common.inc:238-266), Lam = (s, s, 1/s), v the
 // physical shapes and lt, ut the element-local coefficients of lambda and u
-// (signs and the face transform applied: local = M (sign * global)).
+// (signs and the face transform applied: local = M (sign * global)).  The
+// elements taken are the bulk ones, where s = 1 at every point: Lam = 1.
+//
+// The fields at the points are a product on FP64 tensor cores: the basis
+// table, a row per (component, point), times the elements' coefficients, two
+// elements a warp (u.re, u.im, lambda.re, lambda.im each).  A lane ends up
+// with u or lambda at a point and evaluates one direction of the incident
+// waves there.  (A warp per element that summed each point over its lanes and
+// left the waves to lane 0: 345 us on a 271k-row line grating, p = 3; 34 us
+// so.)  Bound: the gathers of u and lambda, and the exponentials.
 // ---------------------------------------------------------------------------
-__global__ void k_eps_grad(int nsel, const int *__restrict__ list, int nd, int p, Rule rm,
-                           const double *__restrict__ J9, const double *__restrict__ Ji9,
-                           const double *__restrict__ detJ, const double *__restrict__ v0,
-                           const int *__restrict__ dof, const double *__restrict__ sign,
-                           const unsigned *__restrict__ fopack, PmlParams pml,
-                           const int *__restrict__ slab_of, const SlabWaveD *__restrict__ waves,
-                           int n_slab, int n_parts, const dcplx *__restrict__ u,
-                           const dcplx *__restrict__ lam, dcplx *__restrict__ grad) {
-  const int lane = threadIdx.x & 31;
-  const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (i >= nsel) return;
-  const int e = list[i];
-  double J[9], Ji[9];
-  for (int t = 0; t < 9; ++t) { J[t] = J9[(size_t)e * 9 + t]; Ji[t] = Ji9[(size_t)e * 9 + t]; }
-  const double det = detJ[e];
-  const double z0 = v0[(size_t)e * 3 + 2];
-  const unsigned fp = fopack ? fopack[e] : 0u;
-  // local coefficients for k = lane and k = lane + 32
-  dcplx lt[2], ut[2];
-  for (int hh = 0; hh < 2; ++hh) {
-    const int k = lane + 32 * hh;
-    dcplx lg = mk(0, 0), ug = mk(0, 0);
-    if (k < nd) {
-      const double sg = sign[(size_t)e * nd + k];
-      const int d = dof[(size_t)e * nd + k];
-      lg = cscale(sg, lam[d]);
-      ug = cscale(sg, u[d]);
+template <int P>
+__global__ void __launch_bounds__(VEC_WARPS * 32)
+k_eps_grad(int nsel, const int *__restrict__ list, Rule rm, const double *__restrict__ J9,
+           const double *__restrict__ Ji9, const double *__restrict__ detJ,
+           const double *__restrict__ v0, const int *__restrict__ dof,
+           const double *__restrict__ sign, const unsigned *__restrict__ fopack, double k0,
+           const int *__restrict__ slab_of, const SlabWaveD *__restrict__ waves, int n_slab,
+           int n_parts, const dcplx *__restrict__ u, const dcplx *__restrict__ lam,
+           dcplx *__restrict__ grad) {
+  constexpr int ND = VecElem<P>::ND, KS = VecElem<P>::KS;
+  __shared__ double As[VEC_Q / 8][3][KS][32];
+  const int lane = threadIdx.x & 31, t4 = lane & 3, g = lane >> 2;
+  const int i0 = (blockIdx.x * VEC_WARPS + (threadIdx.x >> 5)) * 2;
+  // right operand: column g is part g & 3 of element g / 4, rows t4 + 4 s
+  double B[KS];
+  {
+    const int e = list[min(i0 + (g >> 2), nsel - 1)];
+    const double *vec = reinterpret_cast<const double *>(g & 2 ? lam : u) + (g & 1);
+    const unsigned fp = P > 1 ? fopack[e] : 0u;
+    int at[KS];
+#pragma unroll
+    for (int s = 0; s < KS; ++s) {
+      const int k = 4 * s + t4;
+      at[s] = k < ND ? dof[(size_t)e * ND + k] : -1;
+      B[s] = k < ND ? sign[(size_t)e * ND + k] : 0.0;
     }
-    // face pairs: local = M global, M[r][c] = T[2c + r] (column-major)
-    const double olr = __shfl_xor_sync(0xffffffffu, lg.re, 1);
-    const double oli = __shfl_xor_sync(0xffffffffu, lg.im, 1);
-    const double our = __shfl_xor_sync(0xffffffffu, ug.re, 1);
-    const double oui = __shfl_xor_sync(0xffffffffu, ug.im, 1);
-    const int f = (p >= 2 && k < nd) ? face_of(k & ~1, p) : -1;
-    if (f >= 0) {
-      const double *T = c_tinv + 4 * ((fp >> (8 * f)) & 0xffu);
-      const int r = k & 1;
-      const double own = T[2 * r + r], oth = T[2 * (1 - r) + r];
-      lg = mk(own * lg.re + oth * olr, own * lg.im + oth * oli);
-      ug = mk(own * ug.re + oth * our, own * ug.im + oth * oui);
+#pragma unroll
+    for (int s = 0; s < KS; ++s) {
+      const int k = 4 * s + t4;
+      double v = at[s] >= 0 ? B[s] * vec[2 * (size_t)at[s]] : 0.0;
+      if (P > 1) {  // face pairs: local = M global, M[r][c] = T[2c + r] (column-major)
+        const double o = __shfl_xor_sync(0xffffffffu, v, 1);
+        const int f = k < ND ? face_of(k & ~1, P) : -1;
+        if (f >= 0) {
+          const double *T = c_tinv + 4 * ((fp >> (8 * f)) & 0xffu);
+          const int r = k & 1;
+          v = T[2 * r + r] * v + T[2 * (1 - r) + r] * o;
+        }
+      }
+      B[s] = v;
     }
-    lt[hh] = lg;
-    ut[hh] = ug;
   }
+  // the lane's results: u (even t4) or lambda (odd) of element t4 / 2
+  const bool odd = t4 & 1;
+  const int e = list[min(i0 + (t4 >> 1), nsel - 1)];
+  double J[3], Ji[9];
+  for (int t = 0; t < 3; ++t) J[t] = J9[(size_t)e * 9 + 6 + t];
+  for (int t = 0; t < 9; ++t) Ji[t] = Ji9[(size_t)e * 9 + t];
+  const double det = detJ[e], z0 = v0[(size_t)e * 3 + 2];
   const int slab = slab_of[e];
   double gr = 0.0, gi = 0.0;
-  for (int q = 0; q < rm.nq; ++q) {
-    dcplx Lv[3] = {mk(0, 0), mk(0, 0), mk(0, 0)}, Uv[3] = {mk(0, 0), mk(0, 0), mk(0, 0)};
-    for (int hh = 0; hh < 2; ++hh) {
-      const int k = lane + 32 * hh;
-      if (k >= nd) continue;
-      const double *rv = rm.v + ((size_t)q * nd + k) * 3;
-      for (int d = 0; d < 3; ++d) {
-        const double pv = rv[0] * Ji[0 * 3 + d] + rv[1] * Ji[1 * 3 + d] + rv[2] * Ji[2 * 3 + d];
-        Lv[d] = cadd(Lv[d], cscale(pv, lt[hh]));
-        Uv[d] = cadd(Uv[d], cscale(pv, ut[hh]));
-      }
+  for (int q0 = 0; q0 < rm.nq; q0 += VEC_Q) {
+    __syncthreads();
+    for (int t = threadIdx.x; t < VEC_Q / 8 * 3 * KS * 32; t += VEC_WARPS * 32) {
+      const int l = t & 31, s = t / 32 % KS, d = t / (32 * KS) % 3, qt = t / (96 * KS);
+      const int q = q0 + 8 * qt + (l >> 2);
+      As[qt][d][s][l] = q < rm.nq ? rm.vt[((size_t)d * rm.nq + q) * rm.ldt + 4 * s + (l & 3)] : 0.0;
     }
-    for (int o = 16; o; o >>= 1)
+    __syncthreads();
+    for (int qt = 0; qt < VEC_Q / 8 && q0 + 8 * qt < rm.nq; ++qt) {
+      double R[3][2];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) R[d][0] = R[d][1] = 0.0;
+      __syncwarp();
+#pragma unroll
+      for (int s = 0; s < KS; ++s)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) dmma(R[d][0], R[d][1], As[qt][d][s][lane], B[s]);
+      const int q = q0 + 8 * qt + g;
+      dcplx v[3], o[3], acc = mk(0, 0);
+#pragma unroll
       for (int d = 0; d < 3; ++d) {
-        Lv[d].re += __shfl_xor_sync(0xffffffffu, Lv[d].re, o);
-        Lv[d].im += __shfl_xor_sync(0xffffffffu, Lv[d].im, o);
-        Uv[d].re += __shfl_xor_sync(0xffffffffu, Uv[d].re, o);
-        Uv[d].im += __shfl_xor_sync(0xffffffffu, Uv[d].im, o);
+        v[d] = mk(R[0][0] * Ji[d] + R[1][0] * Ji[3 + d] + R[2][0] * Ji[6 + d],
+                  R[0][1] * Ji[d] + R[1][1] * Ji[3 + d] + R[2][1] * Ji[6 + d]);
+        o[d] = mk(__shfl_xor_sync(0xffffffffu, v[d].re, 1), __shfl_xor_sync(0xffffffffu, v[d].im, 1));
       }
-    if (lane == 0) {
+      if (q >= rm.nq) continue;
+      if (!odd)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) acc = cadd(acc, cmul(v[d], o[d]));
       const double *xi = rm.ip + q * 3;
-      const double z = z0 + J[6] * xi[0] + J[7] * xi[1] + J[8] * xi[2];
-      const dcplx s = pml_s(pml, z);
-      const dcplx Lam[3] = {s, s, cinv(s)};
-      dcplx acc = mk(0, 0);
-      for (int d = 0; d < 3; ++d) acc = cadd(acc, cmul(Lam[d], cmul(Lv[d], Uv[d])));
-      if (slab >= 0 && n_parts > 0) {
-        dcplx ev[3] = {mk(0, 0), mk(0, 0), mk(0, 0)};
-        for (int pi = 0; pi < n_parts; ++pi) {
-          const SlabWaveD &sw = waves[(size_t)pi * n_slab + slab];
-          const double da = z - sw.zA, db = z - sw.zB;
-          const double ma = exp(-sw.qA.im * da), mb = exp(-sw.qB.im * db);
-          double sa, ca, sb, cb;
-          sincos(sw.qA.re * da, &sa, &ca);
-          sincos(sw.qB.re * db, &sb, &cb);
-          const dcplx up = mk(ma * ca, ma * sa), dn = mk(mb * cb, mb * sb);
-          for (int d = 0; d < 3; ++d)
-            ev[d] = cadd(ev[d], cadd(cmul(sw.A[d], up), cmul(sw.B[d], dn)));
-        }
-        for (int d = 0; d < 3; ++d) acc = cadd(acc, cmul(Lv[d], ev[d]));
+      const double z = z0 + J[0] * xi[0] + J[1] * xi[1] + J[2] * xi[2];
+      for (int pi = 0; slab >= 0 && pi < n_parts; ++pi) {
+        const SlabWaveD &sw = waves[(size_t)pi * n_slab + slab];
+        dcplx a = mk(0, 0);
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+          a = cadd(a, odd ? cmul(v[d], sw.B[d]) : cmul(o[d], sw.A[d]));
+        acc = cadd(acc, cmul(a, wave_phase(sw, odd, z)));
       }
       const double w = rm.w[q] * det;
       gr += w * acc.re;
       gi += w * acc.im;
     }
   }
-  if (lane == 0) {
-    const double k2 = pml.k0 * pml.k0;
+  for (int x : {1, 4, 8, 16}) {
+    gr += __shfl_xor_sync(0xffffffffu, gr, x);
+    gi += __shfl_xor_sync(0xffffffffu, gi, x);
+  }
+  if (g == 0 && !odd && i0 + (t4 >> 1) < nsel) {
+    const double k2 = k0 * k0;
     grad[e] = mk(k2 * gr, k2 * gi);
   }
 }
