@@ -1802,10 +1802,19 @@ int lfasm_set_basis(lfasm_handle *h, int nmono, const int *exps, const double *c
   }
   LF_CUDA(cudaSetDevice(h->dev));
   dfree(h->bexps); dfree(h->bcoef); dfree(h->bccoef);
-  const size_t nc = (size_t)h->nd * 3 * nmono;
+  // [k][d][m] -> [k & 1][d][m][k / 2]: the layout basis_pair reads
+  auto pair_table = [&](const double *t) {
+    const int np = (h->nd + 1) / 2;
+    std::vector<double> out((size_t)6 * nmono * np, 0.0);
+    for (int k = 0; k < h->nd; ++k)
+      for (int dm = 0; dm < 3 * nmono; ++dm)
+        out[((size_t)(k & 1) * 3 * nmono + dm) * np + k / 2] = t[(size_t)k * 3 * nmono + dm];
+    return out;
+  };
+  const std::vector<double> pv = pair_table(coef), pc = pair_table(curl_coef);
   LF_CUDA(upload(h->bexps, exps, (size_t)nmono * 3));
-  LF_CUDA(upload(h->bcoef, coef, nc));
-  LF_CUDA(upload(h->bccoef, curl_coef, nc));
+  LF_CUDA(upload(h->bcoef, pv.data(), pv.size()));
+  LF_CUDA(upload(h->bccoef, pc.data(), pc.size()));
   h->nmono = nmono;
   return LFASM_OK;
 }
@@ -1832,7 +1841,7 @@ struct DevBufs {
 
 // Sample points of nz planes (heights zs, host) located in the mesh: per
 // plane the elements whose z-range holds it (flags [iz][e], one scan, one
-// compaction), then a warp per point over its plane's candidates; *elem
+// compaction), then its points against its candidates; *elem
 // and *xi (device, nz * nx * ny points) are the caller's to free.
 int plane_locate(lfasm_handle *h, const PlaneGrid &G, int nz, const double *zs, int **elem,
                  double **xi) {
@@ -1860,9 +1869,8 @@ int plane_locate(lfasm_handle *h, const PlaneGrid &G, int nz, const double *zs, 
   LF_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tb, flag, pos, (int)(nf + 1), h->stream));
   k_compact<<<gb, 256, 0, h->stream>>>((int)nf, flag, pos, cand);
   LF_LAUNCHED();
-  const int wpb = 8;
-  k_plane_locate<<<(unsigned)((ntot + wpb - 1) / wpb), wpb * 32, 0, h->stream>>>(
-      G, nz, dz, ne, pos, cand, h->Jinv, h->v0, *elem, *xi, miss);
+  k_plane_locate<<<dim3((unsigned)((npts + LOC_PTS - 1) / LOC_PTS), (unsigned)nz), LOC_T, 0, h->stream>>>(
+      G, dz, ne, pos, cand, h->Jinv, h->v0, *elem, *xi, miss);
   LF_LAUNCHED();
   int nmiss = 0;
   LF_CUDA(cudaMemcpyAsync(&nmiss, miss, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
@@ -1877,6 +1885,21 @@ int plane_locate(lfasm_handle *h, const PlaneGrid &G, int nz, const double *zs, 
                 nmiss, ntot, nz);
   }
   return LFASM_OK;
+}
+
+// E and curl E at npts located points, which are freed
+int plane_eval(lfasm_handle *h, int npts, int *elem, double *xi, const void *d_u, void *d_e,
+               void *d_curl) {
+  const int T = 256;
+  const auto kern = h->p == 1 ? k_plane_eval<4> : h->p == 2 ? k_plane_eval<16> : k_plane_eval<32>;
+  const int per = T / (h->p == 1 ? 4 : h->p == 2 ? 16 : 32);  // 3, 10 and 23 pairs of functions
+  kern<<<(unsigned)((npts + per - 1) / per), T, 0, h->stream>>>(
+      npts, elem, xi, h->nd, h->p, h->nmono, h->bexps, h->bcoef, h->bccoef, h->dof, h->sign,
+      h->fopack, h->J, h->Jinv, h->detJ, (const dcplx *)d_u, (dcplx *)d_e, (dcplx *)d_curl);
+  LF_LAUNCHED();
+  LF_CUDA(cudaStreamSynchronize(h->stream));
+  dfree(elem); dfree(xi);
+  return sync_if(h);
 }
 
 int plane_args(lfasm_handle *h, double lx, double ly, double z, int nx, int ny, PlaneGrid &G) {
@@ -1903,14 +1926,7 @@ int lfasm_sample_plane(lfasm_handle *h, double lx, double ly, double z, int nx, 
   int *elem = nullptr;
   double *xi = nullptr;
   if ((rc = plane_locate(h, G, 1, &z, &elem, &xi))) return rc;
-  const int npts = nx * ny, wpb = 8;
-  k_plane_eval<<<(unsigned)((npts + wpb - 1) / wpb), wpb * 32, 0, h->stream>>>(
-      npts, elem, xi, h->nd, h->p, h->nmono, h->bexps, h->bcoef, h->bccoef, h->dof, h->sign,
-      h->fopack, h->J, h->Jinv, h->detJ, (const dcplx *)d_u, (dcplx *)d_e, (dcplx *)d_curl);
-  LF_LAUNCHED();
-  LF_CUDA(cudaStreamSynchronize(h->stream));
-  dfree(elem); dfree(xi);
-  return sync_if(h);
+  return plane_eval(h, nx * ny, elem, xi, d_u, d_e, d_curl);
 }
 
 int lfasm_plane_seed(lfasm_handle *h, double lx, double ly, double z, int nx, int ny, int comp,
@@ -1951,15 +1967,7 @@ int lfasm_sample_planes(lfasm_handle *h, double lx, double ly, int nz, const dou
   int *elem = nullptr;
   double *xi = nullptr;
   if ((rc = plane_locate(h, G, nz, z, &elem, &xi))) return rc;
-  const long long npts = (long long)nx * ny * nz;
-  const int wpb = 8;
-  k_plane_eval<<<(unsigned)((npts + wpb - 1) / wpb), wpb * 32, 0, h->stream>>>(
-      (int)npts, elem, xi, h->nd, h->p, h->nmono, h->bexps, h->bcoef, h->bccoef, h->dof, h->sign,
-      h->fopack, h->J, h->Jinv, h->detJ, (const dcplx *)d_u, (dcplx *)d_e, (dcplx *)d_curl);
-  LF_LAUNCHED();
-  LF_CUDA(cudaStreamSynchronize(h->stream));
-  dfree(elem); dfree(xi);
-  return sync_if(h);
+  return plane_eval(h, nx * ny * nz, elem, xi, d_u, d_e, d_curl);
 }
 
 int lfasm_plane_orders(lfasm_handle *h, int nz, int nx, int ny, const void *d_e,
@@ -1981,41 +1989,34 @@ int lfasm_plane_orders(lfasm_handle *h, int nz, int nx, int ny, const void *d_e,
                   planes[i].direction);
   g_err.clear();
   LF_CUDA(cudaSetDevice(h->dev));
-  // per-plane scalars packed into one upload: z, z_ref, eps (2), background (6)
-  std::vector<double> hp((size_t)nz * 10);
-  std::vector<int> hd(nz);
+  // per-plane scalars in one upload (a row of ORDER_ROW each)
+  std::vector<double> hp((size_t)nz * ORDER_ROW, 0.0);
   bool any_bg = false;
   for (int i = 0; i < nz; ++i) {
     const lfasm_order_plane &q = planes[i];
-    double *r = hp.data() + (size_t)i * 10;
+    double *r = hp.data() + (size_t)i * ORDER_ROW;
     r[0] = q.z; r[1] = q.z_ref; r[2] = q.eps_re; r[3] = q.eps_im;
-    for (int c = 0; c < 6; ++c) r[4 + c] = q.bg00[c];
+    if (q.has_bg00)
+      for (int c = 0; c < 6; ++c) r[4 + c] = q.bg00[c];
     any_bg = any_bg || q.has_bg00;
-    if (!q.has_bg00)
-      for (int c = 0; c < 6; ++c) r[4 + c] = 0.0;
-    hd[i] = q.direction;
+    r[10] = q.direction;
   }
+  const int all = nx * ny * nz, per = ORDER_THREADS / ORDER_LANES;
+  const unsigned blocks = (unsigned)((all + per - 1) / per);
+  DevBufs B;
   double *dp = nullptr;
-  int *dd = nullptr;
-  LF_CUDA(dmalloc(dp, hp.size()));
-  LF_CUDA(dmalloc(dd, hd.size()));
+  dcplx *R = nullptr;
+  LF_CUDA(B.get(dp, hp.size()));
+  LF_CUDA(B.get(R, (size_t)all * 3));
   LF_CUDA(cudaMemcpyAsync(dp, hp.data(), sizeof(double) * hp.size(), cudaMemcpyHostToDevice,
                           h->stream));
-  LF_CUDA(cudaMemcpyAsync(dd, hd.data(), sizeof(int) * hd.size(), cudaMemcpyHostToDevice,
-                          h->stream));
-  // split the packed rows into the kernel's arrays: z, z_ref, eps, background
-  double *zs = nullptr;
-  LF_CUDA(dmalloc(zs, (size_t)nz * 10));
-  k_unpack_planes<<<(nz + 127) / 128, 128, 0, h->stream>>>(nz, dp, zs, zs + nz, zs + 2 * nz,
-                                                            zs + 4 * nz);
+  k_orders_rows<<<blocks, ORDER_THREADS, 0, h->stream>>>(nx, ny * nz, (const dcplx *)d_e, R);
   LF_LAUNCHED();
   OrderArgs A{a.lx, a.ly, a.k0, a.kx, a.ky, a.inc_flux};
-  k_plane_orders<<<dim3((unsigned)(nx * ny), (unsigned)nz), ORDER_THREADS, 0, h->stream>>>(
-      nx, ny, (const dcplx *)d_e, zs, zs + nz, dd, zs + 2 * nz, any_bg ? zs + 4 * nz : nullptr,
-      A, (dcplx *)d_coef, d_eff);
+  k_plane_orders<<<blocks, ORDER_THREADS, 0, h->stream>>>(nx, ny, nz, R, dp, any_bg, A,
+                                                          (dcplx *)d_coef, d_eff);
   LF_LAUNCHED();
   LF_CUDA(cudaStreamSynchronize(h->stream));
-  dfree(dp); dfree(dd); dfree(zs);
   return sync_if(h);
 }
 

@@ -2735,63 +2735,83 @@ __global__ void k_compact(int n, const int *__restrict__ flag, const int *__rest
   if (e < n && flag[e]) out[pos[e]] = e;
 }
 
-// one warp per sample point of nz planes (point pt of plane pt / (nx ny)):
-// the candidate element of its plane (cand[pos[iz ne] .. pos[(iz + 1) ne]))
-// in which the point is most interior (largest smallest barycentric
-// coordinate; lower index on a tie) and the point's reference coordinates;
-// *missing counts points that lie outside every candidate
-__global__ void k_plane_locate(PlaneGrid G, int nz, const double *__restrict__ zs, int ne,
-                               const int *__restrict__ pos, const int *__restrict__ cand,
-                               const double *__restrict__ Ji9, const double *__restrict__ v0,
-                               int *__restrict__ elem, double *__restrict__ xi,
-                               int *__restrict__ missing) {
-  const int lane = threadIdx.x & 31;
-  const int npts = G.nx * G.ny;
-  const long long ptg = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (ptg >= (long long)npts * nz) return;
-  const int iz = (int)(ptg / npts), pt = (int)ptg;
+// The candidate element of each sample point of plane blockIdx.y
+// (cand[pos[iz ne] .. pos[(iz + 1) ne])) in which the point is most interior
+// (largest smallest barycentric coordinate; lower index on a tie) and the
+// point's reference coordinates; *missing counts points that lie outside every
+// candidate.  A block takes LOC_PTS points and walks through the candidates
+// LOC_CAND at a time: their J^-1 and corner go to shared memory once for all
+// its points, which LOC_LANES lanes each share out.  (A warp a point reading
+// them from global memory, 72 and 24 bytes apart: 44 us for two planes of
+// 48 x 48 points over 15.6k elements; 22 us so.)  Bound: latency.
+constexpr int LOC_T = 128, LOC_LANES = 8, LOC_PTS = LOC_T / LOC_LANES, LOC_CAND = 2 * LOC_T;
+__global__ void __launch_bounds__(LOC_T)
+k_plane_locate(PlaneGrid G, const double *__restrict__ zs, int ne, const int *__restrict__ pos,
+               const int *__restrict__ cand, const double *__restrict__ Ji9,
+               const double *__restrict__ v0, int *__restrict__ elem, double *__restrict__ xi,
+               int *__restrict__ missing) {
+  __shared__ double sg[12][LOC_CAND];
+  __shared__ int se[LOC_CAND];
+  const int npts = G.nx * G.ny, iz = blockIdx.y;
+  const int lp = blockIdx.x * LOC_PTS + threadIdx.x / LOC_LANES, sub = threadIdx.x % LOC_LANES;
   double x[3];
-  plane_point(G, pt % npts, zs[iz], x);
+  plane_point(G, min(lp, npts - 1), zs[iz], x);
   double best = -1e300;
   int be = 0x7fffffff;
   // the compaction kept flattened (plane, element) indices iz ne + e
   const int c0 = pos[(size_t)iz * ne], c1 = pos[(size_t)(iz + 1) * ne];
-  for (int i = c0 + lane; i < c1; i += 32) {
-    const int e = cand[i] - iz * ne;
-    const double *Ji = Ji9 + (size_t)e * 9;
-    const double d0 = x[0] - v0[(size_t)e * 3], d1 = x[1] - v0[(size_t)e * 3 + 1],
-                 d2 = x[2] - v0[(size_t)e * 3 + 2];
-    const double a = Ji[0] * d0 + Ji[1] * d1 + Ji[2] * d2;
-    const double b = Ji[3] * d0 + Ji[4] * d1 + Ji[5] * d2;
-    const double c = Ji[6] * d0 + Ji[7] * d1 + Ji[8] * d2;
-    const double m = fmin(fmin(1.0 - a - b - c, a), fmin(b, c));
-    if (m > best || (m == best && e < be)) { best = m; be = e; }
+  for (int i0 = c0; i0 < c1; i0 += LOC_CAND) {
+    const int n = min(LOC_CAND, c1 - i0);
+    __syncthreads();
+#pragma unroll
+    for (int h = 0; h < LOC_CAND / LOC_T; ++h) {
+      const int c = threadIdx.x + h * LOC_T;
+      if (c >= n) continue;
+      const int e = cand[i0 + c] - iz * ne;
+      se[c] = e;
+#pragma unroll
+      for (int t = 0; t < 9; ++t) sg[t][c] = Ji9[(size_t)e * 9 + t];
+#pragma unroll
+      for (int t = 0; t < 3; ++t) sg[9 + t][c] = v0[(size_t)e * 3 + t];
+    }
+    __syncthreads();
+    for (int c = sub; c < n; c += LOC_LANES) {
+      const int e = se[c];
+      const double d0 = x[0] - sg[9][c], d1 = x[1] - sg[10][c], d2 = x[2] - sg[11][c];
+      const double r = sg[0][c] * d0 + sg[1][c] * d1 + sg[2][c] * d2;
+      const double s = sg[3][c] * d0 + sg[4][c] * d1 + sg[5][c] * d2;
+      const double t = sg[6][c] * d0 + sg[7][c] * d1 + sg[8][c] * d2;
+      const double m = fmin(fmin(1.0 - r - s - t, r), fmin(s, t));
+      if (m > best || (m == best && e < be)) { best = m; be = e; }
+    }
   }
-  for (int o = 16; o; o >>= 1) {
+  for (int o = LOC_LANES / 2; o; o >>= 1) {
     const double ob = __shfl_xor_sync(0xffffffffu, best, o);
     const int oe = __shfl_xor_sync(0xffffffffu, be, o);
     if (ob > best || (ob == best && oe < be)) { best = ob; be = oe; }
   }
-  if (lane == 0) {
-    if (be == 0x7fffffff || best < -1e-9) {
-      atomicAdd(missing, 1);
-      elem[pt] = -1;
-      return;
-    }
-    elem[pt] = be;
-    const double *Ji = Ji9 + (size_t)be * 9;
-    const double d0 = x[0] - v0[(size_t)be * 3], d1 = x[1] - v0[(size_t)be * 3 + 1],
-                 d2 = x[2] - v0[(size_t)be * 3 + 2];
-    xi[pt * 3 + 0] = Ji[0] * d0 + Ji[1] * d1 + Ji[2] * d2;
-    xi[pt * 3 + 1] = Ji[3] * d0 + Ji[4] * d1 + Ji[5] * d2;
-    xi[pt * 3 + 2] = Ji[6] * d0 + Ji[7] * d1 + Ji[8] * d2;
+  if (sub || lp >= npts) return;
+  const int pt = iz * npts + lp;
+  if (be == 0x7fffffff || best < -1e-9) {
+    atomicAdd(missing, 1);
+    elem[pt] = -1;
+    return;
   }
+  elem[pt] = be;
+  const double *Ji = Ji9 + (size_t)be * 9;
+  const double d0 = x[0] - v0[(size_t)be * 3], d1 = x[1] - v0[(size_t)be * 3 + 1],
+               d2 = x[2] - v0[(size_t)be * 3 + 2];
+  xi[pt * 3 + 0] = Ji[0] * d0 + Ji[1] * d1 + Ji[2] * d2;
+  xi[pt * 3 + 1] = Ji[3] * d0 + Ji[4] * d1 + Ji[5] * d2;
+  xi[pt * 3 + 2] = Ji[6] * d0 + Ji[7] * d1 + Ji[8] * d2;
 }
 
 // Global basis functions of element e at reference point xi for the pair of
 // local functions (2 pr, 2 pr + 1): physical values psi (covariant map,
 // v J^-1) and physical curls (J c / detJ), with the face transform applied
-// like in the element kernels.  k >= nd gives zeros.
+// like in the element kernels.  k >= nd gives zeros.  The coefficient tables
+// are laid out [k & 1][d][monomial][pair] (pair_table), so that the lanes of a
+// point, a pair each, read neighbours.
 __device__ __forceinline__ void basis_pair(int e, int pr, const double *xi, int nd, int p,
                                            int nmono, const int *__restrict__ exps,
                                            const double *__restrict__ coef,
@@ -2816,8 +2836,9 @@ __device__ __forceinline__ void basis_pair(int e, int pr, const double *xi, int 
     if (k < nd)
       for (int d = 0; d < 3; ++d)
         for (int m = 0; m < nmono; ++m) {
-          r[d] += coef[((size_t)k * 3 + d) * nmono + m] * mono[m];
-          q[d] += ccoef[((size_t)k * 3 + d) * nmono + m] * mono[m];
+          const int at = ((h * 3 + d) * nmono + m) * ((nd + 1) / 2) + pr;
+          r[d] += coef[at] * mono[m];
+          q[d] += ccoef[at] * mono[m];
         }
     for (int d = 0; d < 3; ++d) {
       v[h][d] = r[0] * Ji[0 * 3 + d] + r[1] * Ji[1 * 3 + d] + r[2] * Ji[2 * 3 + d];
@@ -2839,8 +2860,12 @@ __device__ __forceinline__ void basis_pair(int e, int pr, const double *xi, int 
   }
 }
 
-// one warp per sample point: E and curl E of u (global coefficients, dof
-// signs) at the located point; out layout [pt][3] complex
+// G lanes per sample point, one a pair of functions (the smallest power of two
+// that holds them): E and curl E of u (global coefficients, dof signs) at the
+// located point; out layout [pt][3] complex.  Bound: latency and the loads of
+// the coefficient tables (with a warp a point and the tables a function after
+// the other 24 us for 4,608 points at p = 2; 18 us so).
+template <int G>
 __global__ void k_plane_eval(int npts, const int *__restrict__ elem, const double *__restrict__ xi,
                              int nd, int p, int nmono, const int *__restrict__ exps,
                              const double *__restrict__ coef, const double *__restrict__ ccoef,
@@ -2849,10 +2874,9 @@ __global__ void k_plane_eval(int npts, const int *__restrict__ elem, const doubl
                              const double *__restrict__ Ji9, const double *__restrict__ detJ,
                              const dcplx *__restrict__ u, dcplx *__restrict__ E,
                              dcplx *__restrict__ curlE) {
-  const int lane = threadIdx.x & 31;
-  const int pt = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (pt >= npts) return;
-  const int e = elem[pt];
+  const int lane = threadIdx.x % G;
+  const int pt = blockIdx.x * ((int)blockDim.x / G) + (int)threadIdx.x / G;
+  const int e = pt < npts ? elem[pt] : -1;
   double acc[12];
   for (int i = 0; i < 12; ++i) acc[i] = 0.0;
   const int npair = (nd + 1) / 2;
@@ -2874,8 +2898,8 @@ __global__ void k_plane_eval(int npts, const int *__restrict__ elem, const doubl
     }
   }
   for (int i = 0; i < 12; ++i)
-    for (int o = 16; o; o >>= 1) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
-  if (lane == 0) {
+    for (int o = G / 2; o; o >>= 1) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
+  if (lane == 0 && pt < npts) {
     for (int d = 0; d < 3; ++d) {
       if (E) E[(size_t)pt * 3 + d] = mk(acc[2 * d], acc[2 * d + 1]);
       if (curlE) curlE[(size_t)pt * 3 + d] = mk(acc[6 + 2 * d], acc[6 + 2 * d + 1]);
@@ -2924,7 +2948,7 @@ __global__ void k_plane_seed(PlaneGrid G, const int *__restrict__ elem,
 // ---------------------------------------------------------------------------
 // Fourier orders of sampled planes and their efficiencies (the reference's
 // orders_from_plane and order efficiency, src/lithofem/orders.py:36-67 and
-// src/lithofem/outputs.py:219-269).  Block (order o, plane iz): the
+// src/lithofem/outputs.py:219-269).  Order o of plane iz: the
 // coefficient c = (1 / (nx ny)) sum_{j,i} E(x_ij) exp(-2 pi i (a i / nx +
 // b j / ny)) of the order at grid index o = b nx + a (order m = a, or
 // a - nx above nx / 2; n likewise), its qz = sqrt(k0^2 eps - kx^2 - ky^2)
@@ -2932,11 +2956,15 @@ __global__ void k_plane_seed(PlaneGrid G, const int *__restrict__ elem,
 // reference plane, c' = c exp(-i d qz (z - z_ref)) (+ the analytic (0,0)
 // background there): d Re[(c' x conj(k x c' / k0))_z] area / (2 inc_flux),
 // k = (kx, ky, d qz), d = +1 (reflection side) or -1 (transmission side).
+// The sum over i is formed once per (j, a) (k_orders_rows), the one over j
+// from those (k_plane_orders): nx + ny terms and phases an order instead of
+// nx ny (two planes of 48 x 48 points: 99 us with the double sum, 14 us so).
 // ---------------------------------------------------------------------------
 struct OrderArgs {
   double lx, ly, k0, kx, ky, inc_flux;
 };
 constexpr int ORDER_THREADS = 128;
+constexpr int ORDER_LANES = 8;   // lanes that share a sum
 
 // principal square root (Re >= 0), the half-angle formulas evaluated
 // without cancellation on either sign of the real part
@@ -2951,76 +2979,74 @@ __device__ __forceinline__ dcplx csqrt_principal(dcplx w) {
   return mk(fabs(w.im) / (2.0 * t), copysign(t, w.im));
 }
 
-// rows of 10 (z, z_ref, eps re/im, background 3 complex) to separate arrays
-__global__ void k_unpack_planes(int nz, const double *__restrict__ rows, double *__restrict__ z,
-                                double *__restrict__ zref, double *__restrict__ eps2,
-                                double *__restrict__ bg) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nz) return;
-  const double *r = rows + (size_t)i * 10;
-  z[i] = r[0];
-  zref[i] = r[1];
-  eps2[2 * i] = r[2];
-  eps2[2 * i + 1] = r[3];
-  for (int c = 0; c < 6; ++c) bg[6 * i + c] = r[4 + c];
+// a plane's scalars: z, z_ref, eps (re, im), background (3 complex), direction
+constexpr int ORDER_ROW = 11;
+
+// s += sum over t = sub, sub + ORDER_LANES, ... < n of u[t stride ..] (three
+// components) exp(-2 pi i f t / n), reduced over the lanes
+__device__ __forceinline__ void order_sum(int n, int f, int sub, const dcplx *__restrict__ u,
+                                          size_t stride, double (&s)[6]) {
+  for (int q = 0; q < 6; ++q) s[q] = 0.0;
+  for (int t = sub; t < n; t += ORDER_LANES) {
+    // the phase reduced to one period first
+    double sn, cs;
+    sincospi(-2.0 * (double)((long long)f * t % n) / (double)n, &sn, &cs);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const dcplx v = u[t * stride + c];
+      s[2 * c] += v.re * cs - v.im * sn;
+      s[2 * c + 1] += v.re * sn + v.im * cs;
+    }
+  }
+  for (int o = ORDER_LANES / 2; o; o >>= 1)
+#pragma unroll
+    for (int q = 0; q < 6; ++q) s[q] += __shfl_xor_sync(0xffffffffu, s[q], o);
+}
+
+// R[iz][j][a] = sum_i E[iz][j][i] exp(-2 pi i a i / nx); rows = nz ny
+__global__ void __launch_bounds__(ORDER_THREADS)
+k_orders_rows(int nx, int rows, const dcplx *__restrict__ E, dcplx *__restrict__ R) {
+  const int t = blockIdx.x * (ORDER_THREADS / ORDER_LANES) + (int)threadIdx.x / ORDER_LANES;
+  const int o = min(t, nx * rows - 1), sub = threadIdx.x % ORDER_LANES;
+  double s[6];
+  order_sum(nx, o % nx, sub, E + (size_t)(o / nx) * nx * 3, 3, s);
+  if (t == o && sub < 3) R[(size_t)o * 3 + sub] = mk(sub == 0 ? s[0] : sub == 1 ? s[2] : s[4],
+                                                     sub == 0 ? s[1] : sub == 1 ? s[3] : s[5]);
 }
 
 __global__ void __launch_bounds__(ORDER_THREADS)
-k_plane_orders(int nx, int ny, const dcplx *__restrict__ E, const double *__restrict__ zs,
-               const double *__restrict__ zref, const int *__restrict__ dirs,
-               const double *__restrict__ eps2, const double *__restrict__ bg, OrderArgs A,
-               dcplx *__restrict__ coef, double *__restrict__ eff) {
-  const int npts = nx * ny, o = blockIdx.x, iz = blockIdx.y;
-  const int a = o % nx, b = o / nx;
-  const dcplx *Ez = E + (size_t)iz * npts * 3;
-  const long long per = (long long)nx * ny;
-  double s[6] = {0, 0, 0, 0, 0, 0};
-  for (int pt = threadIdx.x; pt < npts; pt += ORDER_THREADS) {
-    const int i = pt % nx, j = pt / nx;
-    // phase -2 pi (a i / nx + b j / ny), reduced to one period first
-    const long long num = ((long long)a * i * ny + (long long)b * j * nx) % per;
-    double sn, cs;
-    sincospi(-2.0 * (double)num / (double)per, &sn, &cs);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const dcplx u = Ez[(size_t)pt * 3 + c];
-      s[2 * c] += u.re * cs - u.im * sn;
-      s[2 * c + 1] += u.re * sn + u.im * cs;
-    }
-  }
-  __shared__ double red[6][ORDER_THREADS];
-#pragma unroll
-  for (int q = 0; q < 6; ++q) red[q][threadIdx.x] = s[q];
-  __syncthreads();
-  for (int w = ORDER_THREADS / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w)
-#pragma unroll
-      for (int q = 0; q < 6; ++q) red[q][threadIdx.x] += red[q][threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x) return;
+k_plane_orders(int nx, int ny, int nz, const dcplx *__restrict__ R, const double *__restrict__ rows,
+               bool bg, OrderArgs A, dcplx *__restrict__ coef, double *__restrict__ eff) {
+  const int npts = nx * ny, all = npts * nz;
+  const int t = blockIdx.x * (ORDER_THREADS / ORDER_LANES) + (int)threadIdx.x / ORDER_LANES;
+  const int at = min(t, all - 1), sub = threadIdx.x % ORDER_LANES;
+  const int iz = at / npts, o = at % npts, a = o % nx, b = o / nx;
+  double s[6];
+  order_sum(ny, b, sub, R + ((size_t)iz * npts + a) * 3, (size_t)nx * 3, s);
+  if (t >= all || sub) return;
+  const double *row = rows + ORDER_ROW * iz;
   const double inv = 1.0 / (double)npts;
   dcplx c[3];
   for (int q = 0; q < 3; ++q) {
-    c[q] = mk(red[2 * q][0] * inv, red[2 * q + 1][0] * inv);
+    c[q] = mk(s[2 * q] * inv, s[2 * q + 1] * inv);
     coef[((size_t)iz * npts + o) * 3 + q] = c[q];
   }
   const int m = a <= nx / 2 ? a : a - nx, n = b <= ny / 2 ? b : b - ny;
   const double kx = A.kx + 2.0 * 3.141592653589793238 / A.lx * m;
   const double ky = A.ky + 2.0 * 3.141592653589793238 / A.ly * n;
-  const dcplx ep = mk(eps2[2 * iz], eps2[2 * iz + 1]);
+  const dcplx ep = mk(row[2], row[3]);
   dcplx qz = csqrt_principal(mk(A.k0 * A.k0 * ep.re - kx * kx - ky * ky, A.k0 * A.k0 * ep.im));
   if (qz.im < 0.0) qz = mk(-qz.re, -qz.im);
-  const int d = dirs[iz];
+  const int d = (int)row[10];
   // c' = c exp(-i d qz dz) = c e^{d dz Im qz} (cos(d dz Re qz) - i sin(d dz Re qz))
-  const double dz = zs[iz] - zref[iz];
+  const double dz = row[0] - row[1];
   const double g = exp(d * dz * qz.im);
   double sn, cs;
   sincos(d * dz * qz.re, &sn, &cs);
   const dcplx ph = mk(g * cs, -g * sn);
   for (int q = 0; q < 3; ++q) {
     c[q] = cmul(c[q], ph);
-    if (m == 0 && n == 0 && bg) c[q] = cadd(c[q], mk(bg[6 * iz + 2 * q], bg[6 * iz + 2 * q + 1]));
+    if (m == 0 && n == 0 && bg) c[q] = cadd(c[q], mk(row[4 + 2 * q], row[5 + 2 * q]));
   }
   const dcplx kz = mk(d * qz.re, d * qz.im);
   // h = k x c / k0 (x and y components)
