@@ -1068,15 +1068,9 @@ int ensure_lanes(lfsolve *s) {
   int rc;
   if ((rc = lu_clusters<cuComplex>(&s->lu_cluster[LFSOLVE_C64]))) return rc;
   if ((rc = lu_clusters<cuDoubleComplex>(&s->lu_cluster[LFSOLVE_C128]))) return rc;
-  LS_CUDA(cudaFuncSetAttribute(k_leaf<cuComplex, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  LS_CUDA(cudaFuncSetAttribute(k_leaf<cuComplex>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)sizeof(LeafSmem<cuComplex>)));
-  LS_CUDA(cudaFuncSetAttribute(k_leaf<cuComplex, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)sizeof(LeafSmem<cuComplex>)));
-  LS_CUDA(cudaFuncSetAttribute(k_leaf<cuDoubleComplex, true>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)sizeof(LeafSmem<cuDoubleComplex>)));
-  LS_CUDA(cudaFuncSetAttribute(k_leaf<cuDoubleComplex, false>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize,
+  LS_CUDA(cudaFuncSetAttribute(k_leaf<cuDoubleComplex>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)sizeof(LeafSmem<cuDoubleComplex>)));
   LS_CUDA(cudaFuncSetAttribute(k_diag_inverse<cuComplex>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1159,32 +1153,6 @@ int group_product(cublasHandle_t h, const Group<T> &G, int m, int n, int p0, int
   return LFSOLVE_OK;
 }
 
-// one side of the update blocks: leaves and the products between them
-template <typename T, bool LEFT>
-int group_side(cudaStream_t st, cublasHandle_t h, const Group<T> &G) {
-  const int nl = (G.kk + LEAF - 1) / LEAF, ld = G.ld;
-  for (int i = 1; i <= nl; ++i) {
-    k_leaf<T, LEFT><<<dim3((unsigned)((G.r + LEAF_C - 1) / LEAF_C), (unsigned)G.cnt), LEAF_T,
-                      sizeof(LeafSmem<T>), st>>>(G, (i - 1) * LEAF);
-    LS_CUDA(cudaGetLastError());
-    if (i == nl) break;
-    const int t = i & -i, p0 = (i - t) * LEAF, pk = t * LEAF, q0 = i * LEAF;
-    const int qn = std::min(G.kk, std::min(nl, i + t) * LEAF) - q0;
-    T *F = G.F;
-    int rc;
-    if (LEFT)
-      rc = group_product<T>(h, G, qn, G.r, p0, pk, F + q0 + (long long)p0 * ld,
-                            F + p0 + (long long)G.kk * ld, F + q0 + (long long)G.kk * ld, G.AF, q0,
-                            G.BU, 0);
-    else
-      rc = group_product<T>(h, G, G.r, qn, p0, pk, F + G.kk + (long long)p0 * ld,
-                            F + p0 + (long long)q0 * ld, F + G.kk + (long long)q0 * ld, G.AL, 0,
-                            G.BF, q0);
-    if (rc) return rc;
-  }
-  return LFSOLVE_OK;
-}
-
 // floats of split operands a front needs
 inline size_t split_floats(int kk, int r) {
   return (size_t)18 * kk * ((size_t)kk + r);
@@ -1194,6 +1162,7 @@ inline size_t split_floats(int kk, int r) {
 // cores with the split operands there (cnt x split_floats), null: in T
 template <typename T>
 int group_update(cudaStream_t st, cublasHandle_t h, Group<T> G, float *buf) {
+  const int nl = (G.kk + LEAF - 1) / LEAF, ld = G.ld;
   if (buf) {
     float *at = buf;
     auto operand = [&](long long ld, long long n) {
@@ -1205,18 +1174,30 @@ int group_update(cudaStream_t st, cublasHandle_t h, Group<T> G, float *buf) {
     G.BF = operand(0, (long long)G.kk * G.kk);
     G.AL = operand(2LL * G.r, 2LL * G.r * G.kk);
     G.BU = operand(0, (long long)G.kk * G.r);
-    const int nl = (G.kk + LEAF - 1) / LEAF;
     if (nl > 1) {
-      k_split_f11<T><<<dim3((unsigned)(nl - 1), (unsigned)(nl - 1), (unsigned)G.cnt), LEAF_T, 0, st>>>(G);
+      k_split_f11<T><<<dim3((unsigned)(nl - 1), (unsigned)(nl - 1), (unsigned)G.cnt), SPLIT_T, 0, st>>>(G);
       LS_CUDA(cudaGetLastError());
     }
   }
-  int rc = group_side<T, true>(st, h, G);
-  if (rc || (rc = group_side<T, false>(st, h, G))) return rc;
   T *F = G.F;
-  rc = group_product<T>(h, G, G.r, G.r, 0, G.kk, F + G.kk, F + (long long)G.kk * G.ld,
-                        F + G.kk + (long long)G.kk * G.ld, G.AL, 0, G.BU, 0);
-  return rc;
+  int rc;
+  for (int i = 1; i <= nl; ++i) {
+    k_leaf<T><<<dim3((unsigned)((G.r + LEAF_C<T> - 1) / LEAF_C<T>), (unsigned)G.cnt, 2), LEAF_T,
+                sizeof(LeafSmem<T>), st>>>(G, (i - 1) * LEAF);
+    LS_CUDA(cudaGetLastError());
+    if (i == nl) break;
+    const int t = i & -i, p0 = (i - t) * LEAF, pk = t * LEAF, q0 = i * LEAF;
+    const int qn = std::min(G.kk, std::min(nl, i + t) * LEAF) - q0;
+    if ((rc = group_product<T>(h, G, qn, G.r, p0, pk, F + q0 + (long long)p0 * ld,
+                               F + p0 + (long long)G.kk * ld, F + q0 + (long long)G.kk * ld, G.AF, q0,
+                               G.BU, 0)) ||
+        (rc = group_product<T>(h, G, G.r, qn, p0, pk, F + G.kk + (long long)p0 * ld,
+                               F + p0 + (long long)q0 * ld, F + G.kk + (long long)q0 * ld, G.AL, 0,
+                               G.BF, q0)))
+      return rc;
+  }
+  return group_product<T>(h, G, G.r, G.r, 0, G.kk, F + G.kk, F + (long long)G.kk * ld,
+                          F + G.kk + (long long)G.kk * ld, G.AL, 0, G.BU, 0);
 }
 
 // how a depth's fronts are taken: step fronts at once (batched), or one a lane

@@ -27,8 +27,10 @@
 // in one product of depth 6 k left residuals twice as large (1.7e-3 against
 // 0.9e-3 unrefined on a 111k-row contact hole).
 constexpr int LEAF = 64;
-constexpr int LEAF_T = 256;
-constexpr int LEAF_C = 64;      // columns of F12 (rows of F21) a block takes
+constexpr int LEAF_T = 128;
+constexpr int SPLIT_T = 256;
+// columns of F12 (rows of F21) a block takes: three (complex128: two) blocks a SM
+template <typename T> constexpr int LEAF_C = sizeof(T) == 8 ? 64 : 32;
 
 // a group of cnt fronts: front f at F + f S, kk pivot rows (dummies included),
 // r update rows (padding included), leading dimension ld; split operands (null
@@ -88,13 +90,13 @@ __device__ __forceinline__ void put_right(const Operand &, int, int, int, int, i
 // split operands of L11 (below its leaves) and U11 (right of them): block =
 // (leaf, 64 rows or columns further on), front blockIdx.z
 template <typename T>
-__global__ void __launch_bounds__(LEAF_T) k_split_f11(const Group<T> G) {
+__global__ void __launch_bounds__(SPLIT_T) k_split_f11(const Group<T> G) {
   const int p0 = blockIdx.x * LEAF, q0 = (blockIdx.x + 1 + blockIdx.y) * LEAF;
   if (q0 >= G.kk) return;
   const int qn = min(LEAF, G.kk - q0);  // a leaf with others after it is full
   const T *F = G.F + blockIdx.z * G.S;
   const int f = blockIdx.z;
-  for (int t = threadIdx.x; t < LEAF * LEAF; t += LEAF_T) {
+  for (int t = threadIdx.x; t < LEAF * LEAF; t += SPLIT_T) {
     const int i = t % LEAF, l = t / LEAF;
     if (i < qn)
       put_left(G.AF, G.cnt, f, p0, LEAF, q0 + i, l, F[q0 + i + (long long)(p0 + l) * G.ld]);
@@ -105,60 +107,81 @@ __global__ void __launch_bounds__(LEAF_T) k_split_f11(const Group<T> G) {
 
 template <typename T> struct LeafSmem {
   T D[LEAF][LEAF + 1];          // the leaf's triangle: inverses on the diagonal, zero beyond
-  T X[LEAF][LEAF_C + 1];        // pivots x columns (left) or pivots x rows (right)
+  T X[LEAF][LEAF_C<T> + 1];     // pivots x columns (left) or pivots x rows (right)
 };
 
-// X[o0 .. o0 + 32) (+)= sum over l in [l0, l0 + 32) of coef(o, l) X[l], a
-// thread per 2 pivots x 4 columns; base: the value the sum starts from
+// X[o0 .. o0 + 32) (-)= sum over l in [l0, l0 + 32) of coef(o, l) X[l], a
+// thread per 4 pivots x LEAF_C / 16 columns; SUB: taken from X as it is, else
+// a triangle, whose zero 8 x 8 blocks are left out
 template <typename T, bool SUB, class C>
 __device__ __forceinline__ void leaf_product(LeafSmem<T> &sm, int o0, int l0, C coef) {
+  constexpr int NB = LEAF_C<T> / 16;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  T acc[2][4];
+  T acc[4][NB];
 #pragma unroll
-  for (int a = 0; a < 2; ++a)
+  for (int a = 0; a < 4; ++a)
 #pragma unroll
-    for (int b = 0; b < 4; ++b)
-      acc[a][b] = SUB ? sm.X[o0 + ty + 16 * a][tx + 16 * b] : czero<T>();
-#pragma unroll 4
-  for (int l = 0; l < 32; ++l) {
-    T d[2], x[4];
+    for (int b = 0; b < NB; ++b)
+      acc[a][b] = SUB ? sm.X[o0 + ty + 8 * a][tx + 16 * b] : czero<T>();
 #pragma unroll
-    for (int a = 0; a < 2; ++a) d[a] = coef(o0 + ty + 16 * a, l0 + l);
+  for (int q = 0; q < 4; ++q)
+#pragma unroll 2
+    for (int l = 8 * q; l < 8 * q + 8; ++l) {
+      T d[4], x[NB];
 #pragma unroll
-    for (int b = 0; b < 4; ++b) x[b] = sm.X[l0 + l][tx + 16 * b];
+      for (int a = SUB ? 0 : q; a < 4; ++a) d[a] = coef(o0 + ty + 8 * a, l0 + l);
 #pragma unroll
-    for (int a = 0; a < 2; ++a)
+      for (int b = 0; b < NB; ++b) x[b] = sm.X[l0 + l][tx + 16 * b];
 #pragma unroll
-      for (int b = 0; b < 4; ++b)
-        if (SUB) acc[a][b] = cfms(acc[a][b], d[a], x[b]);
-        else cfma(acc[a][b], d[a], x[b]);
-  }
+      for (int a = SUB ? 0 : q; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < NB; ++b)
+          if (SUB) acc[a][b] = cfms(acc[a][b], d[a], x[b]);
+          else cfma(acc[a][b], d[a], x[b]);
+    }
   __syncthreads();
 #pragma unroll
-  for (int a = 0; a < 2; ++a)
+  for (int a = 0; a < 4; ++a)
 #pragma unroll
-    for (int b = 0; b < 4; ++b) sm.X[o0 + ty + 16 * a][tx + 16 * b] = acc[a][b];
+    for (int b = 0; b < NB; ++b) sm.X[o0 + ty + 8 * a][tx + 16 * b] = acc[a][b];
   __syncthreads();
 }
 
-// one leaf (pivots p0 .. p0 + kb) of 64 columns of F12 (LEFT) or 64 rows of F21
 template <typename T, bool LEFT>
-__global__ void __launch_bounds__(LEAF_T) k_leaf(const Group<T> G, int p0) {
-  extern __shared__ __align__(16) unsigned char leaf_raw[];
-  LeafSmem<T> &sm = *reinterpret_cast<LeafSmem<T> *>(leaf_raw);
-  const int kb = min(LEAF, G.kk - p0), c0 = blockIdx.x * LEAF_C, nc = min(LEAF_C, G.r - c0);
+__device__ __forceinline__ void leaf_side(const Group<T> &G, int p0, LeafSmem<T> &sm) {
+  constexpr int NC = LEAF_C<T>, B = 64 / sizeof(T);   // loads of a thread in flight
+  const int kb = min(LEAF, G.kk - p0), c0 = blockIdx.x * NC, nc = min(NC, G.r - c0);
   T *F = G.F + blockIdx.y * G.S;
   const T *D = F + p0 + (long long)p0 * G.ld;
   // F12 rows p0 .., columns c0 ..; F21 rows c0 .., columns p0 ..
   T *X = LEFT ? F + p0 + (long long)(G.kk + c0) * G.ld : F + G.kk + c0 + (long long)p0 * G.ld;
-  for (int t = threadIdx.x; t < LEAF * LEAF; t += LEAF_T) {
-    const int i = t % LEAF, l = t / LEAF;     // i along a column of memory
-    T v = czero<T>();
-    if (i < kb && l < kb && (LEFT ? i > l : i <= l)) v = D[i + (long long)l * G.ld];
-    if (LEFT && i == l) v = CT<T>::mk(1.0, 0.0);
-    sm.D[i][l] = v;
-    if (LEFT) sm.X[i][l] = i < kb && l < nc ? X[i + (long long)l * G.ld] : czero<T>();
-    else sm.X[l][i] = l < kb && i < nc ? X[i + (long long)l * G.ld] : czero<T>();
+  for (int t0 = threadIdx.x; t0 < LEAF * LEAF; t0 += B * LEAF_T) {
+    T v[B];
+#pragma unroll
+    for (int u = 0; u < B; ++u) {
+      const int t = t0 + u * LEAF_T, i = t % LEAF, l = t / LEAF;   // i along a column of memory
+      v[u] = i < kb && l < kb && (LEFT ? i > l : i <= l) ? D[i + (long long)l * G.ld] : czero<T>();
+    }
+#pragma unroll
+    for (int u = 0; u < B; ++u) {
+      const int t = t0 + u * LEAF_T, i = t % LEAF, l = t / LEAF;
+      sm.D[i][l] = LEFT && i == l ? CT<T>::mk(1.0, 0.0) : v[u];
+    }
+  }
+  constexpr int XI = LEFT ? LEAF : NC;   // entries along a column of memory
+  for (int t0 = threadIdx.x; t0 < LEAF * NC; t0 += B * LEAF_T) {
+    T v[B];
+#pragma unroll
+    for (int u = 0; u < B; ++u) {
+      const int t = t0 + u * LEAF_T, i = t % XI, l = t / XI;
+      v[u] = (LEFT ? i < kb && l < nc : l < kb && i < nc) ? X[i + (long long)l * G.ld] : czero<T>();
+    }
+#pragma unroll
+    for (int u = 0; u < B; ++u) {
+      const int t = t0 + u * LEAF_T, i = t % XI, l = t / XI;
+      if (LEFT) sm.X[i][l] = v[u];
+      else sm.X[l][i] = v[u];
+    }
   }
   __syncthreads();
   // X = L^-1 X by halves: X_0 = L_00^-1 X_0; X_1 = L_11^-1 (X_1 - L_10 X_0);
@@ -169,8 +192,9 @@ __global__ void __launch_bounds__(LEAF_T) k_leaf(const Group<T> G, int p0) {
     leaf_product<T, true>(sm, 32, 0, coef);
     leaf_product<T, false>(sm, 32, 32, coef);
   }
-  for (int t = threadIdx.x; t < LEAF * LEAF_C; t += LEAF_T) {
-    const int i = t % LEAF, l = t / LEAF;
+#pragma unroll 4
+  for (int t = threadIdx.x; t < LEAF * NC; t += LEAF_T) {
+    const int i = t % XI, l = t / XI;
     if (LEFT) {
       if (i >= kb || l >= nc) continue;
       const T v = sm.X[i][l];
@@ -183,4 +207,18 @@ __global__ void __launch_bounds__(LEAF_T) k_leaf(const Group<T> G, int p0) {
       if (G.AL.p) put_left(G.AL, G.cnt, blockIdx.y, p0, kb, c0 + i, l, v);
     }
   }
+}
+
+// One leaf (pivots p0 .. p0 + kb) of every front of the group: F12
+// (blockIdx.z = 0) and F21 in one launch, LEAF_C columns (rows) a block.
+// Bound: FP32 (FP64) FMA issue and the stores of the split operands, about
+// equal.  Kernel time over a factorization with a launch a side, 2 pivots a
+// thread and whole 32 x 32 triangles, and so: 113 and 69 ms (complex64,
+// 524k-row line grating), 12.7 and 6.9 ms (complex128, 111k-row hole).
+template <typename T>
+__global__ void __launch_bounds__(LEAF_T, sizeof(T) == 8 ? 3 : 2) k_leaf(const Group<T> G, int p0) {
+  extern __shared__ __align__(16) unsigned char leaf_raw[];
+  LeafSmem<T> &sm = *reinterpret_cast<LeafSmem<T> *>(leaf_raw);
+  if (blockIdx.z == 0) leaf_side<T, true>(G, p0, sm);
+  else leaf_side<T, false>(G, p0, sm);
 }
