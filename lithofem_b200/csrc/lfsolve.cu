@@ -40,6 +40,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <map>
 #include <memory>
 #include <numeric>
 #include <string>
@@ -92,8 +93,15 @@ inline int pad_up(int x) { return (x + FPAD - 1) / FPAD * FPAD; }
 constexpr int MAX_NRHS_PASS = 2;  // right-hand sides per solve pass
 constexpr int SWEEP_BLOCKS = 1184;  // blocks of a sweep phase that fill the GPU (8 a SM)
 constexpr int LANES = 8;          // streams (and library handles) for the fronts
-constexpr int BATCH_MIN = 128;    // depths with this many fronts use batched calls,
-constexpr double BATCH_PADDING = 1.25;  // and those whose fronts padding grows by less
+// What a group of cnt fronts padded to kp pivots and rp update rows is taken to
+// cost, in seconds: per leaf of 64 pivots its launches, and its flops and its
+// entries at the rates of mid-sized fronts.  Fronts share a group where that
+// is the cheaper (group_fronts).  With whole depths as one group where padding
+// grew them by less than a quarter, or from 128 fronts on, and a front a group
+// else, and so: 298 and 278 ms (complex64, 524k-row line grating), 60.3 and
+// 57.9 ms (complex128, 111k-row hole), 4.2 and 3.3 ms (6k-row slab).
+constexpr double GROUP_LEAF_S = 20e-6, GROUP_FLOPS = 6e13, GROUP_ENTRIES = 1.5e11;
+constexpr int GROUP_SHAPES = 64;  // shapes of a depth that are told apart, at most
 // complex64 fronts whose Schur update F22 -= L21 U12 has at least this many
 // complex multiply-adds use three TF32 tensor-core GEMMs on split operands
 constexpr double TF32X3_MIN_MACS = 2e9;
@@ -122,8 +130,8 @@ struct Node {
   long long vec_off = 0;      // solve vector block offset (rows)
   int el0 = 0, el1 = 0;       // element range (leaves)
   int ld = 0;                 // leading dimension of its front in the arena
-  int roff = 0;               // front row of its first update row (k, or the
-                              // padded pivot count of a batched depth)
+  int roff = 0;               // front row of its first update row (its group's
+                              // padded pivot count)
 };
 
 // host array of n values left uninitialised (filled by the caller), the
@@ -140,6 +148,11 @@ struct HostBuf {
   size_t size() const { return n; }
   bool empty() const { return n == 0; }
 };
+
+// cnt fronts of a depth taken together on a uniform padded layout: kp pivot
+// rows (dummy identity pivots after the real ones), rp update rows (zero rows
+// after the real ones), one every `stride` entries of the arena from `off` on
+struct FrontGroup { int cnt, kp, rp; long long off, stride; };
 
 // largest rows, pivots and update rows of a depth's fronts
 struct SolveShape { int m = 0, k = 0, r = 0; };
@@ -158,12 +171,7 @@ struct Plan {
   std::vector<int> r_orig;            // update rows (original indices), node blocks
   std::vector<int> rel;               // rows of each child in its parent front
   std::vector<int> rel_fac;           // the same in the parent's (padded) front layout
-  // depths with many fronts are factored by batched calls on a uniform
-  // padded layout: kpad pivot rows (dummy identity pivots after the real
-  // ones), rpad update rows (zero rows after the real ones), stride per front
-  std::vector<char> batched;
-  std::vector<int> kpad, rpad;
-  std::vector<long long> stride;
+  std::vector<std::vector<FrontGroup>> groups;  // per depth
   std::vector<int> ess;
   // assembly map per depth: CSR position -> arena offset
   std::vector<HostBuf<int>> asm_src;        // every entry is written: no zero fill
@@ -269,6 +277,61 @@ inline int host_workers(int n) {
   return std::max(1, std::min((int)std::min(32u, std::max(1u, std::thread::hardware_concurrency())), n));
 }
 
+// The fronts of one depth in groups that are factored together (FrontGroup):
+// fronts of the same padded shape, and then, pair by pair, the groups whose
+// union costs less than the two.  all: from so many fronts on one group, else
+// a front a group (0: by cost).
+std::vector<std::vector<int>> group_fronts(const Plan &P, const std::vector<int> &fronts, int all) {
+  std::vector<std::vector<int>> out;
+  if (all) {
+    if ((int)fronts.size() >= all) return {fronts};
+    for (int s : fronts) out.push_back({s});
+    return out;
+  }
+  struct Shape { int k = 0, r = 0; std::vector<int> ids; };
+  std::vector<Shape> G;
+  for (int grain = FPAD;; grain *= 2) {
+    std::map<std::pair<int, int>, Shape> by;
+    for (int s : fronts) {
+      const int k = P.nodes[s].k, r = P.nodes[s].m - k;
+      Shape &Z = by[{(k + grain - 1) / grain, (r + grain - 1) / grain}];
+      Z.k = std::max(Z.k, k);
+      Z.r = std::max(Z.r, r);
+      Z.ids.push_back(s);
+    }
+    if ((int)by.size() > GROUP_SHAPES) continue;
+    for (auto &kv : by) G.push_back(std::move(kv.second));
+    break;
+  }
+  auto cost = [](double k, double r, double cnt) {
+    return GROUP_LEAF_S * (1.0 + std::ceil(k / 64)) +
+           cnt * (8.0 * (k * k * k / 3.0 + k * k * r + k * r * r) / GROUP_FLOPS +
+                  (k + r) * (k + r) / GROUP_ENTRIES);
+  };
+  auto gain = [&](const Shape &a, const Shape &b) {
+    const double na = a.ids.size(), nb = b.ids.size();
+    return cost(a.k, a.r, na) + cost(b.k, b.r, nb) -
+           cost(std::max(a.k, b.k), std::max(a.r, b.r), na + nb);
+  };
+  while (G.size() > 1) {
+    double best = 0.0;
+    size_t bi = 0, bj = 0;
+    for (size_t i = 0; i < G.size(); ++i)
+      for (size_t j = i + 1; j < G.size(); ++j) {
+        const double g = gain(G[i], G[j]);
+        if (g > best) { best = g; bi = i; bj = j; }
+      }
+    if (best <= 0.0) break;
+    G[bi].k = std::max(G[bi].k, G[bj].k);
+    G[bi].r = std::max(G[bi].r, G[bj].r);
+    G[bi].ids.insert(G[bi].ids.end(), G[bj].ids.begin(), G[bj].ids.end());
+    G.erase(G.begin() + bj);
+  }
+  for (Shape &Z : G) out.push_back(std::move(Z.ids));
+  return out;
+}
+
+
 int build_plan(int n, const int *I, const int *J, long long nnz, int ne, int nd,
                const int *edof, const double *cen, const int *ess, int n_ess, int leaf,
                Plan &P) {
@@ -367,31 +430,30 @@ int build_plan(int n, const int *I, const int *J, long long nnz, int ne, int nd,
   P.by_depth.assign(P.max_depth + 1, {});
   for (int s : P.post) P.by_depth[P.nodes[s].depth].push_back(s);
   P.arena_size.assign(P.max_depth + 1, 0);
-  P.batched.assign(P.max_depth + 1, 0);
-  P.kpad.assign(P.max_depth + 1, 0);
-  P.rpad.assign(P.max_depth + 1, 0);
-  P.stride.assign(P.max_depth + 1, 0);
-  // LFSOLVE_BATCH_MIN overrides the front count from which a depth is batched
-  int batch_min = BATCH_MIN;
+  P.groups.assign(P.max_depth + 1, {});
+  // LFSOLVE_BATCH_MIN: depths of so many fronts as one group, others a front a group
   const char *batch_env = std::getenv("LFSOLVE_BATCH_MIN");
-  if (batch_env) batch_min = std::max(1, std::atoi(batch_env));
   for (int d = 0; d <= P.max_depth; ++d) {
-    const int cnt = (int)P.by_depth[d].size();
-    int kp = 0, rp = 0;
-    double real = 0.0;  // entries of the fronts as they are
-    for (int s : P.by_depth[d]) {
-      kp = std::max(kp, P.nodes[s].k);
-      rp = std::max(rp, P.nodes[s].m - P.nodes[s].k);
-      real += (double)P.nodes[s].m * P.nodes[s].m;
+    const int all = batch_env ? std::max(1, std::atoi(batch_env)) : 0;
+    for (const std::vector<int> &ids : group_fronts(P, P.by_depth[d], all)) {
+      FrontGroup G{(int)ids.size(), 0, 0, P.arena_size[d], 0};
+      int r = 0;
+      for (int s : ids) {
+        G.kp = std::max(G.kp, pad_up(P.nodes[s].k));
+        r = std::max(r, P.nodes[s].m - P.nodes[s].k);
+      }
+      G.rp = pad_up(r);
+      const long long ld = G.kp + G.rp;
+      G.stride = align_up(ld * ld);
+      for (int s : ids) {
+        Node &N = P.nodes[s];
+        N.arena_off = P.arena_size[d];
+        N.ld = (int)ld;
+        N.roff = G.kp;
+        P.arena_size[d] += G.stride;
+      }
+      P.groups[d].push_back(G);
     }
-    kp = pad_up(kp);
-    const long long ld = pad_up(kp + rp);
-    const bool alike = !batch_env && cnt > 1 && (double)ld * ld * cnt <= BATCH_PADDING * real;
-    if (kp == 0 || (cnt < batch_min && !alike)) continue;
-    P.batched[d] = 1;
-    P.kpad[d] = kp;
-    P.rpad[d] = (int)ld - kp;
-    P.stride[d] = align_up(ld * ld);
   }
   long long fac = 0, roff = 0, vec = 0;
   P.shape.assign(P.max_depth + 1, {});
@@ -402,18 +464,6 @@ int build_plan(int n, const int *I, const int *J, long long nnz, int ne, int nd,
       Z.m = std::max(Z.m, N.m);
       Z.k = std::max(Z.k, N.k);
       Z.r = std::max(Z.r, N.m - N.k);
-      N.arena_off = P.arena_size[d];
-      if (P.batched[d]) {
-        N.ld = P.kpad[d] + P.rpad[d];
-        N.roff = P.kpad[d];
-        P.arena_size[d] += P.stride[d];
-      } else {
-        // dummy identity pivots k .. roff-1 after the real ones, zero rows
-        // and columns past the update rows up to ld
-        N.roff = pad_up(N.k);
-        N.ld = pad_up(N.roff + (N.m - N.k));
-        P.arena_size[d] += align_up((long long)N.ld * N.ld);
-      }
       N.fac_off = fac;
       const long long r = (long long)N.R.size();
       fac += align_up((long long)N.m * N.k + (long long)N.k * r);
@@ -1200,34 +1250,30 @@ int group_update(cudaStream_t st, cublasHandle_t h, Group<T> G, float *buf) {
                           F + G.kk + (long long)G.kk * ld, G.AL, 0, G.BU, 0);
 }
 
-// how a depth's fronts are taken: step fronts at once (batched), or one a lane
-// on `lanes` streams; which go through split operands, and the floats of them
-// in flight
-struct DepthPlan { int step = 1, lanes = 1; size_t floats = 0; };
+// which fronts go through split operands
 template <typename T> bool front_split(lfsolve *s, double r, double kk, double cnt) {
   return use_tf32x3<T>(s) && r * r * kk * cnt >= tf32x3_min();
 }
+// how a depth's groups are taken: on so many lanes, with so many floats of
+// split operands each, a group as many fronts at once as those hold
+struct DepthPlan { int lanes = 1; size_t floats = 0; };
 template <typename T> DepthPlan depth_plan(lfsolve *s, int d) {
-  const Plan &P = s->P;
   DepthPlan Q;
-  if (P.batched[d]) {
-    const int cnt = (int)P.by_depth[d].size(), kp = P.kpad[d], rp = P.rpad[d];
-    Q.step = std::min(cnt, 32768);
-    if (rp > 0 && front_split<T>(s, rp, kp, cnt)) {
-      const size_t per = split_floats(kp, rp);
-      Q.step = (int)std::max<size_t>(1, std::min<size_t>(Q.step, SPLIT_BYTES / (4 * per)));
-      Q.floats = per * Q.step;
-    }
-    return Q;
+  size_t largest = 0;
+  std::vector<std::pair<size_t, size_t>> split;  // floats a front, fronts
+  int busy = 0;
+  for (const FrontGroup &G : s->P.groups[d]) {
+    if (G.kp == 0 || G.rp == 0) continue;
+    ++busy;
+    if (!front_split<T>(s, G.rp, G.kp, G.cnt)) continue;
+    split.push_back({split_floats(G.kp, G.rp), (size_t)G.cnt});
+    largest = std::max(largest, split.back().first);
   }
-  size_t need = 0;
-  for (int id : P.by_depth[d]) {
-    const Node &N = P.nodes[id];
-    if (N.k > 0 && N.m > N.k && front_split<T>(s, N.ld - N.roff, N.roff, 1))
-      need = std::max(need, split_floats(N.roff, N.ld - N.roff));
-  }
-  Q.lanes = need ? (int)std::max<size_t>(1, std::min<size_t>(LANES, SPLIT_BYTES / (4 * need))) : LANES;
-  Q.floats = need * Q.lanes;
+  Q.lanes = std::max(1, std::min(busy, LANES));
+  if (!largest) return Q;
+  Q.lanes = (int)std::max<size_t>(1, std::min<size_t>(Q.lanes, SPLIT_BYTES / (4 * largest)));
+  const size_t cap = std::max(largest, SPLIT_BYTES / 4 / Q.lanes);
+  for (auto &g : split) Q.floats = std::max(Q.floats, g.first * std::min(g.second, cap / g.first));
   return Q;
 }
 
@@ -1367,7 +1413,7 @@ int factor_impl(lfsolve *s, const double2 *vals) {
   for (int d = 0; d < D; ++d) {
     plan[d] = depth_plan<T>(s, d);
     need[d & 1] = std::max(need[d & 1], (size_t)P.arena_size[d] * sizeof(T));
-    floats = std::max(floats, plan[d].floats);
+    floats = std::max(floats, plan[d].floats * plan[d].lanes);
   }
   int rc;
   for (int i = 0; i < 2; ++i)
@@ -1410,31 +1456,29 @@ int factor_impl(lfsolve *s, const double2 *vals) {
       LS_CUDA(cudaGetLastError());
     }
     const DepthPlan &Q = plan[d];
-    if (P.batched[d]) {  // the uniform padded layout
-      const int kp = P.kpad[d], rp = P.rpad[d];
-      for (int f0 = 0; rp > 0 && f0 < cnt; f0 += Q.step) {
-        const Group<T> G{arena[d] + f0 * P.stride[d], P.stride[d], std::min(Q.step, cnt - f0), kp, rp,
-                         kp + rp, {}, {}, {}, {}};
-        if ((rc = group_update<T>(st, s->blas_main, G, Q.floats ? split_buf : nullptr))) return rc;
+    // the groups with most work first, spread over the lanes
+    std::vector<FrontGroup> order;
+    for (const FrontGroup &G : P.groups[d])
+      if (G.kp > 0 && G.rp > 0) order.push_back(G);
+    auto work = [](const FrontGroup &G) { return (double)G.cnt * G.kp * G.rp * (G.kp + G.rp); };
+    std::sort(order.begin(), order.end(),
+              [&](const FrontGroup &a, const FrontGroup &b) { return work(a) > work(b); });
+    const bool fork = Q.lanes > 1;
+    if (fork && (rc = fork_lanes(s))) return rc;
+    int li = 0;
+    for (const FrontGroup &g : order) {
+      const int l = li++ % Q.lanes;
+      const bool split = front_split<T>(s, g.rp, g.kp, g.cnt);
+      const int step = split ? (int)std::min<size_t>(32768, Q.floats / split_floats(g.kp, g.rp)) : 32768;
+      for (int f0 = 0; f0 < g.cnt; f0 += step) {
+        const Group<T> G{arena[d] + g.off + f0 * g.stride, g.stride, std::min(step, g.cnt - f0), g.kp,
+                         g.rp, g.kp + g.rp, {}, {}, {}, {}};
+        if ((rc = group_update<T>(fork ? s->lane[l] : st, fork ? s->blas[l] : s->blas_main, G,
+                                  split ? split_buf + l * Q.floats : nullptr)))
+          return rc;
       }
-    } else {
-      // largest fronts first, spread over the lanes
-      std::vector<int> order;
-      for (int id : P.by_depth[d])
-        if (P.nodes[id].k > 0 && P.nodes[id].m > P.nodes[id].k) order.push_back(id);
-      std::sort(order.begin(), order.end(),
-                [&](int a, int b) { return P.nodes[a].m > P.nodes[b].m; });
-      if ((rc = fork_lanes(s))) return rc;
-      int li = 0;
-      for (int id : order) {
-        const Node &N = P.nodes[id];
-        const int l = li++ % Q.lanes, kk = N.roff, r = N.ld - N.roff;
-        const Group<T> G{arena[d] + N.arena_off, 0, 1, kk, r, N.ld, {}, {}, {}, {}};
-        float *buf = front_split<T>(s, r, kk, 1) ? split_buf + l * (Q.floats / Q.lanes) : nullptr;
-        if ((rc = group_update<T>(s->lane[l], s->blas[l], G, buf))) return rc;
-      }
-      if ((rc = join_lanes(s))) return rc;
     }
+    if (fork && (rc = join_lanes(s))) return rc;
     if (s->n_co[d] > 0) {
       k_copy_out<T><<<s->n_co[d], 256, 0, st>>>(s->d_co[d], s->d_nodes, arena[d], fac);
       LS_CUDA(cudaGetLastError());
