@@ -102,6 +102,11 @@ constexpr int LANES = 8;          // streams (and library handles) for the front
 // 57.9 ms (complex128, 111k-row hole), 4.2 and 3.3 ms (6k-row slab).
 constexpr double GROUP_LEAF_S = 20e-6, GROUP_FLOPS = 6e13, GROUP_ENTRIES = 1.5e11;
 constexpr int GROUP_SHAPES = 64;  // shapes of a depth that are told apart, at most
+// pivot rows left, squared, times fronts from which the next panel is factored
+// beside a step's update (never, from 3e6, 1e6, 3e5 on: 279.6, 266.1, 265.7,
+// 266.3 ms in complex64 on a 524k-row line grating; 57.7, 57.3, 56.8, 56.5 ms
+// in complex128 on a 111k-row hole)
+constexpr double LU_AHEAD_MIN = 1e6;
 // complex64 fronts whose Schur update F22 -= L21 U12 has at least this many
 // complex multiply-adds use three TF32 tensor-core GEMMs on split operands
 constexpr double TF32X3_MIN_MACS = 2e9;
@@ -939,7 +944,8 @@ struct lfsolve {
   std::vector<int> n_ea[2], n_co;
   std::vector<int *> d_all;               // per depth: its fronts
   int *d_rel_fac = nullptr;               // child rows in the parents' front layout
-  LuSwaps *d_swaps = nullptr;             // a step's interchanges (max fronts of a depth)
+  LuSwaps *d_swaps = nullptr;             // interchanges of two steps (n_swaps: max fronts of a depth)
+  size_t n_swaps = 0;
   int *d_src = nullptr;                   // children's vector rows per vector row
   InvItem *d_inv = nullptr;               // diagonal blocks kept as inverses
   std::vector<int> inv_at;                // per depth: its first entry (and the end)
@@ -956,6 +962,9 @@ struct lfsolve {
   void *work[LANES] = {};
   size_t work_bytes[LANES] = {};
   cudaEvent_t ev_main = nullptr, ev_lane[LANES] = {};
+  // panels factored beside the update before them (lu_depth)
+  cudaStream_t ahead = nullptr;
+  cudaEvent_t ev_rest = nullptr;
   // front workspace, kept between factorizations: the fronts of the even and
   // of the odd depths (a depth reads its children's from the other one), and
   // the split operands of the fronts in flight
@@ -1044,7 +1053,8 @@ int ensure_uploaded(lfsolve *s) {
   s->d_all.assign(D, nullptr);
   size_t maxb = 1;
   for (int d = 0; d < D; ++d) maxb = std::max(maxb, P.by_depth[d].size());
-  LS_CUDA(cudaMalloc((void **)&s->d_swaps, sizeof(LuSwaps) * maxb));
+  s->n_swaps = maxb;
+  LS_CUDA(cudaMalloc((void **)&s->d_swaps, sizeof(LuSwaps) * 2 * maxb));
   for (int d = 0; d < D; ++d) {
     if ((rc = upload(&s->d_asm_src[d], P.asm_src[d], st))) return rc;
     if ((rc = upload(&s->d_asm_dst[d], P.asm_dst[d], st))) return rc;
@@ -1137,6 +1147,10 @@ int ensure_lanes(lfsolve *s) {
     LS_CUDA(cudaEventCreateWithFlags(&s->ev_lane[l], cudaEventDisableTiming));
   }
   LS_CUDA(cudaEventCreateWithFlags(&s->ev_main, cudaEventDisableTiming));
+  LS_CUDA(cudaEventCreateWithFlags(&s->ev_rest, cudaEventDisableTiming));
+  int least = 0, greatest = 0;
+  LS_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+  LS_CUDA(cudaStreamCreateWithPriority(&s->ahead, cudaStreamNonBlocking, greatest));
   LS_CUDA(cudaEventCreate(&s->t0));
   LS_CUDA(cudaEventCreate(&s->t1));
   return LFSOLVE_OK;
@@ -1302,8 +1316,42 @@ int lu_depth(lfsolve *s, int d, T *arena, int cap) {
     rmax = std::max(rmax, N.m - N.k);
   }
   const int *list = s->d_all[d];
+  auto strips = [&](cudaStream_t on, int which, int j0) -> int {
+    const int rows = kmax - j0;
+    const int n = (which == LU_NEXT ? LU_NB : kmax + LU_STRIP<T> - 1) / LU_STRIP<T>;
+    // rows of the update split where the strips alone leave SMs idle
+    const int groups = (rows - LU_NB + LU_STRIP_T - 1) / LU_STRIP_T;
+    const bool split = groups > 1 && (which == LU_NEXT ||
+                                      (long long)cnt * ((rows - 1) / LU_STRIP<T>) < 2 * 148);
+    for (int f0 = 0; f0 < cnt; f0 += 65535) {
+      const dim3 g((unsigned)n, (unsigned)std::min(65535, cnt - f0));
+      const int *li = list + f0;
+      const LuSwaps *sw = s->d_swaps + (j0 / LU_NB & 1) * s->n_swaps + f0;
+      if (!split) {
+        k_lu_strip<T, 0><<<g, LU_STRIP_T, 0, on>>>(li, s->d_nodes, arena, j0, cap, sw, which);
+      } else {
+        k_lu_strip<T, 1><<<g, LU_STRIP_T, 0, on>>>(li, s->d_nodes, arena, j0, cap, sw, which);
+        k_lu_strip<T, 2><<<dim3(g.x, g.y, (unsigned)groups), LU_STRIP_T, 0, on>>>(
+            li, s->d_nodes, arena, j0, cap, sw, which);
+      }
+      LS_CUDA(cudaGetLastError());
+    }
+    return LFSOLVE_OK;
+  };
+  // While a step's update is large, the next panel is factored beside it: its
+  // columns are updated first, on a stream of their own, and the panel (few
+  // blocks, a chain of exchanges) goes before the rest's blocks by priority.
+  // The step then takes the longer of the two instead of their sum.
+  bool ahead = false;
+  int rc;
   for (int j0 = 0; j0 < kmax; j0 += LU_NB) {
     const int rows = kmax - j0;
+    const bool was = ahead;
+    ahead = (double)cnt * rows * rows >= LU_AHEAD_MIN;  // rows shrink: on at first, then off
+    if (ahead != was) {  // the panel's stream waits for what came before, or the other way round
+      LS_CUDA(cudaEventRecord(s->ev_main, was ? s->ahead : st));
+      LS_CUDA(cudaStreamWaitEvent(was ? st : s->ahead, s->ev_main, 0));
+    }
     int csize = 1;
     // the fewest blocks that hold the rows: smaller blocks in larger clusters
     // cost more in cluster barriers than they save in issue slots (4,200 pivots
@@ -1311,28 +1359,28 @@ int lu_depth(lfsolve *s, int d, T *arena, int cap) {
     while (csize * LU_ROWS<T> < rows) csize *= 2;
     const int threads = ((rows + csize - 1) / csize + 31) / 32 * 32;
     cudaLaunchAttribute attr;
-    const cudaLaunchConfig_t cfg = lu_panel_config<T>(cnt, csize, threads, st, &attr);
+    const cudaLaunchConfig_t cfg =
+        lu_panel_config<T>(cnt, csize, threads, ahead ? s->ahead : st, &attr);
+    // two sets of interchanges: a step's strips read theirs while the next panel writes
     LS_CUDA(cudaLaunchKernelEx(&cfg, k_lu_panel<T>, list, (const NodeDev *)s->d_nodes, arena, j0,
-                               csize, cap, s->d_swaps, s->d_pperm, s->d_info));
-    const int strips = (kmax + LU_STRIP<T> - 1) / LU_STRIP<T>;
-    if (kmax > LU_NB) {
-      // rows of the update split where the strips alone leave SMs idle
-      const int groups = (rows - LU_NB + LU_STRIP_T - 1) / LU_STRIP_T;
-      const bool split = groups > 1 && (long long)cnt * ((rows - 1) / LU_STRIP<T>) < 2 * 148;
-      for (int f0 = 0; f0 < cnt; f0 += 65535) {
-        const dim3 g((unsigned)strips, (unsigned)std::min(65535, cnt - f0));
-        const int *li = list + f0;
-        const LuSwaps *sw = s->d_swaps + f0;
-        if (!split) {
-          k_lu_strip<T, 0><<<g, LU_STRIP_T, 0, st>>>(li, s->d_nodes, arena, j0, cap, sw);
-        } else {
-          k_lu_strip<T, 1><<<g, LU_STRIP_T, 0, st>>>(li, s->d_nodes, arena, j0, cap, sw);
-          k_lu_strip<T, 2><<<dim3(g.x, g.y, (unsigned)groups), LU_STRIP_T, 0, st>>>(
-              li, s->d_nodes, arena, j0, cap, sw);
-        }
-        LS_CUDA(cudaGetLastError());
-      }
+                               csize, cap, s->d_swaps + (j0 / LU_NB & 1) * s->n_swaps, s->d_pperm,
+                               s->d_info));
+    if (kmax <= LU_NB) break;
+    if (!ahead) {
+      if ((rc = strips(st, LU_ALL, j0))) return rc;
+      continue;
     }
+    LS_CUDA(cudaEventRecord(s->ev_main, s->ahead));
+    // the next panel's columns carry the rest of the step before
+    if (was) LS_CUDA(cudaStreamWaitEvent(s->ahead, s->ev_rest, 0));
+    if ((rc = strips(s->ahead, LU_NEXT, j0))) return rc;
+    LS_CUDA(cudaStreamWaitEvent(st, s->ev_main, 0));
+    if ((rc = strips(st, LU_REST, j0))) return rc;
+    LS_CUDA(cudaEventRecord(s->ev_rest, st));
+  }
+  if (ahead) {
+    LS_CUDA(cudaEventRecord(s->ev_main, s->ahead));
+    LS_CUDA(cudaStreamWaitEvent(st, s->ev_main, 0));
   }
   if (kmax > 1 && rmax > 0) {
     const size_t per = (size_t)kmax * sizeof(T);
@@ -2096,6 +2144,8 @@ void lfsolve_destroy(lfsolve *s) {
   }
   if (s->blas_main) cublasDestroy(s->blas_main);
   if (s->ev_main) cudaEventDestroy(s->ev_main);
+  if (s->ev_rest) cudaEventDestroy(s->ev_rest);
+  if (s->ahead) cudaStreamDestroy(s->ahead);
   if (s->t0) cudaEventDestroy(s->t0);
   if (s->t1) cudaEventDestroy(s->t1);
   delete s;

@@ -211,14 +211,16 @@ k_lu_panel(const int *__restrict__ list, const NodeDev *__restrict__ nodes, T *a
   if (csize > 1) cooperative_groups::this_cluster().sync();  // no block leaves while others push to it
 }
 
-// strip blockIdx.x of the columns outside the panel, front blockIdx.y.
-// PART 0: all of it; where fronts x strips leave SMs idle, PART 1 does the
+// strips of the columns outside the panel, front blockIdx.y: all of them, the
+// next panel's, or all but those (lu_depth).
+enum { LU_ALL, LU_NEXT, LU_REST };
+// PART 0: a whole strip; where fronts x strips leave SMs idle, PART 1 does the
 // exchange and U_j, and PART 2 the update with the rows split over blockIdx.z
 // (a 2,528-pivot front alone: 118 us a step in one part, its first step).
 template <typename T, int PART>
 __global__ void __launch_bounds__(LU_STRIP_T, 2)
 k_lu_strip(const int *__restrict__ list, const NodeDev *__restrict__ nodes, T *arena, int j0,
-           int cap, const LuSwaps *__restrict__ swaps) {
+           int cap, const LuSwaps *__restrict__ swaps, int which) {
   constexpr int SC = LU_STRIP<T>;
   __shared__ __align__(16) T X[LU_NB][SC];     // the pivot rows of the strip, then U_j
   __shared__ T L[LU_NB][LU_NB + 1];            // L_jj
@@ -226,7 +228,9 @@ k_lu_strip(const int *__restrict__ list, const NodeDev *__restrict__ nodes, T *a
   const int f = blockIdx.y, id = list[f];
   const NodeDev N = nodes[id];
   const int k = N.k, nb = min(LU_NB, k - j0), ld = N.ld;
-  const int q0 = blockIdx.x * SC;
+  const int first = j0 / SC, strip = blockIdx.x;
+  const int q0 = SC * (which == LU_NEXT ? first + strip
+                       : which == LU_REST && strip >= first ? strip + LU_NB / SC : strip);
   if (nb <= 0 || k > cap || q0 >= k - nb) return;
   const bool right = q0 >= j0;                 // j0 is a multiple of the strip width
   if (PART == 2 && !right) return;
