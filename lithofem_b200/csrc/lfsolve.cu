@@ -1138,6 +1138,10 @@ int ensure_lanes(lfsolve *s) {
   LS_CUDA(cudaFuncSetAttribute(k_diag_inverse<cuDoubleComplex>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)inv_smem<cuDoubleComplex>()));
+  for (auto kern : {k_sweep_tri<1, 0, 0>, k_sweep_tri<1, 0, 1>, k_sweep_tri<1, 1, 0>,
+                    k_sweep_tri<1, 1, 1>, k_sweep_tri<2, 0, 0>, k_sweep_tri<2, 0, 1>,
+                    k_sweep_tri<2, 1, 0>, k_sweep_tri<2, 1, 1>})
+    LS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TRI_SMEM));
   for (int l = 0; l < LANES; ++l) {
     LS_CUDA(cudaStreamCreateWithFlags(&s->lane[l], cudaStreamNonBlocking));
     LS_BLAS(cublasCreate(&s->blas[l]));
@@ -1555,32 +1559,64 @@ int factor_impl(lfsolve *s, const double2 *vals) {
   return LFSOLVE_OK;
 }
 
-// one launch of a phase over the fronts of a depth, at most nch chunks each in
-// nz parts; it may start while the launch before it is still running
-template <typename T, int NR, int TRANS, int PH>
-int sweep_phase(const Sweep<T> &S, int nch, int fronts, int j0, cudaStream_t st, int nz = 1) {
-  if (nch <= 0) return LFSOLVE_OK;
+// one launch that may start while the launch before it is still running
+template <typename T>
+int sweep_launch(void (*kern)(Sweep<T>, int), const Sweep<T> &S, dim3 grid, size_t smem, int j0,
+                 cudaStream_t st) {
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(SW_T);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  LS_CUDA(cudaLaunchKernelEx(&cfg, kern, S, j0));
+  return LFSOLVE_OK;
+}
+
+// Depths of at most so many fronts are bound by the latency of a step's two
+// phases and take the kernels that hold their factors on chip; with more, HBM
+// is the bound, and blocks that stream them with more of their kind on an SM
+// are the faster (524k-row line grating, held and streamed, forward + backward:
+// 1 front 0.29 and 0.68 ms, 4 fronts 0.56 and 0.70, 16 fronts 0.36 and 0.39,
+// 32 fronts 0.47 and 0.48, 64 fronts 0.45 and 0.42, 256 fronts 0.31 and 0.27).
+constexpr int HELD_FRONTS = 32;
+
+// one launch of a phase over the fronts of a depth, at most nch chunks each in
+// nz parts
+template <typename T, int NR, int TRANS, int PH>
+int sweep_phase(const Sweep<T> &S, int nch, int fronts, int j0, cudaStream_t st, int nz = 1) {
+  if (nch <= 0) return LFSOLVE_OK;
+  constexpr bool FWD = PH == PH_FWD_A || PH == PH_FWD_B;
   // grid.y holds 65,535 fronts
   for (int f0 = 0; f0 < fronts; f0 += 65535) {
     Sweep<T> P = S;
     P.list = S.list + f0;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)nch, (unsigned)std::min(65535, fronts - f0), (unsigned)nz);
-    cfg.blockDim = dim3(SW_T);
-    cfg.stream = st;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    LS_CUDA(cudaLaunchKernelEx(&cfg, k_sweep<T, NR, TRANS, PH>, P, j0));
+    const unsigned nf = (unsigned)std::min(65535, fronts - f0);
+    const dim3 grid((unsigned)nch, nf, (unsigned)nz);
+    void (*kern)(Sweep<T>, int) = k_sweep<T, NR, TRANS, PH>;
+    size_t smem = 0;
+    if constexpr (sizeof(T) == 8) {
+      if constexpr (PH == PH_FWD_A || PH == PH_BWD_A)
+        if (fronts <= HELD_FRONTS) kern = k_sweep_tri<NR, TRANS, !FWD>, smem = TRI_SMEM;
+      if constexpr (PH == PH_FWD_B || PH == PH_BWD_B)
+        if (fronts <= HELD_FRONTS) kern = k_sweep_apply<NR, TRANS, !FWD>;
+    }
+    if (int rc = sweep_launch<T>(kern, P, grid, smem, j0, st)) return rc;
   }
   return LFSOLVE_OK;
 }
 
-// A block per front walks through its phases where that fills the GPU or the
-// fronts are so small that launches would dominate; else a launch per phase.
-bool front_per_block(size_t fronts, int max_m) { return fronts >= 512 || max_m <= 160; }
+// A block per front walks through its phases where that fills the GPU evenly
+// (three blocks a SM: 512 fronts of 1,029 rows take 0.30 ms so, 0.21 ms by
+// phases; of 282 rows they are too small for phases) or the fronts are so small
+// that launches would dominate; else a launch per phase.
+bool front_per_block(size_t fronts, int max_m) {
+  return fronts >= 1024 || (fronts >= 512 && max_m <= 512) || max_m <= 160;
+}
 
 // one pass of NR columns: b (n x NR, ld n, precision T, original numbering)
 // -> x (same layout)

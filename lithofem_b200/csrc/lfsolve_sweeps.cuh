@@ -577,6 +577,213 @@ __global__ void __launch_bounds__(SW_T) k_sweep(const Sweep<T> S, int j0) {
   if (PH == PH_BWD_B) F.bwd_b(j0, ch);
 }
 
+// The same for the two phases of a step of few fronts in complex64, where a
+// block can hold its part of the factors: all of it is on chip before the phase before is
+// waited for, and what is left is arithmetic and the vectors' latency.
+//
+// k_sweep_tri: a step's triangle, a block a front.  The 28 off-diagonal 32 x 32
+// blocks in shared memory (224 kB of the 227 an SM has), every warp's inverse
+// in its registers.  Warp s multiplies by its inverse, and hands its 32 results
+// to the warps after it over a barrier of its own, so that no warp waits for
+// one that is behind it.  The results lie where the warp's last used block was.
+// A step (triangle and columns) of a 271k-row line grating's root front: 26 us
+// with the links loaded a link ahead and a block-wide barrier each, 7 us so.
+constexpr int TRI_TILE = 32 * 32;
+constexpr size_t TRI_SMEM = (size_t)(28 * TRI_TILE + 128) * sizeof(cuComplex);
+__device__ __forceinline__ int tri_tile(int a, int b) {
+  const int hi = max(a, b), lo = min(a, b);
+  return (hi * (hi - 1) / 2 + lo) * TRI_TILE;
+}
+__device__ __forceinline__ void tri_copy(cuComplex *dst, const cuComplex *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                   (unsigned)__cvta_generic_to_shared(dst)), "l"(src));
+}
+template <int NR, int TRANS, int BWD>
+__global__ void __launch_bounds__(SW_T, 1) k_sweep_tri(const Sweep<cuComplex> S, int j0) {
+  using T = cuComplex;
+  extern __shared__ __align__(16) unsigned char tri_raw[];
+  T *tiles = reinterpret_cast<T *>(tri_raw);
+  cudaTriggerProgrammaticLaunchCompletion();
+  const NodeDev N = S.nodes[S.list[blockIdx.y]];
+  const int k = N.k, m = N.m, t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const int nb = min(SB, k - j0), links = (nb + 31) / 32;
+  const bool on = nb > 0;
+  const T *D = S.fac + N.fac_off + j0 + (long long)j0 * m;
+  T own[32];
+  if (on) {
+    // block (w2, s2): rows (TRANS: columns) of warp w2 against link s2, four of
+    // its lines a warp; lanes along the contiguous rows of D, so that transposed
+    // blocks are swizzled
+    T *dst = tiles;
+    for (int hi = 1; hi < links; ++hi)
+      for (int lo = 0; lo < hi; ++lo, dst += TRI_TILE) {
+        const int w2 = BWD ? lo : hi, s2 = BWD ? hi : lo;
+        // row and column of D of this lane's entry of line w
+        const int row = 32 * (TRANS ? s2 : w2) + lane, col = 32 * (TRANS ? w2 : s2) + w;
+        const T *src = D + row + (long long)col * m;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int i = w + 8 * u;
+          T *to = dst + (TRANS ? lane * 32 + (i ^ lane) : i * 32 + lane);
+          if (row < nb && col + 8 * u < nb) tri_copy(to, src + (long long)(8 * u) * m);
+          else *to = czero<T>();
+        }
+      }
+#pragma unroll
+    for (int l = 0; l < 32; ++l) {
+      const int o = 32 * w + l;
+      const bool in = TRANS ? (BWD ? l > lane : l <= lane) : (BWD ? l >= lane : l < lane);
+      own[l] = in && t < nb && o < nb ? D[TRANS ? o + (long long)t * m : t + (long long)o * m] : czero<T>();
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+  }
+  cudaGridDependencySynchronize();
+  if (!on || w >= links) return;
+  T v[NR];
+#pragma unroll
+  for (int q = 0; q < NR; ++q)
+    v[q] = t >= nb ? czero<T>()
+           : BWD   ? S.Y[N.p0 + j0 + t + (long long)q * S.nn]
+                   : S.V[N.vec_off + j0 + t + q * S.VR];
+  // the results of link s: 32 NR entries after as many of the warp's input
+  auto slot = [&](int s) {
+    const int first = BWD ? links - 1 : 0;
+    return s == first ? tiles + 28 * TRI_TILE : tiles + tri_tile(s, BWD ? s + 1 : s - 1);
+  };
+  const int before = BWD ? links - 1 - w : w;   // links this warp takes results from
+  for (int u = 0; u < before; ++u) {
+    const int s = BWD ? links - 1 - u : u;
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + s), "r"(32 * (links - u)) : "memory");
+    const T *y = slot(s) + 32 * NR, *c = tiles + tri_tile(w, s);
+    T o[NR];
+#pragma unroll
+    for (int q = 0; q < NR; ++q) o[q] = czero<T>();
+#pragma unroll
+    for (int l = 0; l < 32; ++l) {
+      const T a = c[l * 32 + (TRANS ? lane ^ l : lane)];
+#pragma unroll
+      for (int q = 0; q < NR; ++q) cfma(o[q], a, y[l * NR + q]);
+    }
+#pragma unroll
+    for (int q = 0; q < NR; ++q) v[q] = csub(v[q], o[q]);
+  }
+  {
+    T *in = slot(w), *y = in + 32 * NR;
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < NR; ++q) in[lane * NR + q] = v[q];
+    __syncwarp();
+    T o[NR];
+#pragma unroll
+    for (int q = 0; q < NR; ++q) o[q] = (TRANS == BWD) ? v[q] : czero<T>();  // unit diagonal of L
+#pragma unroll
+    for (int l = 0; l < 32; ++l)
+#pragma unroll
+      for (int q = 0; q < NR; ++q) cfma(o[q], own[l], in[l * NR + q]);
+#pragma unroll
+    for (int q = 0; q < NR; ++q) {
+      v[q] = o[q];
+      y[lane * NR + q] = o[q];
+    }
+    if (before + 1 < links)
+      asm volatile("bar.arrive %0, %1;" ::"r"(1 + w), "r"(32 * (links - before)) : "memory");
+  }
+  if (t >= nb) return;
+  if (!BWD) {
+#pragma unroll
+    for (int q = 0; q < NR; ++q) S.Y[N.p0 + j0 + t + (long long)q * S.nn] = v[q];
+    return;
+  }
+  const int g = S.perm[N.p0 + (TRANS ? S.pperm[N.p0 + j0 + t] : j0 + t)];
+#pragma unroll
+  for (int q = 0; q < NR; ++q) {
+    S.V[N.vec_off + j0 + t + q * S.VR] = v[q];
+    S.x[(long long)q * S.n + g] = v[q];
+  }
+}
+
+// k_sweep_apply: a step's columns on SW_CHUNK rows (A^T: columns) outside its
+// triangle, 32 entries a thread in registers
+template <int NR, int TRANS, int BWD>
+__global__ void __launch_bounds__(SW_T) k_sweep_apply(const Sweep<cuComplex> S, int j0) {
+  using T = cuComplex;
+  __shared__ SweepSmem<T, NR> sm;
+  cudaTriggerProgrammaticLaunchCompletion();
+  const NodeDev N = S.nodes[S.list[blockIdx.y]];
+  const int k = N.k, m = N.m, t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const int nb = min(SB, k - j0), j1 = j0 + nb;
+  // the rows (columns) of the pivot block's step it applies to: [r0, r1)
+  const int r0 = (BWD ? 0 : j1) + (int)blockIdx.x * SW_CHUNK, r1 = BWD ? j0 : TRANS ? k : m;
+  const bool on = nb > 0 && r0 < r1;
+  const T *P = S.fac + N.fac_off;
+  T a[32];
+  if (on) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      // rows: column w + 8 i of the step; columns: column w + 8 (i / 8) of the
+      // chunk, rows lane + 32 (i % 8) of the step
+      const int o = TRANS ? lane + 32 * (i & 7) : w + SW_W * i;
+      const int r = min(r0 + (TRANS ? w + SW_W * (i >> 3) : lane), r1 - 1);
+      a[i] = o < nb ? P[TRANS ? j0 + o + (long long)r * m : r + (long long)(j0 + o) * m] : czero<T>();
+    }
+  }
+  cudaGridDependencySynchronize();
+  if (!on) return;
+  T *const out = BWD ? S.Y + N.p0 : S.V + N.vec_off;
+  const long long so = BWD ? S.nn : S.VR;
+  // the entry this thread writes, and the step's vector
+  const int mine = r0 + (TRANS ? w + SW_W * lane : t);
+  const bool writes = (TRANS ? lane < SW_CHUNK / SW_W : t < SW_CHUNK) && mine < r1;
+  T old[NR];
+#pragma unroll
+  for (int q = 0; q < NR; ++q) {
+    old[q] = writes ? out[mine + q * so] : czero<T>();
+    sm.in[t * NR + q] = t >= nb ? czero<T>()
+                        : BWD   ? S.V[N.vec_off + j0 + t + q * S.VR]
+                                : S.Y[N.p0 + j0 + t + (long long)q * S.nn];
+  }
+  __syncthreads();
+  if (TRANS) {
+    T acc[4][NR];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int q = 0; q < NR; ++q) {
+        acc[u][q] = czero<T>();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) cfma(acc[u][q], a[8 * u + i], sm.in[(lane + 32 * i) * NR + q]);
+        for (int x = 16; x; x >>= 1) {
+          acc[u][q].x += __shfl_xor_sync(0xffffffffu, acc[u][q].x, x);
+          acc[u][q].y += __shfl_xor_sync(0xffffffffu, acc[u][q].y, x);
+        }
+      }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (lane == u && writes)
+#pragma unroll
+        for (int q = 0; q < NR; ++q) out[mine + q * so] = csub(old[q], acc[u][q]);
+  } else {
+    T acc[NR];
+#pragma unroll
+    for (int q = 0; q < NR; ++q) {
+      acc[q] = czero<T>();
+#pragma unroll
+      for (int i = 0; i < 32; ++i) cfma(acc[q], a[i], sm.in[(w + SW_W * i) * NR + q]);
+      sm.red[(w * SW_CHUNK + lane) * NR + q] = acc[q];
+    }
+    __syncthreads();
+    if (writes)
+#pragma unroll
+      for (int q = 0; q < NR; ++q) {
+        T v = sm.red[lane * NR + q];
+#pragma unroll
+        for (int u = 1; u < SW_W; ++u) v = cadd(v, sm.red[(u * SW_CHUNK + lane) * NR + q]);
+        out[mine + q * so] = csub(old[q], v);
+      }
+  }
+}
+
 // Inverses of the 32 x 32 blocks on the diagonals of L11 and U11 of a depth's
 // fronts, in place: a warp per (front, block), by substitution, a lane per
 // column of the inverse in registers, the block in shared memory.
