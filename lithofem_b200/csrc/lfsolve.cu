@@ -10,9 +10,9 @@
 //     postorder elimination tree, every front's index list (its pivots, then
 //     the ancestor DOFs its subtree touches) and the maps below;
 //   factor (device): depth by depth from the deepest level, the fronts of a
-//     level are zeroed, receive their original entries (CSR position ->
-//     front offset map) and their children's Schur complements (extend-add),
-//     and are partially factored: P F11 = L11 U11 with partial pivoting among
+//     level are written from their children's Schur complements, receive their
+//     original entries (CSR position -> front offset map) and are partially
+//     factored, in groups of similar shape: P F11 = L11 U11 with partial pivoting among
 //     the front's pivot rows, all fronts of the level together in own kernels
 //     (lfsolve_lu.cuh), U12 = L11^-1 P F12 and L21 = F21 U11^-1 in leaves of
 //     64 pivots with matrix products between them (lfsolve_trsm.cuh), F22 -=
@@ -175,7 +175,6 @@ struct Plan {
   long long factor_entries = 0, vec_rows = 0;
   std::vector<int> r_orig;            // update rows (original indices), node blocks
   std::vector<int> rel;               // rows of each child in its parent front
-  std::vector<int> rel_fac;           // the same in the parent's (padded) front layout
   std::vector<std::vector<FrontGroup>> groups;  // per depth
   std::vector<int> ess;
   // assembly map per depth: CSR position -> arena offset
@@ -491,7 +490,6 @@ int build_plan(int n, const int *I, const int *J, long long nnz, int ne, int nd,
   // each child's update rows located in its parent's front
   std::vector<int> loc(P.nn, -1);
   P.rel.assign(roff, 0);
-  P.rel_fac.assign(roff, 0);
   for (int s = 0; s < ns; ++s) {
     const Node &N = P.nodes[s];
     if (N.nchild == 0) continue;
@@ -504,7 +502,6 @@ int build_plan(int n, const int *I, const int *J, long long nnz, int ne, int nd,
         const int l = loc[C.R[t]];
         if (l < 0) return fail(LFSOLVE_ERR_ARG, "internal: child row missing from its parent front");
         P.rel[C.r_off + t] = l;
-        P.rel_fac[C.r_off + t] = l < N.k ? l : N.roff + (l - N.k);
       }
     }
     for (int t = 0; t < N.k; ++t) loc[N.p0 + t] = -1;
@@ -633,7 +630,13 @@ template <typename T> __device__ __forceinline__ T cfms(T a, T b, T c) {
   return a;
 }
 
-// original entries into the fronts of one depth
+struct StripItem { int node, col0; };
+struct NodeDev {  // per-node data the kernels read
+  long long arena_off, fac_off, r_off, vec_off;
+  int parent, k, m, p0, depth, ld, roff;
+};
+
+// original entries into the fronts of one depth (each position once)
 template <typename T>
 __global__ void k_assemble(long long cnt, const int *__restrict__ src,
                            const long long *__restrict__ dst, const double2 *__restrict__ vals,
@@ -641,35 +644,66 @@ __global__ void k_assemble(long long cnt, const int *__restrict__ src,
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < cnt;
        t += (long long)gridDim.x * blockDim.x) {
     const double2 v = __ldg(vals + src[t]);
-    arena[dst[t]] = CT<T>::mk(v.x, v.y);
+    T *d = arena + dst[t];
+    *d = cadd(*d, CT<T>::mk(v.x, v.y));
   }
 }
 
-// Extend-add of one child slot: item = (child node, first column of a strip
-// of 32 update columns); F_parent[rel[a], rel[b]] += U_child[a, b].
-struct EaItem { int child, col0; };
-struct NodeDev {  // per-node data the kernels read
-  long long arena_off, fac_off, r_off, vec_off;
-  int parent, k, m, p0, depth, ld, roff;
-};
+// Every entry of a depth's fronts, from the children's update blocks: item =
+// (front, first of a strip of 32 columns of its padded layout).  The entry of
+// rows a and b is the sum over the children that have both (src: the child's
+// vector row of a front's row, -1: none), the diagonal of a dummy pivot is one,
+// all else zero.  A thread keeps its row's places in the children over the
+// strip.  Bound: HBM; each entry is written once and each child entry read
+// once.  (Zeroed, then added to by a launch a child: 22.6 ms of a factorization
+// of a 524k-row line grating in complex64, 11.7 ms so.)
+constexpr int BUILD_T = 256, BUILD_C = 32;
 template <typename T>
-__global__ void k_extend_add(const EaItem *__restrict__ items, const NodeDev *__restrict__ nodes,
-                             const int *__restrict__ rel, const T *__restrict__ child_arena,
-                             T *__restrict__ arena) {
-  const EaItem it = items[blockIdx.x];
-  const NodeDev C = nodes[it.child];
-  const NodeDev Pn = nodes[C.parent];
-  const int r = C.m - C.k;
-  const T *U = child_arena + C.arena_off + C.roff + (long long)C.roff * C.ld;  // child's F22
-  T *F = arena + Pn.arena_off;
-  const int *rl = rel + C.r_off;  // child rows in the parent's front layout
-  const int c1 = min(it.col0 + 32, r);
-  for (int b = it.col0; b < c1; ++b) {
-    const long long cb = (long long)rl[b] * Pn.ld;
-    const T *Ub = U + (long long)b * C.ld;
-    for (int a = threadIdx.x; a < r; a += blockDim.x) {
-      T *f = F + rl[a] + cb;
-      *f = cadd(*f, Ub[a]);
+__global__ void __launch_bounds__(BUILD_T)
+k_build_fronts(const StripItem *__restrict__ items, const NodeDev *__restrict__ nodes,
+               const int *__restrict__ child, const int2 *__restrict__ src,
+               const T *__restrict__ child_arena, T *__restrict__ arena) {
+  __shared__ int col[2][BUILD_C];   // the strip's columns in the children, -1: none
+  const StripItem it = items[blockIdx.x];
+  const NodeDev N = nodes[it.node];
+  const int c[2] = {child[2 * it.node], child[2 * it.node + 1]};
+  const T *U[2] = {nullptr, nullptr};   // the children's F22
+  int ld[2] = {0, 0}, base[2] = {0, 0};
+#pragma unroll
+  for (int q = 0; q < 2; ++q)
+    if (c[q] >= 0) {
+      const NodeDev C = nodes[c[q]];
+      U[q] = child_arena + C.arena_off + C.roff + (long long)C.roff * C.ld;
+      ld[q] = C.ld;
+      base[q] = (int)C.vec_off + C.k;
+    }
+  // a row of the padded layout in the children (update rows of each)
+  auto places = [&](int i, int (&p)[2]) {
+    const int v = i < N.k ? i : i >= N.roff && i - N.roff < N.m - N.k ? N.k + i - N.roff : -1;
+    const int2 s = v < 0 ? make_int2(-1, -1) : src[N.vec_off + v];
+    p[0] = s.x < 0 ? -1 : s.x - base[0];
+    p[1] = s.y < 0 ? -1 : s.y - base[1];
+  };
+  const int nc = min(BUILD_C, N.ld - it.col0);
+  if (threadIdx.x < nc) {
+    int p[2];
+    places(it.col0 + threadIdx.x, p);
+    col[0][threadIdx.x] = p[0];
+    col[1][threadIdx.x] = p[1];
+  }
+  __syncthreads();
+  T *F = arena + N.arena_off + (long long)it.col0 * N.ld;
+  for (int i = threadIdx.x; i < N.ld; i += BUILD_T) {
+    int p[2];
+    places(i, p);
+    const int one = i >= N.k && i < N.roff ? i - it.col0 : -1;
+#pragma unroll 4
+    for (int j = 0; j < nc; ++j) {
+      const int a = col[0][j], b = col[1][j];
+      T v = CT<T>::mk(j == one ? 1.0 : 0.0, 0.0);
+      if (p[0] >= 0 && a >= 0) v = U[0][p[0] + (long long)a * ld[0]];
+      if (p[1] >= 0 && b >= 0) v = cadd(v, U[1][p[1] + (long long)b * ld[1]]);
+      F[i + (long long)j * N.ld] = v;
     }
   }
 }
@@ -677,10 +711,10 @@ __global__ void k_extend_add(const EaItem *__restrict__ items, const NodeDev *__
 // copy the L and U blocks of the factored fronts to the factor store:
 // P = F[:, 0:k] (m x k) then U12 = F[0:k, k:m] (k x r); item = (node, col0)
 template <typename T>
-__global__ void k_copy_out(const EaItem *__restrict__ items, const NodeDev *__restrict__ nodes,
+__global__ void k_copy_out(const StripItem *__restrict__ items, const NodeDev *__restrict__ nodes,
                            const T *__restrict__ arena, T *__restrict__ fac) {
-  const EaItem it = items[blockIdx.x];
-  const NodeDev N = nodes[it.child];
+  const StripItem it = items[blockIdx.x];
+  const NodeDev N = nodes[it.node];
   const T *F = arena + N.arena_off;
   T *Pf = fac + N.fac_off;
   T *U12 = Pf + (long long)N.m * N.k;
@@ -717,17 +751,6 @@ __global__ void k_swap_cols(int k, int ncol, const int *__restrict__ ipiv, T *__
       col[p] = t;
     }
   }
-}
-
-// dummy identity pivots of each front (rows / columns k .. roff-1), one
-// block per front of the depth (list in arena order)
-template <typename T>
-__global__ void k_dummy_diag(const int *__restrict__ list, const NodeDev *__restrict__ nodes,
-                             T *__restrict__ arena) {
-  const NodeDev N = nodes[list[blockIdx.x]];
-  T *F = arena + N.arena_off;
-  for (int i = N.k + threadIdx.x; i < N.roff; i += blockDim.x)
-    F[i + (long long)i * N.ld] = CT<T>::mk(1.0, 0.0);
 }
 
 // y = A x (or A^T x through the transposed positions) in FP64, a warp per
@@ -936,14 +959,13 @@ struct lfsolve {
   lfsolve_stats st{};
   // device copies of the plan
   NodeDev *d_nodes = nullptr;
-  int *d_child = nullptr, *d_rel = nullptr, *d_perm = nullptr, *d_rorig = nullptr,
+  int *d_child = nullptr, *d_perm = nullptr, *d_rorig = nullptr,
       *d_ess = nullptr, *d_tpos = nullptr;
   std::vector<int *> d_asm_src;
   std::vector<long long *> d_asm_dst;
-  std::vector<EaItem *> d_ea[2], d_co;    // per depth: extend-add items per slot, copy-out items
-  std::vector<int> n_ea[2], n_co;
+  std::vector<StripItem *> d_bf, d_co;    // per depth: strips to build, to copy out
+  std::vector<int> n_bf, n_co;
   std::vector<int *> d_all;               // per depth: its fronts
-  int *d_rel_fac = nullptr;               // child rows in the parents' front layout
   LuSwaps *d_swaps = nullptr;             // interchanges of two steps (n_swaps: max fronts of a depth)
   size_t n_swaps = 0;
   int *d_src = nullptr;                   // children's vector rows per vector row
@@ -1019,8 +1041,6 @@ int ensure_uploaded(lfsolve *s) {
   int rc;
   if ((rc = upload(&s->d_nodes, nd, st))) return rc;
   if ((rc = upload(&s->d_child, child, st))) return rc;
-  if ((rc = upload(&s->d_rel, P.rel, st))) return rc;
-  if ((rc = upload(&s->d_rel_fac, P.rel_fac, st))) return rc;
   if ((rc = upload(&s->d_perm, P.perm, st))) return rc;
   if ((rc = upload(&s->d_rorig, P.r_orig, st))) return rc;
   if ((rc = upload(&s->d_ess, P.ess, st))) return rc;
@@ -1047,7 +1067,8 @@ int ensure_uploaded(lfsolve *s) {
   const int D = P.max_depth + 1;
   s->d_asm_src.assign(D, nullptr);
   s->d_asm_dst.assign(D, nullptr);
-  for (int q = 0; q < 2; ++q) { s->d_ea[q].assign(D, nullptr); s->n_ea[q].assign(D, 0); }
+  s->d_bf.assign(D, nullptr);
+  s->n_bf.assign(D, 0);
   s->d_co.assign(D, nullptr);
   s->n_co.assign(D, 0);
   s->d_all.assign(D, nullptr);
@@ -1058,20 +1079,14 @@ int ensure_uploaded(lfsolve *s) {
   for (int d = 0; d < D; ++d) {
     if ((rc = upload(&s->d_asm_src[d], P.asm_src[d], st))) return rc;
     if ((rc = upload(&s->d_asm_dst[d], P.asm_dst[d], st))) return rc;
-    std::vector<EaItem> ea[2], co;
+    std::vector<StripItem> bf, co;
     for (int id : P.by_depth[d]) {
       const Node &N = P.nodes[id];
-      for (int q = 0; q < N.nchild; ++q) {
-        const Node &C = P.nodes[N.child[q]];
-        const int r = C.m - C.k;
-        for (int c0 = 0; c0 < r; c0 += 32) ea[q].push_back({N.child[q], c0});
-      }
+      for (int c0 = 0; c0 < N.ld; c0 += BUILD_C) bf.push_back({id, c0});
       for (int c0 = 0; c0 < N.m; c0 += 32) co.push_back({id, c0});
     }
-    for (int q = 0; q < 2; ++q) {
-      if ((rc = upload(&s->d_ea[q][d], ea[q], st))) return rc;
-      s->n_ea[q][d] = (int)ea[q].size();
-    }
+    if ((rc = upload(&s->d_bf[d], bf, st))) return rc;
+    s->n_bf[d] = (int)bf.size();
     if ((rc = upload(&s->d_co[d], co, st))) return rc;
     s->n_co[d] = (int)co.size();
     if ((rc = upload(&s->d_all[d], P.by_depth[d], st))) return rc;
@@ -1480,25 +1495,19 @@ int factor_impl(lfsolve *s, const double2 *vals) {
   if (const char *e = std::getenv("LFSOLVE_LU_MAX")) lu_cap = std::min(lu_cap, std::max(0, std::atoi(e)));
   for (int d = D - 1; d >= 0; --d) {
     if (prof) LS_CUDA(cudaEventRecord(evs[2 * d], st));
-    const size_t bytes = (size_t)P.arena_size[d] * sizeof(T);
-    LS_CUDA(cudaMemsetAsync(arena[d], 0, bytes, st));
+    const int cnt = (int)P.by_depth[d].size();
+    if (s->n_bf[d] > 0) {
+      k_build_fronts<T><<<s->n_bf[d], BUILD_T, 0, st>>>(s->d_bf[d], s->d_nodes, s->d_child,
+                                                        reinterpret_cast<const int2 *>(s->d_src),
+                                                        d + 1 < D ? arena[d + 1] : nullptr, arena[d]);
+      LS_CUDA(cudaGetLastError());
+    }
     const long long na = (long long)P.asm_src[d].size();
     if (na > 0) {
       k_assemble<T><<<grid_for(na, 256), 256, 0, st>>>(na, s->d_asm_src[d], s->d_asm_dst[d], vals,
                                                        arena[d]);
       LS_CUDA(cudaGetLastError());
     }
-    if (d + 1 < D) {
-      for (int q = 0; q < 2; ++q)
-        if (s->n_ea[q][d] > 0) {
-          k_extend_add<T><<<s->n_ea[q][d], 256, 0, st>>>(s->d_ea[q][d], s->d_nodes, s->d_rel_fac,
-                                                         arena[d + 1], arena[d]);
-          LS_CUDA(cudaGetLastError());
-        }
-    }
-    const int cnt = (int)P.by_depth[d].size();
-    k_dummy_diag<T><<<cnt, 128, 0, st>>>(s->d_all[d], s->d_nodes, arena[d]);
-    LS_CUDA(cudaGetLastError());
     if ((rc = lu_depth<T>(s, d, arena[d], lu_cap)) || (rc = lu_library<T>(s, d, arena[d], lu_cap))) return rc;
     // the update blocks and the sweeps read the diagonal blocks as inverses
     const int ni = s->inv_at[d + 1] - s->inv_at[d];
@@ -2158,16 +2167,15 @@ void lfsolve_destroy(lfsolve *s) {
   if (s->stream) cudaStreamSynchronize(s->stream);
   free_factors(s);
   free_workspace(s);
-  void *bufs[] = {s->d_nodes, s->d_child, s->d_rel, s->d_perm, s->d_rorig, s->d_ess, s->d_tpos,
+  void *bufs[] = {s->d_nodes, s->d_child, s->d_perm, s->d_rorig, s->d_ess, s->d_tpos,
                   s->d_info, s->d_V, s->d_Y, s->d_part_y, s->d_bw, s->d_src, s->d_inv, s->d_r, s->d_part, s->d_scale,
                   s->d_pperm};
   for (void *p : bufs)
     if (p) cudaFree(p);
   for (auto *p : s->d_asm_src) if (p) cudaFree(p);
   for (auto *p : s->d_asm_dst) if (p) cudaFree(p);
-  for (int q = 0; q < 2; ++q) for (auto *p : s->d_ea[q]) if (p) cudaFree(p);
+  for (auto *p : s->d_bf) if (p) cudaFree(p);
   for (auto *p : s->d_co) if (p) cudaFree(p);
-  if (s->d_rel_fac) cudaFree(s->d_rel_fac);
   if (s->d_swaps) cudaFree(s->d_swaps);
   for (auto *p : s->d_all) if (p) cudaFree(p);
   for (int l = 0; l < LANES; ++l) {
