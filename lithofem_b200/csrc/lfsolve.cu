@@ -709,29 +709,28 @@ k_build_fronts(const StripItem *__restrict__ items, const NodeDev *__restrict__ 
 }
 
 // copy the L and U blocks of the factored fronts to the factor store:
-// P = F[:, 0:k] (m x k) then U12 = F[0:k, k:m] (k x r); item = (node, col0)
+// P = F[:, 0:k] (m x k) then U12 = F[0:k, k:m] (k x r); item = (node, col0).  A
+// warp a column, eight loads in flight: a block a column left most threads of
+// small fronts idle (149 us over a 6k-row slab's fronts, 92 us so).  Bound: HBM.
 template <typename T>
 __global__ void k_copy_out(const StripItem *__restrict__ items, const NodeDev *__restrict__ nodes,
                            const T *__restrict__ arena, T *__restrict__ fac) {
   const StripItem it = items[blockIdx.x];
   const NodeDev N = nodes[it.node];
+  const int lane = threadIdx.x & 31, gap = N.roff - N.k;   // dummy pivots
   const T *F = arena + N.arena_off;
   T *Pf = fac + N.fac_off;
   T *U12 = Pf + (long long)N.m * N.k;
   const int c1 = min(it.col0 + 32, N.m);
-  for (int c = it.col0; c < c1; ++c) {
+  for (int c = it.col0 + (threadIdx.x >> 5); c < c1; c += (int)blockDim.x >> 5) {
     // compact column c: a pivot column (< k) or update column c - k, which
     // sits at front column roff + c - k
-    const int fc = c < N.k ? c : N.roff + (c - N.k);
-    const T *Fc = F + (long long)fc * N.ld;
-    if (c < N.k) {
-      T *dst = Pf + (long long)c * N.m;
-      for (int a = threadIdx.x; a < N.m; a += blockDim.x)
-        dst[a] = Fc[a < N.k ? a : N.roff + (a - N.k)];
-    } else {
-      T *dst = U12 + (long long)(c - N.k) * N.k;
-      for (int a = threadIdx.x; a < N.k; a += blockDim.x) dst[a] = Fc[a];
-    }
+    const bool piv = c < N.k;
+    const T *__restrict__ Fc = F + (long long)(piv ? c : c + gap) * N.ld;
+    T *__restrict__ dst = piv ? Pf + (long long)c * N.m : U12 + (long long)(c - N.k) * N.k;
+    const int n = piv ? N.m : N.k;
+#pragma unroll 8
+    for (int a = lane; a < n; a += 32) dst[a] = Fc[a < N.k ? a : a + gap];
   }
 }
 
