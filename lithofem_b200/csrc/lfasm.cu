@@ -949,7 +949,7 @@ static int launch_bulk(lfasm_handle *h, int mask, int te, int mode, int eliminat
     const bool fused = ((mask & LFASM_CROSS0) != 0) == ((mask & LFASM_CROSS1) != 0);
     double *recm = h->rec_mma + (size_t)b0 * (fused ? BK : BREC);
     if (prep) {
-      k_prep_bulk_mma<<<(nb + 127) / 128, 128, 0, st>>>(nb, blist, h->J, h->Jinv, h->detJ,
+      k_prep_bulk_mma<<<(nb + PREP_T - 1) / PREP_T, PREP_T, 0, st>>>(nb, blist, h->J, h->Jinv, h->detJ,
                                                         h->attr, h->eps_tab, h->elem_eps, h->pml,
                                                         mask, fused ? 1 : 0, recm);
       LF_LAUNCHED();

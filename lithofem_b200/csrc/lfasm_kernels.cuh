@@ -397,15 +397,22 @@ __device__ __forceinline__ void bulk_record_fused(const double *J, const double 
       }
 }
 
-__global__ void k_prep_bulk_mma(int nb, const int *__restrict__ list,
+// A thread per element.  The fused records are formed in shared memory and
+// stored by the block as one run: a thread storing its own (256 bytes from the
+// next one's, zeroed first) took 14 us for the bulk of a 255k-row hole (40k elements in all), 6 us
+// so.  Bound: latency of the loads.
+constexpr int PREP_T = 64;
+__global__ void __launch_bounds__(PREP_T)
+k_prep_bulk_mma(int nb, const int *__restrict__ list,
                             const double *__restrict__ J9, const double *__restrict__ Ji9,
                             const double *__restrict__ detJ, const int *__restrict__ attr,
                             const dcplx *__restrict__ eps_tab,
                             const dcplx *__restrict__ elem_eps, PmlParams pml,
                             int mask, int fused, double *__restrict__ rec) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nb) return;
-  const int e = list[i];
+  __shared__ double rows[PREP_T][BK + 1];
+  const int i = blockIdx.x * PREP_T + threadIdx.x;
+  if (!fused && i >= nb) return;
+  const int e = list[min(i, nb - 1)];
   double J[9], Ji[9];
 #pragma unroll
   for (int t = 0; t < 9; ++t) {
@@ -425,8 +432,10 @@ __global__ void k_prep_bulk_mma(int nb, const int *__restrict__ list,
                          kx * kx + ky * ky};
   const double me_re = -k2 * eps.re, me_im = -k2 * eps.im;
   if (fused) {
-    bulk_record_fused(J, Ji, det, me_re, me_im, K, mKK, cc, ms, c0 && c1, kl,
-                      rec + (size_t)i * BK);
+    bulk_record_fused(J, Ji, det, me_re, me_im, K, mKK, cc, ms, c0 && c1, kl, rows[threadIdx.x]);
+    __syncthreads();
+    const int i0 = blockIdx.x * PREP_T, n = min(PREP_T, nb - i0) * BK;
+    for (int t = threadIdx.x; t < n; t += PREP_T) rec[(size_t)i0 * BK + t] = rows[t / BK][t % BK];
     return;
   }
   for (int t = 0; t < BK; ++t) { re[t] = 0.0; im[t] = 0.0; }
