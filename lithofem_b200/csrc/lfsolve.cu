@@ -1619,9 +1619,10 @@ int sweep_phase(const Sweep<T> &S, int nch, int fronts, int j0, cudaStream_t st,
 }
 
 // A block per front walks through its phases where that fills the GPU evenly
-// (three blocks a SM: 512 fronts of 1,029 rows take 0.30 ms so, 0.21 ms by
-// phases; of 282 rows they are too small for phases) or the fronts are so small
-// that launches would dominate; else a launch per phase.
+// (three blocks a SM: the 512 leaf fronts of a 271k-row line grating, more than
+// one wave, take 0.59 ms a sweep pair so and 0.52 ms by phases) or the fronts
+// are so small that launches would dominate (512 of 282 rows: a design step of
+// 40.5 ms so, 41.4 ms by phases); else a launch per phase.
 bool front_per_block(size_t fronts, int max_m) {
   return fronts >= 1024 || (fronts >= 512 && max_m <= 512) || max_m <= 160;
 }

@@ -586,8 +586,9 @@ __global__ void __launch_bounds__(SW_T) k_sweep(const Sweep<T> S, int j0) {
 // in its registers.  Warp s multiplies by its inverse, and hands its 32 results
 // to the warps after it over a barrier of its own, so that no warp waits for
 // one that is behind it.  The results lie where the warp's last used block was.
-// A step (triangle and columns) of a 271k-row line grating's root front: 26 us
-// with the links loaded a link ahead and a block-wide barrier each, 7 us so.
+// Forward sweep of a 271k-row line grating's root front (six steps, triangle and
+// columns): 114 us with the links loaded a link ahead and a block-wide barrier
+// each, 53 us so.
 constexpr int TRI_TILE = 32 * 32;
 constexpr size_t TRI_SMEM = (size_t)(28 * TRI_TILE + 128) * sizeof(cuComplex);
 __device__ __forceinline__ int tri_tile(int a, int b) {
