@@ -184,6 +184,9 @@ k_lu_panel(const int *__restrict__ list, const NodeDev *__restrict__ nodes, T *a
   const NodeDev N = nodes[id];
   const int k = N.k, nb = min(LU_NB, k - j0);
   if (nb <= 0 || k > cap) return;  // the whole cluster
+  // a block's shared memory is another block's to write only once it runs: every
+  // block reports here, and waits for the others behind its loads
+  if (csize > 1) cooperative_groups::this_cluster().barrier_arrive();
   const int tid = threadIdx.x;
   const int row = j0 + rank * (int)blockDim.x + tid;
   const bool mine = row < k;
@@ -198,6 +201,7 @@ k_lu_panel(const int *__restrict__ list, const NodeDev *__restrict__ nodes, T *a
   R.place = row;
   R.active = mine;
   int bad = 0;
+  if (csize > 1) cooperative_groups::this_cluster().barrier_wait();
   lu_columns<T, 32>(sm, R, done, 0, min(nb, 12), j0, csize, rank, bad);
   lu_columns<T, 20>(sm, R, done, 12, min(nb, 22), j0, csize, rank, bad);
   lu_columns<T, 10>(sm, R, done, 22, nb, j0, csize, rank, bad);
