@@ -25,12 +25,21 @@ constexpr int LU_STRIP_T = 256;            // threads of a strip block
 // j0 + i goes to dst[i]
 struct LuSwaps { int src[LU_NB], dst[LU_NB]; };
 
-// ordered key of |re| + |im| (its leading 32 bits; NaN above infinity)
+// ordered key of |re| + |im| (NaN above infinity), and its largest over a warp
+template <typename T> struct LuKeyOf { using type = unsigned; };
+template <> struct LuKeyOf<cuDoubleComplex> { using type = unsigned long long; };
+template <typename T> using LuKey = typename LuKeyOf<T>::type;
 __device__ __forceinline__ unsigned lu_key(cuComplex v) {
   return __float_as_uint(fabsf(v.x) + fabsf(v.y));
 }
-__device__ __forceinline__ unsigned lu_key(cuDoubleComplex v) {
-  return (unsigned)__double2hiint(fabs(v.x) + fabs(v.y));
+__device__ __forceinline__ unsigned long long lu_key(cuDoubleComplex v) {
+  return (unsigned long long)__double_as_longlong(fabs(v.x) + fabs(v.y));
+}
+__device__ __forceinline__ unsigned lu_max(unsigned k) { return __reduce_max_sync(0xffffffffu, k); }
+__device__ __forceinline__ unsigned long long lu_max(unsigned long long k) {
+  const unsigned hi = lu_max((unsigned)(k >> 32));
+  const unsigned lo = lu_max((unsigned)(k >> 32) == hi ? (unsigned)k : 0u);
+  return (unsigned long long)hi << 32 | lo;
 }
 
 // 1 / v, scaled by |re| + |im| so that neither square over- nor underflows
@@ -49,9 +58,9 @@ template <typename T> struct __align__(16) LuCand { T rp, unused, row[LU_NB]; };
 template <typename T> struct LuSmem {
   // per warp (one block) or per rank (a cluster)
   LuCand<T> cand[2][LU_ROWS<T> / 32 > LU_MAX_CLUSTER ? LU_ROWS<T> / 32 : LU_MAX_CLUSTER];
-  unsigned key[2][32];                         // per warp
+  LuKey<T> key[2][32];                         // per warp
   int tid[2][32], place[2][32];
-  unsigned ckey[2][LU_MAX_CLUSTER];            // per cluster rank
+  LuKey<T> ckey[2][LU_MAX_CLUSTER];            // per cluster rank
   int cplace[2][LU_MAX_CLUSTER];
 };
 
@@ -88,8 +97,8 @@ __device__ __forceinline__ void lu_columns(LuSmem<T> &sm, LuRow<T> &R, T *done, 
     const int b = j & 1;
     // the block's largest entry of the column (ties: the lowest thread); every
     // row works out its reciprocal while the reduction is under way
-    const unsigned key = R.active ? lu_key(R.a[0]) : 0u;
-    const unsigned best = __reduce_max_sync(0xffffffffu, key);
+    const LuKey<T> key = R.active ? lu_key(R.a[0]) : 0;
+    const LuKey<T> best = lu_max(key);
     const unsigned at = __ballot_sync(0xffffffffu, R.active && key == best);
     const T rp = lu_rcp(R.a[0]);
     auto put = [&](LuCand<T> &C) {
@@ -108,8 +117,8 @@ __device__ __forceinline__ void lu_columns(LuSmem<T> &sm, LuRow<T> &R, T *done, 
     }
     __syncthreads();
     const int wt = lane < nw ? sm.tid[b][lane] : -1;
-    const unsigned wk = wt >= 0 ? sm.key[b][lane] : 0u;
-    const unsigned top = __reduce_max_sync(0xffffffffu, wk);
+    const LuKey<T> wk = wt >= 0 ? sm.key[b][lane] : 0;
+    const LuKey<T> top = lu_max(wk);
     const unsigned from = __ballot_sync(0xffffffffu, wt >= 0 && wk == top);
     int src = __ffs(from) - 1;                       // the winning warp, -1: no row left here
     const int win = src >= 0 ? sm.tid[b][src] : -1;
@@ -139,8 +148,8 @@ __device__ __forceinline__ void lu_columns(LuSmem<T> &sm, LuRow<T> &R, T *done, 
       cl.sync();
       // the best of the blocks' rows (one is left as long as j < je)
       const int cp = lane < csize ? sm.cplace[b][lane] : -1;
-      const unsigned ck = cp >= 0 ? sm.ckey[b][lane] : 0u;
-      const unsigned ct = __reduce_max_sync(0xffffffffu, ck);
+      const LuKey<T> ck = cp >= 0 ? sm.ckey[b][lane] : 0;
+      const LuKey<T> ct = lu_max(ck);
       src = __ffs(__ballot_sync(0xffffffffu, cp >= 0 && ck == ct)) - 1;
       pl = sm.cplace[b][src];
       here = src == rank;
