@@ -111,8 +111,8 @@ template <typename T> struct LeafSmem {
 };
 
 // X[o0 .. o0 + 32) (-)= sum over l in [l0, l0 + 32) of coef(o, l) X[l], a
-// thread per 4 pivots x LEAF_C / 16 columns; SUB: taken from X as it is, else
-// a triangle, whose zero 8 x 8 blocks are left out
+// thread per 4 pivots x LEAF_C / 16 columns; SUB: the sum (formed by itself)
+// taken from X, else a triangle, whose zero 8 x 8 blocks are left out
 template <typename T, bool SUB, class C>
 __device__ __forceinline__ void leaf_product(LeafSmem<T> &sm, int o0, int l0, C coef) {
   constexpr int NB = LEAF_C<T> / 16;
@@ -121,8 +121,7 @@ __device__ __forceinline__ void leaf_product(LeafSmem<T> &sm, int o0, int l0, C 
 #pragma unroll
   for (int a = 0; a < 4; ++a)
 #pragma unroll
-    for (int b = 0; b < NB; ++b)
-      acc[a][b] = SUB ? sm.X[o0 + ty + 8 * a][tx + 16 * b] : czero<T>();
+    for (int b = 0; b < NB; ++b) acc[a][b] = czero<T>();
 #pragma unroll
   for (int q = 0; q < 4; ++q)
 #pragma unroll 2
@@ -143,7 +142,10 @@ __device__ __forceinline__ void leaf_product(LeafSmem<T> &sm, int o0, int l0, C 
 #pragma unroll
   for (int a = 0; a < 4; ++a)
 #pragma unroll
-    for (int b = 0; b < NB; ++b) sm.X[o0 + ty + 8 * a][tx + 16 * b] = acc[a][b];
+    for (int b = 0; b < NB; ++b) {
+      T &x = sm.X[o0 + ty + 8 * a][tx + 16 * b];
+      x = SUB ? cadd(x, acc[a][b]) : acc[a][b];
+    }
   __syncthreads();
 }
 
