@@ -20,10 +20,9 @@
 //     the L and U blocks are copied to the factor store;
 //   solve (device): forward and backward sweeps over the tree, each front's
 //     right-hand side gathered from the global vector and its children's
-//     update vectors (no atomics), the triangles in steps of 256 pivots with
-//     the 32 x 32 diagonal blocks kept as inverses (lfsolve_sweeps.cuh); A^T
-//     is solved with the same factors (U^T forward, L^T backward, inverse
-//     pivots last);
+//     update vectors (no atomics), the triangles in steps of 256 pivots
+//     (lfsolve_sweeps.cuh); A^T is solved with the same factors (U^T forward,
+//     L^T backward, inverse pivots last);
 //   refine: FP64 residual on the complex128 CSR, corrections from the
 //     factors, per right-hand-side column.
 #include <cublas_v2.h>
@@ -968,8 +967,8 @@ struct lfsolve {
   LuSwaps *d_swaps = nullptr;             // interchanges of two steps (n_swaps: max fronts of a depth)
   size_t n_swaps = 0;
   int *d_src = nullptr;                   // children's vector rows per vector row
-  InvItem *d_inv = nullptr;               // diagonal blocks kept as inverses
-  std::vector<int> inv_at;                // per depth: its first entry (and the end)
+  DiagItem *d_diag = nullptr;             // 32 x 32 diagonal blocks of the fronts
+  std::vector<int> diag_at;               // per depth: its first entry (and the end)
   // factors
   int prec = -1;
   void *d_fac = nullptr;
@@ -1054,15 +1053,15 @@ int ensure_uploaded(lfsolve *s) {
         src[2 * (size_t)(N.vec_off + P.rel[C.r_off + t]) + q] = (int)(C.vec_off + C.k + t);
     }
   }
-  std::vector<InvItem> inv;
-  s->inv_at.assign(1, 0);
+  std::vector<DiagItem> diag;
+  s->diag_at.assign(1, 0);
   for (const auto &fronts : P.by_depth) {
     for (int i : fronts)
-      for (int j0 = 0; j0 < P.nodes[i].k; j0 += 32) inv.push_back({i, j0});
-    s->inv_at.push_back((int)inv.size());
+      for (int j0 = 0; j0 < P.nodes[i].k; j0 += 32) diag.push_back({i, j0});
+    s->diag_at.push_back((int)diag.size());
   }
   if ((rc = upload(&s->d_src, src, st))) return rc;
-  if ((rc = upload(&s->d_inv, inv, st))) return rc;
+  if ((rc = upload(&s->d_diag, diag, st))) return rc;
   const int D = P.max_depth + 1;
   s->d_asm_src.assign(D, nullptr);
   s->d_asm_dst.assign(D, nullptr);
@@ -1146,12 +1145,6 @@ int ensure_lanes(lfsolve *s) {
                                (int)sizeof(LeafSmem<cuComplex>)));
   LS_CUDA(cudaFuncSetAttribute(k_leaf<cuDoubleComplex>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)sizeof(LeafSmem<cuDoubleComplex>)));
-  LS_CUDA(cudaFuncSetAttribute(k_diag_inverse<cuComplex>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)inv_smem<cuComplex>()));
-  LS_CUDA(cudaFuncSetAttribute(k_diag_inverse<cuDoubleComplex>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)inv_smem<cuDoubleComplex>()));
   for (auto kern : {k_sweep_tri<1, 0, 0>, k_sweep_tri<1, 0, 1>, k_sweep_tri<1, 1, 0>,
                     k_sweep_tri<1, 1, 1>, k_sweep_tri<2, 0, 0>, k_sweep_tri<2, 0, 1>,
                     k_sweep_tri<2, 1, 0>, k_sweep_tri<2, 1, 1>})
@@ -1508,11 +1501,11 @@ int factor_impl(lfsolve *s, const double2 *vals) {
       LS_CUDA(cudaGetLastError());
     }
     if ((rc = lu_depth<T>(s, d, arena[d], lu_cap)) || (rc = lu_library<T>(s, d, arena[d], lu_cap))) return rc;
-    // the update blocks and the sweeps read the diagonal blocks as inverses
-    const int ni = s->inv_at[d + 1] - s->inv_at[d];
+    // the update blocks and the sweeps read U's diagonal blocks divided by their pivots
+    const int ni = s->diag_at[d + 1] - s->diag_at[d];
     if (ni > 0) {
-      k_diag_inverse<T><<<(ni + INV_WARPS - 1) / INV_WARPS, INV_WARPS * 32, inv_smem<T>(), st>>>(
-          ni, s->d_inv + s->inv_at[d], s->d_nodes, arena[d]);
+      k_diag_scale<T><<<(ni + DIAG_WARPS - 1) / DIAG_WARPS, DIAG_WARPS * 32, 0, st>>>(
+          ni, s->d_diag + s->diag_at[d], s->d_nodes, arena[d]);
       LS_CUDA(cudaGetLastError());
     }
     const DepthPlan &Q = plan[d];
@@ -2168,7 +2161,7 @@ void lfsolve_destroy(lfsolve *s) {
   free_factors(s);
   free_workspace(s);
   void *bufs[] = {s->d_nodes, s->d_child, s->d_perm, s->d_rorig, s->d_ess, s->d_tpos,
-                  s->d_info, s->d_V, s->d_Y, s->d_part_y, s->d_bw, s->d_src, s->d_inv, s->d_r, s->d_part, s->d_scale,
+                  s->d_info, s->d_V, s->d_Y, s->d_part_y, s->d_bw, s->d_src, s->d_diag, s->d_r, s->d_part, s->d_scale,
                   s->d_pperm};
   for (void *p : bufs)
     if (p) cudaFree(p);

@@ -5,12 +5,14 @@
 // substitution with L11 or U11 is a serial chain of k pivots.  Here it is cut
 // into steps of SB pivots: one block solves a step's SB x SB triangle
 // (diag_solve), then as many blocks as there are rows apply its columns.
-// Inside the triangle the chain is cut to SB / 32 links, because the 32 x 32
-// blocks on the diagonal of L11 and U11 are kept as their inverses
-// (k_diag_inverse, once per factorization, in place).  32 is as far as the
-// inverses go: with 32 x 32 blocks the residuals of complex128 solves are
-// those of plain substitution (1.5e-12 on a 111k-row contact hole, 1.6e-12
-// before), with 256 x 256 blocks they grow up to elevenfold.
+// Inside the triangle a warp substitutes through a link of 32 pivots by itself
+// (unit_solve), a lane a pivot, and hands the results to the others.  The rows
+// of U's 32 x 32 diagonal blocks are kept divided by their pivots, and the
+// pivots as their reciprocals (k_diag_scale, once per factorization, in place),
+// so that a link is a unit triangle in all four sweeps: no division and no
+// multiplication in its chain.  (Inverses of the blocks in their place were
+// faster, a product without a chain, but no longer backward stable: a block of
+// condition number c left residuals c times those of substitution.)
 //
 // Bound: every factor entry is read once a sweep pair from HBM; on the
 // smallest systems the launches.
@@ -203,14 +205,50 @@ __device__ __forceinline__ void each_col(T (&out)[SW_CHUNK / SW_W][NR], int c0, 
   }
 }
 
+// A unit triangle of 32 pivots across the warp, pivots h H .. h H + H - 1 of
+// them: a[i] = the lane's entry of pivot h H + i (zero but for the pivots before
+// the lane's in the order of substitution), v = the lane's entry, in place.  W
+// pivots a round: every lane takes their entries, works through their W x W
+// corner by itself and subtracts all W, so that a round waits for one shuffle.
+template <typename T> constexpr int UNIT_W = sizeof(T) == 8 ? 4 : 2;
+template <typename T, int NR, int BWD, int H>
+__device__ __forceinline__ void unit_solve(const T (&a)[H], int h, T (&v)[NR]) {
+  constexpr int W = UNIT_W<T>;
+  auto from = [](T x, int p) {
+    x.x = __shfl_sync(0xffffffffu, x.x, p);
+    x.y = __shfl_sync(0xffffffffu, x.y, p);
+    return x;
+  };
+#pragma unroll
+  for (int g = 0; g < H; g += W) {
+    T x[W][NR];
+    auto at = [&](int j) { return BWD ? H - 1 - g - j : g + j; };   // the round's pivot j
+#pragma unroll
+    for (int j = 0; j < W; ++j)
+#pragma unroll
+      for (int q = 0; q < NR; ++q) x[j][q] = from(v[q], h * H + at(j));
+#pragma unroll
+    for (int j = 1; j < W; ++j)
+#pragma unroll
+      for (int i = 0; i < j; ++i) {
+        const T c = from(a[at(i)], h * H + at(j));
+#pragma unroll
+        for (int q = 0; q < NR; ++q) x[j][q] = cfms(x[j][q], c, x[i][q]);
+      }
+#pragma unroll
+    for (int j = 0; j < W; ++j)
+#pragma unroll
+      for (int q = 0; q < NR; ++q) v[q] = cfms(v[q], a[at(j)], x[j][q]);
+  }
+}
+
 // The triangle of one step, v[q] = this thread's pivot of the step (thread t:
 // pivot t < nb), in place: forward with L (TRANS = 0) or U^T, backward with U
 // or L^T.  A thread keeps its own entry in a register and reads its row (for
 // the transposed triangles its column) of D a link of 32 entries at a time:
 // AHEAD a whole link before it is used (a block alone on its SM), else 16
 // entries at once (several blocks a SM, fewer registers).  The warp of a link
-// multiplies by the inverse through shuffles and hands its 32 results to the
-// others.
+// substitutes through it (unit_solve) and hands its 32 results to the others.
 template <typename T, int NR, int TRANS, int BWD, bool AHEAD>
 __device__ __forceinline__ void diag_solve(const T *__restrict__ D, int ld, int nb, T (&v)[NR],
                                            T *ys) {
@@ -218,15 +256,15 @@ __device__ __forceinline__ void diag_solve(const T *__restrict__ D, int ld, int 
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
   const int links = (nb + 31) / 32;
   T a[H], nx[AHEAD ? 32 : 1];
+  constexpr bool UNIT = TRANS == BWD;   // L; U's pivots come as reciprocals
+  const T rd = !UNIT && t < nb ? D[t + (long long)t * ld] : CT<T>::mk(1.0, 0.0);
   auto load = [&](int s, int l0, T *dst) {
-    // entries a link needs: its own warp's inverse, later warps' updates
+    // entries a link needs: its own warp's triangle, later warps' updates
     const bool need = t < nb && (BWD ? w <= s : w >= s);
 #pragma unroll
     for (int i = 0; i < H; ++i) {
       const int l = l0 + i, o = 32 * s + l;
-      const bool on = w != s ? true
-                     : TRANS ? (BWD ? l > lane : l <= lane)
-                             : (BWD ? l >= lane : l < lane);
+      const bool on = w != s || (BWD ? l > lane : l < lane);
       dst[i] = need && on && o < nb ? D[TRANS ? o + (long long)t * ld : t + (long long)o * ld]
                                     : czero<T>();
     }
@@ -239,30 +277,23 @@ __device__ __forceinline__ void diag_solve(const T *__restrict__ D, int ld, int 
       for (int l = 0; l < H; ++l) a[l] = nx[AHEAD ? l : 0];
       if (u + 1 < links) load(BWD ? s - 1 : s + 1, 0, nx);
     } else {
-      load(s, 0, a);
+      load(s, BWD && w == s ? 32 - H : 0, a);
     }
     T *y = ys + (u & 1) * 32 * NR;
     if (w == s) {
-      T o[NR];
+      if (!UNIT && BWD)
 #pragma unroll
-      for (int q = 0; q < NR; ++q) o[q] = (TRANS == BWD) ? v[q] : czero<T>();  // unit diagonal of L
+        for (int q = 0; q < NR; ++q) v[q] = cmul(v[q], rd);
 #pragma unroll
-      for (int h = 0; h < 32 / H; ++h) {
-        if (h > 0) load(s, h * H, a);
-#pragma unroll
-        for (int i = 0; i < H; ++i)
-#pragma unroll
-          for (int q = 0; q < NR; ++q) {
-            T b;
-            b.x = __shfl_sync(0xffffffffu, v[q].x, h * H + i);
-            b.y = __shfl_sync(0xffffffffu, v[q].y, h * H + i);
-            cfma(o[q], a[i], b);
-          }
+      for (int i = 0; i < 32 / H; ++i) {
+        const int h = BWD ? 32 / H - 1 - i : i;
+        if (i > 0) load(s, h * H, a);
+        unit_solve<T, NR, BWD, H>(a, h, v);
       }
 #pragma unroll
       for (int q = 0; q < NR; ++q) {
-        v[q] = o[q];
-        y[lane * NR + q] = o[q];
+        if (!UNIT && !BWD) v[q] = cmul(v[q], rd);
+        y[lane * NR + q] = v[q];
       }
     }
     __syncthreads();
@@ -582,15 +613,15 @@ __global__ void __launch_bounds__(SW_T) k_sweep(const Sweep<T> S, int j0) {
 // waited for, and what is left is arithmetic and the vectors' latency.
 //
 // k_sweep_tri: a step's triangle, a block a front.  The 28 off-diagonal 32 x 32
-// blocks in shared memory (224 kB of the 227 an SM has), every warp's inverse
-// in its registers.  Warp s multiplies by its inverse, and hands its 32 results
-// to the warps after it over a barrier of its own, so that no warp waits for
-// one that is behind it.  The results lie where the warp's last used block was.
+// blocks in shared memory (224 kB of the 227 an SM has), every warp's own
+// triangle in its registers.  Warp s substitutes through it, and hands its 32
+// results to the warps after it over a barrier of its own, so that no warp waits
+// for one that is behind it.  The results lie where the warp's last used block was.
 // Forward sweep of a 271k-row line grating's root front (six steps, triangle and
 // columns): 114 us with the links loaded a link ahead and a block-wide barrier
 // each, 53 us so.
 constexpr int TRI_TILE = 32 * 32;
-constexpr size_t TRI_SMEM = (size_t)(28 * TRI_TILE + 128) * sizeof(cuComplex);
+constexpr size_t TRI_SMEM = (size_t)(28 * TRI_TILE + 64) * sizeof(cuComplex);
 __device__ __forceinline__ int tri_tile(int a, int b) {
   const int hi = max(a, b), lo = min(a, b);
   return (hi * (hi - 1) / 2 + lo) * TRI_TILE;
@@ -610,7 +641,8 @@ __global__ void __launch_bounds__(SW_T, 1) k_sweep_tri(const Sweep<cuComplex> S,
   const int nb = min(SB, k - j0), links = (nb + 31) / 32;
   const bool on = nb > 0;
   const T *D = S.fac + N.fac_off + j0 + (long long)j0 * m;
-  T own[32];
+  constexpr bool UNIT = TRANS == BWD;   // L; U's pivots come as reciprocals
+  T own[32], rd = CT<T>::mk(1.0, 0.0);
   if (on) {
     // block (w2, s2): rows (TRANS: columns) of warp w2 against link s2, four of
     // its lines a warp; lanes along the contiguous rows of D, so that transposed
@@ -633,9 +665,10 @@ __global__ void __launch_bounds__(SW_T, 1) k_sweep_tri(const Sweep<cuComplex> S,
 #pragma unroll
     for (int l = 0; l < 32; ++l) {
       const int o = 32 * w + l;
-      const bool in = TRANS ? (BWD ? l > lane : l <= lane) : (BWD ? l >= lane : l < lane);
+      const bool in = BWD ? l > lane : l < lane;
       own[l] = in && t < nb && o < nb ? D[TRANS ? o + (long long)t * m : t + (long long)o * m] : czero<T>();
     }
+    if (!UNIT && t < nb) rd = D[t + (long long)t * m];
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
   }
@@ -647,7 +680,7 @@ __global__ void __launch_bounds__(SW_T, 1) k_sweep_tri(const Sweep<cuComplex> S,
     v[q] = t >= nb ? czero<T>()
            : BWD   ? S.Y[N.p0 + j0 + t + (long long)q * S.nn]
                    : S.V[N.vec_off + j0 + t + q * S.VR];
-  // the results of link s: 32 NR entries after as many of the warp's input
+  // the results of link s: 32 NR entries
   auto slot = [&](int s) {
     const int first = BWD ? links - 1 : 0;
     return s == first ? tiles + 28 * TRI_TILE : tiles + tri_tile(s, BWD ? s + 1 : s - 1);
@@ -656,7 +689,7 @@ __global__ void __launch_bounds__(SW_T, 1) k_sweep_tri(const Sweep<cuComplex> S,
   for (int u = 0; u < before; ++u) {
     const int s = BWD ? links - 1 - u : u;
     asm volatile("bar.sync %0, %1;" ::"r"(1 + s), "r"(32 * (links - u)) : "memory");
-    const T *y = slot(s) + 32 * NR, *c = tiles + tri_tile(w, s);
+    const T *y = slot(s), *c = tiles + tri_tile(w, s);
     T o[NR];
 #pragma unroll
     for (int q = 0; q < NR; ++q) o[q] = czero<T>();
@@ -670,22 +703,16 @@ __global__ void __launch_bounds__(SW_T, 1) k_sweep_tri(const Sweep<cuComplex> S,
     for (int q = 0; q < NR; ++q) v[q] = csub(v[q], o[q]);
   }
   {
-    T *in = slot(w), *y = in + 32 * NR;
-    __syncwarp();
+    T *y = slot(w);
+    if (!UNIT && BWD)
 #pragma unroll
-    for (int q = 0; q < NR; ++q) in[lane * NR + q] = v[q];
-    __syncwarp();
-    T o[NR];
-#pragma unroll
-    for (int q = 0; q < NR; ++q) o[q] = (TRANS == BWD) ? v[q] : czero<T>();  // unit diagonal of L
-#pragma unroll
-    for (int l = 0; l < 32; ++l)
-#pragma unroll
-      for (int q = 0; q < NR; ++q) cfma(o[q], own[l], in[l * NR + q]);
+      for (int q = 0; q < NR; ++q) v[q] = cmul(v[q], rd);
+    unit_solve<T, NR, BWD, 32>(own, 0, v);
+    __syncwarp();   // every lane has read the slot as a block
 #pragma unroll
     for (int q = 0; q < NR; ++q) {
-      v[q] = o[q];
-      y[lane * NR + q] = o[q];
+      if (!UNIT && !BWD) v[q] = cmul(v[q], rd);
+      y[lane * NR + q] = v[q];
     }
     if (before + 1 < links)
       asm volatile("bar.arrive %0, %1;" ::"r"(1 + w), "r"(32 * (links - before)) : "memory");
@@ -785,55 +812,26 @@ __global__ void __launch_bounds__(SW_T) k_sweep_apply(const Sweep<cuComplex> S, 
   }
 }
 
-// Inverses of the 32 x 32 blocks on the diagonals of L11 and U11 of a depth's
-// fronts, in place: a warp per (front, block), by substitution, a lane per
-// column of the inverse in registers, the block in shared memory.
-constexpr int INV_WARPS = 4;
-struct InvItem { int node, j0; };
+// The 32 x 32 blocks on the diagonals of U11 of a depth's fronts, in place: rows
+// divided by their pivots, the pivots as reciprocals; a warp per (front, block),
+// a lane a row.
+constexpr int DIAG_WARPS = 4;
+struct DiagItem { int node, j0; };
 template <typename T>
-__global__ void __launch_bounds__(INV_WARPS * 32)
-k_diag_inverse(int cnt, const InvItem *__restrict__ items, const NodeDev *__restrict__ nodes,
-               T *arena) {
-  extern __shared__ __align__(16) unsigned char inv_raw[];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int i0 = blockIdx.x * INV_WARPS + w;
+__global__ void __launch_bounds__(DIAG_WARPS * 32)
+k_diag_scale(int cnt, const DiagItem *__restrict__ items, const NodeDev *__restrict__ nodes,
+             T *arena) {
+  const int lane = threadIdx.x & 31, i0 = blockIdx.x * DIAG_WARPS + (threadIdx.x >> 5);
   if (i0 >= cnt) return;
-  T(*B)[33] = reinterpret_cast<T(*)[33]>(inv_raw) + 32 * w;
-  const InvItem it = items[i0];
+  const DiagItem it = items[i0];
   const NodeDev N = nodes[it.node];
-  const int ld = N.ld, n = min(32, N.k - it.j0);
-  T *D = arena + N.arena_off + it.j0 + (long long)it.j0 * ld;
-  for (int c = 0; c < 32; ++c)  // identity past the block
-    B[lane][c] = lane < n && c < n ? D[lane + (long long)c * ld]
-                                   : CT<T>::mk(lane == c ? 1.0 : 0.0, 0.0);
-  __syncwarp();
-  T x[32];
-  // column `lane` of L^-1
-#pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    T s = CT<T>::mk(i == lane ? 1.0 : 0.0, 0.0);
-#pragma unroll
-    for (int l = 0; l < i; ++l) s = cfms(s, B[i][l], x[l]);
-    x[i] = s;
+  const int n = min(32, N.k - it.j0);
+  if (lane >= n) return;
+  T *D = arena + N.arena_off + it.j0 + (long long)it.j0 * N.ld + lane;
+  const T rd = cdiv(CT<T>::mk(1.0, 0.0), D[(long long)lane * N.ld]);
+#pragma unroll 8
+  for (int c = 0; c < n; ++c) {
+    T &d = D[(long long)c * N.ld];
+    if (c >= lane) d = c == lane ? rd : cmul(d, rd);
   }
-  __syncwarp();
-#pragma unroll
-  for (int i = 0; i < 32; ++i)
-    if (i > lane && i < n) D[i + (long long)lane * ld] = x[i];
-  // column `lane` of U^-1 (the diagonal's reciprocals are shared first)
-  const T rd = cdiv(CT<T>::mk(1.0, 0.0), B[lane][lane]);
-  __syncwarp();
-  B[lane][lane] = rd;
-  __syncwarp();
-#pragma unroll
-  for (int i = 31; i >= 0; --i) {
-    T s = CT<T>::mk(i == lane ? 1.0 : 0.0, 0.0);
-#pragma unroll
-    for (int l = i + 1; l < 32; ++l) s = cfms(s, B[i][l], x[l]);
-    x[i] = cmul(s, B[i][i]);
-  }
-#pragma unroll
-  for (int i = 0; i < 32; ++i)
-    if (i <= lane && lane < n) D[i + (long long)lane * ld] = x[i];
 }
-template <typename T> constexpr size_t inv_smem() { return (size_t)INV_WARPS * 32 * 33 * sizeof(T); }

@@ -2,9 +2,10 @@
 // namespace after lfsolve_sweeps.cuh: U12 = L11^-1 P F12 and L21 = F21 U11^-1
 // of a group of fronts of the same (padded) shape.
 //
-// The pivots are taken in leaves of 64.  A leaf's triangle is applied here
-// (its 32 x 32 diagonal blocks are inverses already, so a leaf is three small
-// products), and what a solved range of leaves contributes to the next one is
+// The pivots are taken in leaves of 64.  A leaf's triangle is applied here by
+// substitution, eight pivots at a time (leaf_triangle; U's 32 x 32 diagonal
+// blocks come as unit triangles and reciprocal pivots, k_diag_scale), and what a
+// solved range of leaves contributes to the next one is
 // a matrix product, binary: after leaf i, with 2^t the power of two in i, the
 // last 2^t leaves update the next 2^t.  So all but k x 64 of the work is in
 // products at least 64 deep, half of it in products of half the pivots.
@@ -106,15 +107,14 @@ __global__ void __launch_bounds__(SPLIT_T) k_split_f11(const Group<T> G) {
 }
 
 template <typename T> struct LeafSmem {
-  T D[LEAF][LEAF + 1];          // the leaf's triangle: inverses on the diagonal, zero beyond
+  T D[LEAF][LEAF + 1];          // the leaf's triangle, zero beyond
   T X[LEAF][LEAF_C<T> + 1];     // pivots x columns (left) or pivots x rows (right)
 };
 
-// X[o0 .. o0 + 32) (-)= sum over l in [l0, l0 + 32) of coef(o, l) X[l], a
-// thread per 4 pivots x LEAF_C / 16 columns; SUB: the sum (formed by itself)
-// taken from X, else a triangle, whose zero 8 x 8 blocks are left out
-template <typename T, bool SUB, class C>
-__device__ __forceinline__ void leaf_product(LeafSmem<T> &sm, int o0, int l0, C coef) {
+// rows [o0 + 8 q0, o0 + 32) of X -= sum over l in [l0, l0 + n) of coef(o, l) X[l],
+// the sums formed by themselves, a thread per 4 pivots x LEAF_C / 16 columns
+template <typename T, class C>
+__device__ __forceinline__ void leaf_update(LeafSmem<T> &sm, int o0, int q0, int l0, int n, C coef) {
   constexpr int NB = LEAF_C<T> / 16;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   T acc[4][NB];
@@ -122,31 +122,57 @@ __device__ __forceinline__ void leaf_product(LeafSmem<T> &sm, int o0, int l0, C 
   for (int a = 0; a < 4; ++a)
 #pragma unroll
     for (int b = 0; b < NB; ++b) acc[a][b] = czero<T>();
-#pragma unroll
-  for (int q = 0; q < 4; ++q)
 #pragma unroll 2
-    for (int l = 8 * q; l < 8 * q + 8; ++l) {
-      T d[4], x[NB];
+  for (int l = l0; l < l0 + n; ++l) {
+    T d[4], x[NB];
 #pragma unroll
-      for (int a = SUB ? 0 : q; a < 4; ++a) d[a] = coef(o0 + ty + 8 * a, l0 + l);
+    for (int a = q0; a < 4; ++a) d[a] = coef(o0 + ty + 8 * a, l);
 #pragma unroll
-      for (int b = 0; b < NB; ++b) x[b] = sm.X[l0 + l][tx + 16 * b];
+    for (int b = 0; b < NB; ++b) x[b] = sm.X[l][tx + 16 * b];
 #pragma unroll
-      for (int a = SUB ? 0 : q; a < 4; ++a)
+    for (int a = q0; a < 4; ++a)
 #pragma unroll
-        for (int b = 0; b < NB; ++b)
-          if (SUB) acc[a][b] = cfms(acc[a][b], d[a], x[b]);
-          else cfma(acc[a][b], d[a], x[b]);
-    }
-  __syncthreads();
+      for (int b = 0; b < NB; ++b) acc[a][b] = cfms(acc[a][b], d[a], x[b]);
+  }
 #pragma unroll
-  for (int a = 0; a < 4; ++a)
+  for (int a = q0; a < 4; ++a)
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
       T &x = sm.X[o0 + ty + 8 * a][tx + 16 * b];
-      x = SUB ? cadd(x, acc[a][b]) : acc[a][b];
+      x = cadd(x, acc[a][b]);
     }
   __syncthreads();
+}
+
+// A unit triangle of 32 pivots from o0 on: eight pivots of a column by a thread,
+// then their part of the rows left.  SCALE: the results times the reciprocal
+// pivots at the end, eight rows at a time by the threads without a column.
+template <typename T, bool SCALE, class C>
+__device__ __forceinline__ void leaf_triangle(LeafSmem<T> &sm, int o0, C coef) {
+  constexpr int NC = LEAF_C<T>;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int l0 = o0 + 8 * q;
+    if (threadIdx.x < NC) {
+      T x[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) x[i] = sm.X[l0 + i][threadIdx.x];
+#pragma unroll
+      for (int i = 0; i < 7; ++i)
+#pragma unroll
+        for (int j = i + 1; j < 8; ++j) x[j] = cfms(x[j], coef(l0 + j, l0 + i), x[i]);
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        sm.X[l0 + i][threadIdx.x] = SCALE && q == 3 ? cmul(x[i], sm.D[l0 + i][l0 + i]) : x[i];
+    } else if (SCALE && q > 0) {
+      for (int t = threadIdx.x - NC; t < 8 * NC; t += LEAF_T - NC) {
+        const int l = l0 - 8 + t / NC;
+        sm.X[l][t % NC] = cmul(sm.X[l][t % NC], sm.D[l][l]);
+      }
+    }
+    __syncthreads();
+    if (q < 3) leaf_update<T>(sm, o0, q + 1, l0, 8, coef);
+  }
 }
 
 template <typename T, bool LEFT>
@@ -167,7 +193,7 @@ __device__ __forceinline__ void leaf_side(const Group<T> &G, int p0, LeafSmem<T>
 #pragma unroll
     for (int u = 0; u < B; ++u) {
       const int t = t0 + u * LEAF_T, i = t % LEAF, l = t / LEAF;
-      sm.D[i][l] = LEFT && i == l ? CT<T>::mk(1.0, 0.0) : v[u];
+      sm.D[i][l] = v[u];
     }
   }
   constexpr int XI = LEFT ? LEAF : NC;   // entries along a column of memory
@@ -189,10 +215,10 @@ __device__ __forceinline__ void leaf_side(const Group<T> &G, int p0, LeafSmem<T>
   // X = L^-1 X by halves: X_0 = L_00^-1 X_0; X_1 = L_11^-1 (X_1 - L_10 X_0);
   // for F21 the same with the transposed coefficients of U
   auto coef = [&](int o, int l) { return LEFT ? sm.D[o][l] : sm.D[l][o]; };
-  leaf_product<T, false>(sm, 0, 0, coef);
-  if (kb > 32) {
-    leaf_product<T, true>(sm, 32, 0, coef);
-    leaf_product<T, false>(sm, 32, 32, coef);
+#pragma unroll 1
+  for (int o0 = 0; o0 < kb; o0 += 32) {
+    if (o0) leaf_update<T>(sm, 32, 0, 0, 32, coef);
+    leaf_triangle<T, !LEFT>(sm, o0, coef);
   }
 #pragma unroll 4
   for (int t = threadIdx.x; t < LEAF * NC; t += LEAF_T) {
@@ -214,9 +240,9 @@ __device__ __forceinline__ void leaf_side(const Group<T> &G, int p0, LeafSmem<T>
 // One leaf (pivots p0 .. p0 + kb) of every front of the group: F12
 // (blockIdx.z = 0) and F21 in one launch, LEAF_C columns (rows) a block.
 // Bound: FP32 (FP64) FMA issue and the stores of the split operands, about
-// equal.  Kernel time over a factorization with a launch a side, 2 pivots a
-// thread and whole 32 x 32 triangles, and so: 113 and 69 ms (complex64,
-// 524k-row line grating), 12.7 and 6.9 ms (complex128, 111k-row hole).
+// equal.  The substitution takes what products with the inverses of the 32 x 32
+// blocks took (a factorization 235.3 and 234.6 ms in complex64 on a 524k-row line
+// grating, 52.1 and 51.6 ms in complex128 on a 111k-row hole).
 template <typename T>
 __global__ void __launch_bounds__(LEAF_T, sizeof(T) == 8 ? 3 : 2) k_leaf(const Group<T> G, int p0) {
   extern __shared__ __align__(16) unsigned char leaf_raw[];
