@@ -109,13 +109,21 @@ constexpr double LU_AHEAD_MIN = 1e6;
 // complex64 fronts whose Schur update F22 -= L21 U12 has at least this many
 // complex multiply-adds use three TF32 tensor-core GEMMs on split operands
 constexpr double TF32X3_MIN_MACS = 2e9;
-// pivots one product of the large TF32 terms accumulates: the tensor cores
-// truncate as they add, so that deeper products lose accuracy (residual after
-// two corrections on a 271k-row line grating: 8.6e-10 with all pivots at once,
-// 3.0e-10 with 512, 1.0e-10 with 256, 5.6e-11 with 128; 1.3e-9 before the
-// update blocks ran in this form), and each piece reads and writes the result
-// once more (its factorization: 99.8, 100.7, 103.1, 109.6 ms)
-constexpr int TF32_PIVOTS = 512;
+// Pivots one product of the large TF32 terms runs through.  The tensor cores cut
+// every partial sum off towards zero, so that the error grows with the depth, and
+// every further piece reads and writes the result once more.  Unrefined errors
+// (solution, transposed solution, their residuals; 271k-row line grating) over
+// those of FP32 substitution with F22's product in split form and one piece, and
+// the time of a factorization (524k-row one):
+//   512 everywhere       1.19  1.38  0.73  2.50    235 ms
+//   256 everywhere       0.91  1.09  0.67  2.67    246 ms
+//   128 everywhere       0.63  0.74  0.60  2.00    276 ms
+//   256 large, 64 else   0.43  0.68  0.59  1.03    262 ms
+//   64 everywhere        0.42  0.68  0.57  0.94    341 ms
+//   FP32 products        0.34  0.61  0.59  1.35    413 ms
+// Large are the fronts that are split by themselves (TF32X3_MIN_MACS); the others,
+// many to a group, lose most where their pivots go in one piece.
+constexpr int TF32_PIVOTS = 64, TF32_PIVOTS_LARGE = 256;
 // memory the split operands of fronts in flight may take
 constexpr size_t SPLIT_BYTES = (size_t)6 << 30;
 
@@ -1217,8 +1225,9 @@ int group_product(cublasHandle_t h, const Group<T> &G, int m, int n, int p0, int
           CUDA_R_32F, 2 * G.ld, 2 * G.S, G.cnt, CUBLAS_COMPUTE_32F_FAST_TF32, CUBLAS_GEMM_DEFAULT);
     };
     LS_BLAS(product(4, As.both(0), Bs.both(0), p0, k));
-    for (int q0 = p0; q0 < p0 + k; q0 += TF32_PIVOTS)
-      LS_BLAS(product(2, As.hi(G.cnt, 0), Bs.hi(G.cnt, 0), q0, std::min(TF32_PIVOTS, p0 + k - q0)));
+    const int piece = (double)G.r * G.r * G.kk >= TF32X3_MIN_MACS ? TF32_PIVOTS_LARGE : TF32_PIVOTS;
+    for (int q0 = p0; q0 < p0 + k; q0 += piece)
+      LS_BLAS(product(2, As.hi(G.cnt, 0), Bs.hi(G.cnt, 0), q0, std::min(piece, p0 + k - q0)));
     return LFSOLVE_OK;
   }
   const T mone = CT<T>::mk(-1.0, 0.0), one = CT<T>::mk(1.0, 0.0);
