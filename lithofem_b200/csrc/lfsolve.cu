@@ -1005,7 +1005,7 @@ struct lfsolve {
   double2 *d_r = nullptr, *d_x64 = nullptr;
   size_t r_bytes = 0;
   double *d_part = nullptr, *d_scale = nullptr;
-  size_t part_bytes = 0;
+  size_t part_bytes = 0, scale_bytes = 0;
   cudaEvent_t t0 = nullptr, t1 = nullptr;
 };
 
@@ -1028,8 +1028,36 @@ int upload(T **dst, const std::vector<T> &v, cudaStream_t st) {
   return LFSOLVE_OK;
 }
 
+template <typename T> void drop(T *&p) {
+  if (p) cudaFree(p);
+  p = nullptr;
+}
+
+void free_factors(lfsolve *s) {
+  drop(s->d_fac);
+  s->prec = -1;
+}
+
+// the factors, and everything on the device that was sized for a plan
+void free_plan(lfsolve *s) {
+  free_factors(s);
+  s->uploaded = false;
+  drop(s->d_nodes);
+  for (int **p : {&s->d_child, &s->d_perm, &s->d_rorig, &s->d_ess, &s->d_tpos, &s->d_src, &s->d_info,
+                  &s->d_pperm})
+    drop(*p);
+  drop(s->d_diag);
+  drop(s->d_swaps);
+  for (auto &p : s->d_asm_src) drop(p);
+  for (auto &p : s->d_asm_dst) drop(p);
+  for (auto &p : s->d_bf) drop(p);
+  for (auto &p : s->d_co) drop(p);
+  for (auto &p : s->d_all) drop(p);
+}
+
 int ensure_uploaded(lfsolve *s) {
   if (s->uploaded) return LFSOLVE_OK;
+  free_plan(s);   // what an upload that failed midway left
   Plan &P = s->P;
   const int ns = (int)P.nodes.size();
   std::vector<NodeDev> nd(ns);
@@ -1720,24 +1748,13 @@ int solve_pass(lfsolve *s, int nr, const T *b, T *x, int trans) {
 int ensure_solve_scratch(lfsolve *s, size_t es) {
   Plan &P = s->P;
   const size_t V = (size_t)P.vec_rows * MAX_NRHS_PASS * es;
-  if (s->V_bytes < V) {
-    if (s->d_V) LS_CUDA(cudaFree(s->d_V));
-    LS_CUDA(cudaMalloc(&s->d_V, V));
-    s->V_bytes = V;
-  }
   const size_t Y = (size_t)std::max(1, P.nn) * MAX_NRHS_PASS * es;
-  if (s->Y_bytes < Y) {
-    if (s->d_Y) LS_CUDA(cudaFree(s->d_Y));
-    LS_CUDA(cudaMalloc(&s->d_Y, Y));
-    s->Y_bytes = Y;
-  }
-  if (int rc = ensure_bytes(&s->d_part_y, &s->part_y_bytes, Y * SW_PARTS)) return rc;
   const size_t bw = (size_t)P.n * 2 * MAX_NRHS_PASS * es;  // b and x in the factor precision
-  if (s->bw_bytes < bw) {
-    if (s->d_bw) LS_CUDA(cudaFree(s->d_bw));
-    LS_CUDA(cudaMalloc(&s->d_bw, bw));
-    s->bw_bytes = bw;
-  }
+  int rc;
+  if ((rc = ensure_bytes(&s->d_V, &s->V_bytes, V)) || (rc = ensure_bytes(&s->d_Y, &s->Y_bytes, Y)) ||
+      (rc = ensure_bytes(&s->d_part_y, &s->part_y_bytes, Y * SW_PARTS)) ||
+      (rc = ensure_bytes(&s->d_bw, &s->bw_bytes, bw)))
+    return rc;
   return LFSOLVE_OK;
 }
 
@@ -1915,12 +1932,6 @@ void free_workspace(lfsolve *s) {
   s->split_bytes = 0;
 }
 
-void free_factors(lfsolve *s) {
-  if (s->d_fac) cudaFree(s->d_fac);
-  s->d_fac = nullptr;
-  s->prec = -1;
-}
-
 }  // namespace
 
 extern "C" {
@@ -1956,11 +1967,15 @@ int lfsolve_analyze(lfsolve *s, int n, const int *I, const int *J, long long nnz
   if (I[0] != 0 || I[n] != nnz) return fail(LFSOLVE_ERR_ARG, "row pointer does not span nnz");
   const auto t0 = std::chrono::steady_clock::now();
   const int leaf = leaf_elements > 0 ? leaf_elements : 32;
+  // the device tables, the factors and the buffers sized by the plan go with it
+  if (s->blas_main) {
+    LS_CUDA(cudaSetDevice(s->dev));
+    free_plan(s);
+  }
   const int rc = build_plan(n, I, J, nnz, ne, nd, elem_dof, centroid, ess, n_ess, leaf, s->P);
   if (rc) return rc;
   const auto t1 = std::chrono::steady_clock::now();
   s->analyzed = true;
-  s->uploaded = false;
   lfsolve_stats &st = s->st;
   st = lfsolve_stats{};
   st.n = n;
@@ -2062,21 +2077,14 @@ int lfsolve_solve_refined(lfsolve *s, const int *d_I, const int *d_J, const void
   const int n = s->P.n;
   cudaStream_t st = s->stream;
   const size_t rb = (size_t)n * nrhs * sizeof(double2);
-  if (s->r_bytes < rb) {
-    if (s->d_r) LS_CUDA(cudaFree(s->d_r));
-    LS_CUDA(cudaMalloc((void **)&s->d_r, rb));
-    s->r_bytes = rb;
-  }
+  int rc;
+  if ((rc = ensure_bytes((void **)&s->d_r, &s->r_bytes, rb))) return rc;
   const int wpb = 8;
   const int nblk = (n + wpb - 1) / wpb;
   const size_t pb = (size_t)3 * nblk * nrhs * sizeof(double) + (size_t)3 * nrhs * sizeof(double);
-  if (s->part_bytes < pb) {
-    if (s->d_part) LS_CUDA(cudaFree(s->d_part));
-    LS_CUDA(cudaMalloc((void **)&s->d_part, pb));
-    s->part_bytes = pb;
-    if (s->d_scale) LS_CUDA(cudaFree(s->d_scale));
-    LS_CUDA(cudaMalloc((void **)&s->d_scale, sizeof(double) * 2 * nrhs));
-  }
+  if ((rc = ensure_bytes((void **)&s->d_part, &s->part_bytes, pb)) ||
+      (rc = ensure_bytes((void **)&s->d_scale, &s->scale_bytes, sizeof(double) * 2 * nrhs)))
+    return rc;
   double *sums = s->d_part + (size_t)3 * nblk * nrhs;
   const double2 *b = static_cast<const double2 *>(d_b);
   double2 *x = static_cast<double2 *>(d_x);
@@ -2104,8 +2112,7 @@ int lfsolve_solve_refined(lfsolve *s, const int *d_I, const int *d_J, const void
     return LFSOLVE_OK;
   };
   LS_CUDA(cudaEventRecord(s->t0, st));
-  int rc = solve_dispatch(s, nrhs, b, x, transpose != 0, nullptr, 0);
-  if (rc) return rc;
+  if ((rc = solve_dispatch(s, nrhs, b, x, transpose != 0, nullptr, 0))) return rc;
   double worst = 0.0;
   int it = 0, steps = 0;
   if ((rc = residual(&worst))) return rc;
@@ -2165,19 +2172,11 @@ void lfsolve_destroy(lfsolve *s) {
   if (!s) return;
   cudaSetDevice(s->dev);
   if (s->stream) cudaStreamSynchronize(s->stream);
-  free_factors(s);
+  free_plan(s);
   free_workspace(s);
-  void *bufs[] = {s->d_nodes, s->d_child, s->d_perm, s->d_rorig, s->d_ess, s->d_tpos,
-                  s->d_info, s->d_V, s->d_Y, s->d_part_y, s->d_bw, s->d_src, s->d_diag, s->d_r, s->d_part, s->d_scale,
-                  s->d_pperm};
+  void *bufs[] = {s->d_V, s->d_Y, s->d_part_y, s->d_bw, s->d_r, s->d_part, s->d_scale};
   for (void *p : bufs)
     if (p) cudaFree(p);
-  for (auto *p : s->d_asm_src) if (p) cudaFree(p);
-  for (auto *p : s->d_asm_dst) if (p) cudaFree(p);
-  for (auto *p : s->d_bf) if (p) cudaFree(p);
-  for (auto *p : s->d_co) if (p) cudaFree(p);
-  if (s->d_swaps) cudaFree(s->d_swaps);
-  for (auto *p : s->d_all) if (p) cudaFree(p);
   for (int l = 0; l < LANES; ++l) {
     if (s->work[l]) cudaFree(s->work[l]);
     if (s->lpiv[l]) cudaFree(s->lpiv[l]);
