@@ -1972,6 +1972,7 @@ int lfsolve_analyze(lfsolve *s, int n, const int *I, const int *J, long long nnz
     LS_CUDA(cudaSetDevice(s->dev));
     free_plan(s);
   }
+  s->analyzed = false;   // until the plan stands
   const int rc = build_plan(n, I, J, nnz, ne, nd, elem_dof, centroid, ess, n_ess, leaf, s->P);
   if (rc) return rc;
   const auto t1 = std::chrono::steady_clock::now();
