@@ -52,7 +52,7 @@ typedef struct lfsolve_stats {
   int n, n_ess, n_fronts, depth, max_front, max_pivots;
   long long factor_entries;   /* stored L and U entries                    */
   double factor_flops;        /* real flops of the numeric factorization   */
-  long long peak_front_entries; /* front workspace of the two busiest depths */
+  long long peak_front_entries; /* front workspace held: largest even + largest odd depth */
   double analyze_s;           /* host seconds of lfsolve_analyze           */
   float factor_ms;            /* device ms of the last lfsolve_factor      */
   float solve_ms;             /* device ms of the last triangular solve    */

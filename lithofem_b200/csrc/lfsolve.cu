@@ -486,9 +486,10 @@ int build_plan(int n, const int *I, const int *J, long long nnz, int ne, int nd,
   P.factor_entries = fac;
   P.vec_rows = vec;
   if (vec >= (1LL << 31)) return fail(LFSOLVE_ERR_ARG, "the fronts' rows exceed 2^31");
-  for (int d = 0; d <= P.max_depth; ++d)
-    P.peak_front_entries = std::max(P.peak_front_entries,
-                                    P.arena_size[d] + (d < P.max_depth ? P.arena_size[d + 1] : 0));
+  // the workspace a factorization holds: the largest even and the largest odd depth
+  long long half[2] = {0, 0};
+  for (int d = 0; d <= P.max_depth; ++d) half[d & 1] = std::max(half[d & 1], P.arena_size[d]);
+  P.peak_front_entries = half[0] + half[1];
   P.r_orig.resize(roff);
   for (int s = 0; s < ns; ++s) {
     const Node &N = P.nodes[s];

@@ -44,3 +44,23 @@ def test_a_refused_argument_keeps_the_analysis():
     assert not s.Analyze(c.ad, short, J) and s.last_error[0] == ERR_ARG
     assert solver.lib().lfsolve_get_fronts(s._s, None, None, None, None) == 0
     s.Release()
+
+
+def test_workspace_figure_is_what_the_factorization_takes(monkeypatch):
+    """peak_front_entries: the largest even and the largest odd depth, which
+    are held together but need not be neighbours (a front a group, so that the
+    padded layout follows from pivots and rows: both parts to 16, fronts to 32
+    entries)."""
+    monkeypatch.setenv("LFSOLVE_BATCH_MIN", "1000000")
+    c = configs.small_case("grating", 3, 6.0, seed=5)
+    I, J = oracle.csr(c.ad)
+    s = solver.DirectSolver(0)
+    assert s.Analyze(c.ad, I, J), s.last_error
+    f = s.Fronts()
+    pad = lambda v, a: (v.astype(np.int64) + a - 1) // a * a
+    entries = pad((pad(f["k"], 16) + pad(f["m"] - f["k"], 16)) ** 2, 32)
+    depth = np.bincount(f["depth"], weights=entries).astype(np.int64)
+    held = depth[::2].max() + depth[1::2].max()
+    assert held > (depth[1:] + depth[:-1]).max()      # not neighbours here
+    assert s.Stats()["peak_front_entries"] == held
+    s.Release()
