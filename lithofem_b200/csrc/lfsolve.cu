@@ -1622,29 +1622,22 @@ int sweep_launch(void (*kern)(Sweep<T>, int), const Sweep<T> &S, dim3 grid, size
 // 32 fronts 0.47 and 0.48, 64 fronts 0.45 and 0.42, 256 fronts 0.31 and 0.27).
 constexpr int HELD_FRONTS = 32;
 
-// one launch of a phase over the fronts of a depth, at most nch chunks each in
-// nz parts
+// one launch of a phase over the fronts of a depth (fewer than 1,024,
+// front_per_block), at most nch chunks each in nz parts
 template <typename T, int NR, int TRANS, int PH>
 int sweep_phase(const Sweep<T> &S, int nch, int fronts, int j0, cudaStream_t st, int nz = 1) {
   if (nch <= 0) return LFSOLVE_OK;
   constexpr bool FWD = PH == PH_FWD_A || PH == PH_FWD_B;
-  // grid.y holds 65,535 fronts
-  for (int f0 = 0; f0 < fronts; f0 += 65535) {
-    Sweep<T> P = S;
-    P.list = S.list + f0;
-    const unsigned nf = (unsigned)std::min(65535, fronts - f0);
-    const dim3 grid((unsigned)nch, nf, (unsigned)nz);
-    void (*kern)(Sweep<T>, int) = k_sweep<T, NR, TRANS, PH>;
-    size_t smem = 0;
-    if constexpr (sizeof(T) == 8) {
-      if constexpr (PH == PH_FWD_A || PH == PH_BWD_A)
-        if (fronts <= HELD_FRONTS) kern = k_sweep_tri<NR, TRANS, !FWD>, smem = TRI_SMEM;
-      if constexpr (PH == PH_FWD_B || PH == PH_BWD_B)
-        if (fronts <= HELD_FRONTS) kern = k_sweep_apply<NR, TRANS, !FWD>;
-    }
-    if (int rc = sweep_launch<T>(kern, P, grid, smem, j0, st)) return rc;
+  const dim3 grid((unsigned)nch, (unsigned)fronts, (unsigned)nz);
+  void (*kern)(Sweep<T>, int) = k_sweep<T, NR, TRANS, PH>;
+  size_t smem = 0;
+  if constexpr (sizeof(T) == 8) {
+    if constexpr (PH == PH_FWD_A || PH == PH_BWD_A)
+      if (fronts <= HELD_FRONTS) kern = k_sweep_tri<NR, TRANS, !FWD>, smem = TRI_SMEM;
+    if constexpr (PH == PH_FWD_B || PH == PH_BWD_B)
+      if (fronts <= HELD_FRONTS) kern = k_sweep_apply<NR, TRANS, !FWD>;
   }
-  return LFSOLVE_OK;
+  return sweep_launch<T>(kern, S, grid, smem, j0, st);
 }
 
 // A block per front walks through its phases where that fills the GPU evenly
