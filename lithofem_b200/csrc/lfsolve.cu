@@ -1649,6 +1649,14 @@ bool front_per_block(size_t fronts, int max_m) {
   return fronts >= 1024 || (fronts >= 512 && max_m <= 512) || max_m <= 160;
 }
 
+// Parts that a depth's first backward product takes its update rows in: where the
+// pivot chunks alone are too few blocks (or rows) to keep HBM busy, at least 256
+// rows each; 1: no partial sums
+int sweep_parts(const SolveShape &Z, int fronts) {
+  if (Z.k == 0 || Z.r == 0 || front_per_block(fronts, Z.m)) return 1;
+  return std::max(1, std::min(std::min(SW_PARTS, Z.r / 256), SWEEP_BLOCKS / (chunks(Z.k) * fronts)));
+}
+
 // one pass of NR columns: b (n x NR, ld n, precision T, original numbering)
 // -> x (same layout)
 template <typename T, int NR, int TRANS>
@@ -1703,10 +1711,7 @@ int solve_pass(lfsolve *s, const T *b, T *x) {
       LS_CUDA(cudaGetLastError());
     } else if (Z.k > 0) {
       if (Z.r > 0) {
-        // the update rows in parts where the pivot chunks alone are too few
-        // blocks (or rows) to keep HBM busy, at least 256 rows each
-        const int nz = std::max(1, std::min(std::min(SW_PARTS, Z.r / 256),
-                                            SWEEP_BLOCKS / (chunks(Z.k) * cnt)));
+        const int nz = sweep_parts(Z, cnt);
         if ((rc = sweep_phase<T, NR, TRANS, PH_BWD_R>(S, chunks(Z.k), cnt, 0, st, nz))) return rc;
         if (nz > 1 && (rc = sweep_phase<T, NR, TRANS, PH_BWD_S>(S, (Z.k + SW_T - 1) / SW_T, cnt, nz, st)))
           return rc;
@@ -1744,9 +1749,11 @@ int ensure_solve_scratch(lfsolve *s, size_t es) {
   const size_t V = (size_t)P.vec_rows * MAX_NRHS_PASS * es;
   const size_t Y = (size_t)std::max(1, P.nn) * MAX_NRHS_PASS * es;
   const size_t bw = (size_t)P.n * 2 * MAX_NRHS_PASS * es;  // b and x in the factor precision
-  int rc;
+  int rc, parts = 1;
+  for (int d = 0; d <= P.max_depth; ++d)
+    parts = std::max(parts, sweep_parts(P.shape[d], (int)P.by_depth[d].size()));
   if ((rc = ensure_bytes(&s->d_V, &s->V_bytes, V)) || (rc = ensure_bytes(&s->d_Y, &s->Y_bytes, Y)) ||
-      (rc = ensure_bytes(&s->d_part_y, &s->part_y_bytes, Y * SW_PARTS)) ||
+      (rc = ensure_bytes(&s->d_part_y, &s->part_y_bytes, parts > 1 ? Y * parts : 0)) ||
       (rc = ensure_bytes(&s->d_bw, &s->bw_bytes, bw)))
     return rc;
   return LFSOLVE_OK;
