@@ -1618,8 +1618,8 @@ int sweep_launch(void (*kern)(Sweep<T>, int), const Sweep<T> &S, dim3 grid, size
 // phases and take the kernels that hold their factors on chip; with more, HBM
 // is the bound, and blocks that stream them with more of their kind on an SM
 // are the faster (524k-row line grating, held and streamed, forward + backward:
-// 1 front 0.29 and 0.68 ms, 4 fronts 0.56 and 0.70, 16 fronts 0.36 and 0.39,
-// 32 fronts 0.47 and 0.48, 64 fronts 0.45 and 0.42, 256 fronts 0.31 and 0.27).
+// 1 front 0.32 and 0.64 ms, 4 fronts 0.62 and 0.75, 16 fronts 0.39 and 0.42,
+// 32 fronts 0.51 and 0.53, 64 fronts 0.48 and 0.48, 256 fronts 0.33 and 0.31).
 constexpr int HELD_FRONTS = 32;
 
 // one launch of a phase over the fronts of a depth (fewer than 1,024,
@@ -1641,10 +1641,12 @@ int sweep_phase(const Sweep<T> &S, int nch, int fronts, int j0, cudaStream_t st,
 }
 
 // A block per front walks through its phases where that fills the GPU evenly
-// (three blocks a SM: the 512 leaf fronts of a 271k-row line grating, more than
-// one wave, take 0.59 ms a sweep pair so and 0.52 ms by phases) or the fronts
-// are so small that launches would dominate (512 of 282 rows: a design step of
-// 40.5 ms so, 41.4 ms by phases); else a launch per phase.
+// (three blocks a SM) or the fronts are so small that launches would dominate;
+// else a launch per phase.  512 fronts are between the two (more than one wave);
+// a sweep pair of one column in complex64, so and by phases: 0.089 and 0.097 ms
+// with at most 282 rows, 0.124 and 0.124 with 360, 0.366 and 0.369 with 633,
+// 0.565 and 0.557 with 861; of two columns 0.102 and 0.109, 0.139 and 0.143,
+// 0.409 and 0.391, 0.622 and 0.575.
 bool front_per_block(size_t fronts, int max_m) {
   return fronts >= 1024 || (fronts >= 512 && max_m <= 512) || max_m <= 160;
 }
