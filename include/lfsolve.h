@@ -72,7 +72,7 @@ int lfsolve_set_stream(lfsolve *s, void *stream);
  * the device CSR's structure), the mesh's ne elements with nd DOFs each
  * (elem_dof, ne * nd) and their centroids (ne * 3), and the n_ess essential
  * rows.  Subdomains of at most leaf_elements elements (<= 0: 32) are not
- * split further. */
+ * split further.  Replaces the previous analysis and releases its factors. */
 int lfsolve_analyze(lfsolve *s, int n, const int *I, const int *J, long long nnz, int ne,
                     int nd, const int *elem_dof, const double *centroid, const int *ess,
                     int n_ess, int leaf_elements);
